@@ -243,6 +243,10 @@ constexpr int MQ_KB = 8, MQ_NST = 3, MQ_PITCH = 34 * MQ_KB, MQ_DPITCH = 12;   //
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+// 16 bytes, or 16 zeros without reading anything
+__device__ __forceinline__ void cp_async16_or_zeros(uint32_t dst, const void *src, bool read) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(read ? 16 : 0) : "memory");
+}
 __device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
@@ -252,7 +256,11 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint
 template <int BM, int BN>
 __host__ __device__ constexpr int mq_stage_bytes() { return (BM + BN) * MQ_PITCH + BN * MQ_DPITCH * 4; }
 
-template <int BM, int BN>
+// RAGGED: activation rows that are not there arrive as zeros.  With copies of the last row in their place every CTA read one
+// row up to 55 times over: 9, 65 and 600 rows against a [37984 x 1024] head took 143, 169 and 310 us (64 rows: 35), and 33, 57
+// and 248 with the zeros.  The test costs full tiles 1 % (5 % at 700 rows of [2048 x 7168]): they, and tiles that lack an
+// eighth of their rows at most, keep the plain copies.
+template <int BM, int BN, bool RAGGED>
 __global__ void __launch_bounds__(128) q8_0_mma_kernel(float *__restrict__ y, int ldy, const uint8_t *__restrict__ w,
                                                        const int8_t *__restrict__ xq, const float *__restrict__ xd, int S,
                                                        int I, int O, int accumulate) {
@@ -271,15 +279,19 @@ __global__ void __launch_bounds__(128) q8_0_mma_kernel(float *__restrict__ y, in
             cp_async16(dst + r * MQ_PITCH + 16 * k, w + (size_t)min(o0 + r, O - 1) * rb + (size_t)st * MQ_PITCH + 16 * k);
         }
     };
+    auto copy_x = [&](uint32_t dst, const void *src, int r) {
+        if (RAGGED) cp_async16_or_zeros(dst, src, s0 + r < S);
+        else cp_async16(dst, src);
+    };
     auto load_x = [&](int st) {
         const uint32_t dst = base + (st % MQ_NST) * STAGE + BM * MQ_PITCH;
         for (int i = tid; i < BN * 16; i += 128) {
             const int r = i >> 4, k = i & 15;
-            cp_async16(dst + r * MQ_PITCH + 16 * k, xq + (size_t)min(s0 + r, S - 1) * I + st * (32 * MQ_KB) + 16 * k);
+            copy_x(dst + r * MQ_PITCH + 16 * k, xq + (size_t)min(s0 + r, S - 1) * I + st * (32 * MQ_KB) + 16 * k, r);
         }
         for (int i = tid; i < BN * 2; i += 128) {
             const int r = i >> 1, k = i & 1;
-            cp_async16(dst + BN * MQ_PITCH + r * MQ_DPITCH * 4 + 16 * k, xd + (size_t)min(s0 + r, S - 1) * nb + st * MQ_KB + 4 * k);
+            copy_x(dst + BN * MQ_PITCH + r * MQ_DPITCH * 4 + 16 * k, xd + (size_t)min(s0 + r, S - 1) * nb + st * MQ_KB + 4 * k, r);
         }
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
@@ -751,7 +763,8 @@ int launch_quantize_q8_0(const float *x, int ldx, int8_t *q, float *d, int rows,
 template <int BM, int BN>
 int launch_q8_0_mma(float *y, int ldy, const void *w, const int8_t *xq, const float *xd, int S, int I, int O, int accumulate,
                     cudaStream_t st) {
-    auto fn = q8_0_mma_kernel<BM, BN>;
+    const int lacking = (BN - S % BN) % BN;   // rows of the last tile past the batch
+    auto fn = lacking > BN / 8 ? q8_0_mma_kernel<BM, BN, true> : q8_0_mma_kernel<BM, BN, false>;
     const size_t smem = (size_t)MQ_NST * mq_stage_bytes<BM, BN>();
     if (raise_dynamic_smem(reinterpret_cast<const void *>(fn), smem) != ZMOE_OK) return ZMOE_ERR_CUDA;
     count_launches(1);
