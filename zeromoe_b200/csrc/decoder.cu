@@ -363,7 +363,10 @@ __global__ void __launch_bounds__(128) q8_0_mma_kernel(float *__restrict__ y, in
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const float v = __fsub_rn(part[i][j][k], comp[i][j][k]), t = __fadd_rn(acc[i][j][k], v);
-                    comp[i][j][k] = __fsub_rn(__fsub_rn(t, acc[i][j][k]), v);
+                    // An infinite scale makes the sum infinite and its compensation NaN; the sum has to stay what it is.  The
+                    // maximum drops a NaN, and finite scales never come near its bound: a block is at most 32 * 127 * 127 *
+                    // 65504^2 = 2^51, so is the compensation of fewer than 2^24 of them.
+                    comp[i][j][k] = fmaxf(__fsub_rn(__fsub_rn(t, acc[i][j][k]), v), -0x1p105f);
                     acc[i][j][k] = t;
                 }
     }
