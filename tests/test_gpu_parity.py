@@ -288,10 +288,11 @@ def test_tiled_router_vs_decode_router(zlib, dev, T, E, K, D):
     assert sure > 0
 
 
-@pytest.mark.parametrize("T", [8, 9, 257, 1100])
+@pytest.mark.parametrize("T", [8, 9, 16, 17, 257, 1024, 1100])
 def test_planner_runs_of_pairs(zlib, dev, T):
-    """the planner gives each of its warps a run of pairs: one run, two with a short second, and more pairs than are mirrored
-    in shared memory, with inactive routes among them.  One pair at a time (path 3) a token's row does not depend on the
+    """the planner gives each of its warps a run of pairs: one run (up to 128 pairs), three with a short last, more pairs than are
+    mirrored in shared memory, and the 8192 up to which there are runs, with inactive routes among them; more pairs take places
+    in any order.  One pair at a time (path 3) a token's row does not depend on the
     others, so a batch must return what its tokens return four at a time."""
     import torch
     D, F, E, K = 256, 256, 40, 8

@@ -134,8 +134,9 @@ __global__ void __launch_bounds__(ROUTER_THREADS) router_decode_kernel(const Rou
     PlanOut po{a.plan.hdr, a.plan.active, a.plan.offs, a.plan.slot, a.plan.item_offs_gu, a.plan.item_offs_dn,
                a.plan.freq, a.plan.aoffs, a.plan.antok, a.nrt_gu, a.nrt_dn, a.plan.pos, a.plan.mt_gu, a.plan.mt_dn};
     // the routing scratch at the start of dyn is free again: 2 * NW * E words, NW * E of them for the planner's counts
-    // (a run per 64 pairs, as in the stand-alone planner: with eight runs three tokens paid half a microsecond per call for empty ones)
-    build_plan_cta(a.ids, a.T * a.K, a.E, po, cnt_s, pre_s, ids_s, reinterpret_cast<int *>(dyn), min(NW, (a.T * a.K + 63) / 64));
+    const int nfill = plan_runs(a.T * a.K, NW);
+    if (nfill == 1) build_plan_cta<PLAN_ONE_RUN>(a.ids, a.T * a.K, a.E, po, cnt_s, pre_s, ids_s, nullptr, 1);
+    else build_plan_cta<PLAN_RUNS>(a.ids, a.T * a.K, a.E, po, cnt_s, pre_s, ids_s, reinterpret_cast<int *>(dyn), nfill);
     if (tid == 0 && n_tg > 1) a.ticket[0] = 0u;
 #ifdef ZMOE_GEMM_STATS
     // phases of the CTA that ends the kernel, in ns: logits + quantise, ticket, routing, ticket, plan; calls
@@ -306,8 +307,11 @@ struct RouteIngest {
     int ids_ld = 0, w_ld = 0;
 };
 
-__global__ void __launch_bounds__(1024) plan_from_ids_kernel(const int32_t *ids, int P, int E, PlanOut po, RouteIngest in,
-                                                             int nfill) {
+// 64 registers a thread instead of 32 take a tenth off a call of few pairs; the fill in any order keeps 32, because a CTA of all
+// of an SM's registers has to wait until the selection before it has left one (a route call of 2000 tokens: 99 us, 94 with 32).
+template <PlanFill FILL>
+__global__ void __launch_bounds__(1024, FILL == PLAN_ANY_ORDER ? 2 : 1)
+plan_from_ids_kernel(const int32_t *ids, int P, int E, PlanOut po, RouteIngest in, int nfill) {
     extern __shared__ int plan_s[];
     pdl_wait_prior_grid();
     pdl_launch_dependents();
@@ -320,8 +324,8 @@ __global__ void __launch_bounds__(1024) plan_from_ids_kernel(const int32_t *ids,
         }
         __syncthreads();
     }
-    int *wcnt_s = plan_s + 2 * (E + 1);
-    build_plan_cta(ids, P, E, po, plan_s, plan_s + E + 1, P <= ROUTER_IDS_SMEM ? wcnt_s + nfill * E : nullptr, wcnt_s, nfill);
+    int *wcnt_s = plan_s + 2 * (E + 1), *ids_s = wcnt_s + (FILL == PLAN_RUNS ? nfill * E : 0);
+    build_plan_cta<FILL>(ids, P, E, po, plan_s, plan_s + E + 1, P <= ROUTER_IDS_SMEM ? ids_s : nullptr, wcnt_s, nfill);
 }
 
 static int launch_plan(const int32_t *ids, int P, int E, const PlanBuffers &plan, int nrt_gu, int nrt_dn,
@@ -330,15 +334,15 @@ static int launch_plan(const int32_t *ids, int P, int E, const PlanBuffers &plan
                plan.aoffs, plan.antok, nrt_gu, nrt_dn, plan.pos, plan.mt_gu, plan.mt_dn};
     const size_t fixed = (size_t)2 * (E + 1) * sizeof(int) + (P <= ROUTER_IDS_SMEM ? (size_t)P * sizeof(int) : 0);
     if (fixed > 48 * 1024) return ZMOE_ERR_SHAPE;
-    // warps that fill: one per 64 pairs, as many as there is room to count for
-    int nfill = (P + 63) / 64;
-    if (nfill > 32) nfill = 32;
+    // warps that fill, as many as there is room to count for
     const size_t room = (200 * 1024 - fixed) / ((size_t)E * sizeof(int));
-    if ((size_t)nfill > room) nfill = (int)room;
-    const size_t smem = fixed + (size_t)nfill * E * sizeof(int);
-    if (smem > 48 * 1024 && raise_dynamic_smem(reinterpret_cast<const void *>(plan_from_ids_kernel), 200 * 1024) != ZMOE_OK)
-        return ZMOE_ERR_CUDA;
-    return launch_pdl(plan_from_ids_kernel, dim3(1), dim3(1024), smem, st, ids, P, E, po, in, nfill) == cudaSuccess
+    const int nfill = plan_runs(P, room < 32 ? (int)room : 32);
+    const PlanFill fill = P > PLAN_RUNS_PAIRS ? PLAN_ANY_ORDER : nfill == 1 ? PLAN_ONE_RUN : PLAN_RUNS;
+    auto fn = fill == PLAN_ANY_ORDER ? plan_from_ids_kernel<PLAN_ANY_ORDER>
+              : fill == PLAN_ONE_RUN ? plan_from_ids_kernel<PLAN_ONE_RUN> : plan_from_ids_kernel<PLAN_RUNS>;
+    const size_t smem = fixed + (fill == PLAN_RUNS ? (size_t)nfill * E * sizeof(int) : 0);
+    if (smem > 48 * 1024 && raise_dynamic_smem(reinterpret_cast<const void *>(fn), 200 * 1024) != ZMOE_OK) return ZMOE_ERR_CUDA;
+    return launch_pdl(fn, dim3(1), dim3(1024), smem, st, ids, P, E, po, in, nfill) == cudaSuccess
                ? ZMOE_OK
                : ZMOE_ERR_CUDA;
 }

@@ -152,35 +152,66 @@ __device__ void route_token_warp(const RouterSpec &sp, const float *row_in, floa
     }
 }
 
+// How the planner fills an expert's list.  Up to 128 pairs one warp takes them all (a single run: its counts are the totals and
+// its cursors the experts' offsets, which saves a pass and a barrier: 8 tokens of 8 among 128 experts, quantiser and planner
+// 7.0 -> 6.0 us); then a run of pairs per warp.  Above 8192 pairs the runs take longer than atomics (32 warps share one SM's
+// rate of match instructions: 16000 pairs 29 us, 64000 102), and a pair takes the next place, whichever that is (20, 68): the
+// order inside an expert then differs from call to call; a pair's row does not depend on its place.
+enum PlanFill { PLAN_ONE_RUN, PLAN_RUNS, PLAN_ANY_ORDER };
+constexpr int PLAN_ONE_RUN_PAIRS = 128, PLAN_RUNS_PAIRS = 8192;
+// runs of pairs: one per 64, at most `most`
+__host__ __device__ inline int plan_runs(int P, int most) {
+    const int runs = P <= PLAN_ONE_RUN_PAIRS ? 1 : (P + 63) / 64;
+    return runs < most ? runs : most;
+}
+
 // CSR of pairs by expert plus the item spaces of the projections.  Called by
 // all threads of ONE CTA; cnt_s/pre_s: shared scratch of E+1 ints each; ids_s:
-// optional shared scratch of P ints (a copy of ids that the stable fill scans); wcnt_s: shared scratch of
+// optional shared scratch of P ints (a copy of ids that the stable fill scans); wcnt_s (PLAN_RUNS): shared scratch of
 // nfill * E ints, nfill a number of the CTA's warps.
 // ids: [T*K] (entries outside [0,E) are skipped: negative = inactive route,
 // reference backends/ggml/mmid_route_skip.hpp:60-67).
-__device__ void build_plan_cta(const int32_t *ids, int P, int E, const PlanOut &po, int *cnt_s, int *pre_s,
-                               int *ids_s, int *wcnt_s, int nfill) {
+template <PlanFill FILL>
+__device__ __forceinline__ void build_plan_cta(const int32_t *ids, int P, int E, const PlanOut &po, int *cnt_s, int *pre_s,
+                                               int *ids_s, int *wcnt_s, int nfill) {
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
     // warp w of the first nfill takes the w-th run of pairs (a multiple of 32 long), here and in the fill below
-    const int run_len = ((P + nfill - 1) / nfill + 31) & ~31;
-    const int p_lo = min(P, warp * run_len), p_hi = warp < nfill ? min(P, p_lo + run_len) : p_lo;
-    for (int i = tid; i < nfill * E; i += nt) wcnt_s[i] = 0;
-    __syncthreads();
-    for (int p = p_lo + lane; p < p_hi; p += 32) {
-        const int e = ids[p];
-        if (ids_s) ids_s[p] = e;
-        if (e >= 0 && e < E) atomicAdd(&wcnt_s[warp * E + e], 1);
-    }
-    __syncthreads();
-    // per expert: the pairs of the runs before each run, and of all
-    for (int e = tid; e < E; e += nt) {
-        int before = 0;
-        for (int w = 0; w < nfill; ++w) {
-            const int c = wcnt_s[w * E + e];
-            wcnt_s[w * E + e] = before;
-            before += c;
+    int p_lo = 0, p_hi = warp == 0 ? P : 0;
+    if (FILL != PLAN_RUNS) {
+        for (int e = tid; e < E; e += nt) cnt_s[e] = 0;
+        __syncthreads();
+        for (int p = tid; p < P; p += nt) {
+            const int e = ids[p];
+            if (ids_s) ids_s[p] = e;
+            if (e >= 0 && e < E) atomicAdd(&cnt_s[e], 1);
         }
-        cnt_s[e] = before;
+    } else {
+        const int run_len = ((P + nfill - 1) / nfill + 31) & ~31;
+        p_lo = min(P, warp * run_len);
+        p_hi = warp < nfill ? min(P, p_lo + run_len) : p_lo;
+        for (int i = tid; i < nfill * E; i += nt) wcnt_s[i] = 0;
+        __syncthreads();
+        for (int p0 = p_lo + lane; p0 < p_hi; p0 += 128) {
+            int e[4];                                  // four loads on their way at once
+#pragma unroll
+            for (int i = 0; i < 4; ++i) e[i] = p0 + 32 * i < p_hi ? ids[p0 + 32 * i] : -1;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (ids_s && p0 + 32 * i < p_hi) ids_s[p0 + 32 * i] = e[i];
+                if (e[i] >= 0 && e[i] < E) atomicAdd(&wcnt_s[warp * E + e[i]], 1);
+            }
+        }
+        __syncthreads();
+        // per expert: the pairs of the runs before each run, and of all
+        for (int e = tid; e < E; e += nt) {
+            int before = 0;
+            for (int w = 0; w < nfill; ++w) {
+                const int c = wcnt_s[w * E + e];
+                wcnt_s[w * E + e] = before;
+                before += c;
+            }
+            cnt_s[e] = before;
+        }
     }
     __syncthreads();
     if (tid < 32) {
@@ -234,15 +265,26 @@ __device__ void build_plan_cta(const int32_t *ids, int P, int E, const PlanOut &
         }
     }
     __syncthreads();
+    if (FILL == PLAN_ANY_ORDER) {
+        for (int p = tid; p < P; p += nt) {
+            const int e = ids[p];
+            const bool on = e >= 0 && e < E;
+            const int at = on ? atomicAdd(&pre_s[e], 1) : -1;
+            if (on) po.slot[at] = p;
+            if (po.pos) po.pos[p] = at;
+        }
+        return;
+    }
     // Stable fill, a run of pairs per warp, 32 pairs at a time: lanes that name the same expert find each other
     // (match), the first of them takes the run's cursor for the expert and moves it on, each writes its pair at
     // cursor + its rank among them.  (A thread per expert walking all pairs costs P dependent steps, 44 us at 1024 pairs;
     // one warp for all pairs P / 32 of them.)
     const int *src = ids_s ? ids_s : ids;
-    int *cur = wcnt_s + warp * E;
+    int *cur = FILL == PLAN_ONE_RUN ? pre_s : wcnt_s + warp * E;
+    int ahead = p_lo + lane < p_hi ? src[p_lo + lane] : -1;    // the next step's load flies during this step
     for (int p0 = p_lo; p0 < p_hi; p0 += 32) {
-        const int p = p0 + lane;
-        const int e = p < p_hi ? src[p] : -1;
+        const int p = p0 + lane, e = ahead;
+        ahead = p + 32 < p_hi ? src[p + 32] : -1;
         const bool on = e >= 0 && e < E;
         const unsigned peers = __match_any_sync(0xffffffffu, on ? e : -1 - lane);
         const int leader = __ffs(peers) - 1;
@@ -252,7 +294,7 @@ __device__ void build_plan_cta(const int32_t *ids, int P, int E, const PlanOut &
             cur[e] = base + __popc(peers);
         }
         base = __shfl_sync(0xffffffffu, base, leader);
-        if (on) base += pre_s[e];
+        if (FILL == PLAN_RUNS && on) base += pre_s[e];
         const int at = base + __popc(peers & ((1u << lane) - 1u));
         if (on) po.slot[at] = p;
         if (po.pos && p < p_hi) po.pos[p] = on ? at : -1;
