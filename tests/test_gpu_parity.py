@@ -252,11 +252,12 @@ def test_layer_router_vs_oracle(zlib, oracle, dev, case, T):
     assert np.array_equal(ctx.expert_freq(E), np.diff(offs))
 
 
-@pytest.mark.parametrize("T,E,K,D", [(97, 128, 8, 2048), (256, 11, 4, 512), (700, 200, 8, 4096), (100, 1600, 8, 256)])
+@pytest.mark.parametrize("T,E,K,D", [(97, 128, 8, 2048), (256, 11, 4, 512), (700, 200, 8, 4096), (100, 1600, 8, 256), (200, 8, 2, 4096)])
 def test_tiled_router_vs_decode_router(zlib, dev, T, E, K, D):
     """batches above 96 tokens take the tiled router (k split, partials summed in order); batches of up to 96 the one the
     oracle test pins.  The same tokens through both: probabilities to f32 summation order, the same experts wherever the
-    last chosen and the first left out differ by more than that (1e-5 of a probability).  1600 experts stay on the decode router."""
+    last chosen and the first left out differ by more than that (1e-5 of a probability).  1600 experts stay on the decode router, and so do 8
+    at 200 tokens."""
     import torch
     F = 256
     gen = torch.Generator(device=dev).manual_seed(31)
@@ -286,6 +287,38 @@ def test_tiled_router_vs_decode_router(zlib, dev, T, E, K, D):
         assert np.array_equal(ids[t0:t0 + n][ok], part[ok])
         assert np.allclose(wts[t0:t0 + n][ok], pw[ok], atol=1e-5)
     assert sure > 0
+
+
+@pytest.mark.parametrize("T,E,K,D", [(160, 128, 8, 2048), (256, 11, 4, 512), (240, 200, 8, 7168)])
+def test_tiled_router_sums_as_close_to_64_bits_as_the_decode_router(zlib, dev, T, E, K, D):
+    """up to 256 tokens the tiled router stands in for the decode router, whose sums are short: its logits must not be further
+    from 64 bits (a tenth is left for the sample).  Logits are read back as log probabilities, less their row's mean; with a
+    spread of 8 the exponential's own rounding is small beside theirs."""
+    import torch
+    F = 256
+    gen = torch.Generator(device=dev).manual_seed(36)
+    w = torch.zeros((E, F, D // 256 * 144), dtype=torch.uint8, device=dev)
+    wd = torch.zeros((E, D, F // 256 * 144), dtype=torch.uint8, device=dev)
+    wr = torch.randn((E, D), device=dev, generator=gen) * (8.0 * D ** -0.5)
+    x = torch.randn((T, D), device=dev, generator=gen)
+    ctx = zlib.Context(T, D, F, E, K)
+    layer = zlib.Layer(ctx, D, F, E, K, (synth.Q4_K,) * 3, w, w, wd, router_w=wr)
+    ref = torch.log_softmax(x.double() @ wr.double().T, dim=1).cpu().numpy()
+
+    def deviation(step):
+        total, count = 0.0, 0
+        for t0 in range(0, T, step):
+            n = min(step, T - t0)
+            layer.route(x[t0:t0 + n].contiguous())
+            _sync()
+            p = ctx.probs(n, E).astype(np.float64)
+            ok = p > 1e-25
+            d = np.where(ok, np.log(np.maximum(p, 1e-300)) - ref[t0:t0 + n], 0.0)
+            d = np.where(ok, d - (d.sum(axis=1) / ok.sum(axis=1))[:, None], 0.0)
+            total, count = total + (d * d).sum(), count + ok.sum()
+        ctx.check()
+        return np.sqrt(total / count)
+    assert deviation(T) < 1.1 * deviation(80)
 
 
 @pytest.mark.parametrize("T", [8, 9, 16, 17, 257, 1024, 1100])

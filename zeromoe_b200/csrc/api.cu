@@ -386,7 +386,7 @@ int zmoe_route(zmoe_layer *L, const float *x_dev, int T, void *stream) {
     a.logits_part = c->logits_part;
     a.logits_part_rows = router_part_rows(c->max_t) * c->max_e / L->d.n_experts;
     a.n_sm = c->n_sm;
-    const bool big = T > 256 || (T > ROUTER_TILED_TOKENS && a.E <= ROUTER_TILED_EXPERTS);
+    const bool big = router_takes_tiles(T, a.D, a.E);
     // the tensor-core path quantises the rows itself while it gathers them: the large-batch router then skips q8x
     a.want_q8x = !(big && takes_gemm(L, T));
     int rc = big ? launch_router_prefill(a, static_cast<cudaStream_t>(stream))

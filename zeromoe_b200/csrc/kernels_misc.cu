@@ -176,7 +176,12 @@ int launch_router_decode(const RouterArgs &a, cudaStream_t st) {
 // take a third fewer shared-memory cycles per product than four, but leave half as many CTAs.  8192 tokens of 7168 against
 // 256 experts: 1175 us with one buffer and 64-token tiles, 852 now; a route call of 700 tokens of 4096, 128 experts, 119 -> 65.
 // ------------------------------------------------------------------------
-template <int TM>
+// SHORT: batches of up to 256 tokens, which one CTA per expert and four tokens would take (router_decode_kernel), keep the
+// short sums they have there: a chain of the D / ksplit products of a part is two to three times as far from 64 bits as that
+// kernel's chains of 4 to 28 products and a tree over the CTA.  Here a step's products are chains of four and a tree, four steps
+// a chain, then those.  RMS deviation from 64 bits at hidden 2048 / 4096 / 7168, in 1e-7 of the logits' spread:
+// decode router 1.23, 1.35, 1.52, one chain per part 2.29, 3.06, 3.94, this 1.19, 1.24, 1.32.
+template <int TM, bool SHORT>
 __global__ void __launch_bounds__(256) router_logits_gemm_kernel(const float *__restrict__ x,
                                                                  const float *__restrict__ wr,
                                                                  float *__restrict__ logits, int T, int D, int E,
@@ -211,29 +216,60 @@ __global__ void __launch_bounds__(256) router_logits_gemm_kernel(const float *__
         }
         ws[b][lc + 0][lr] = wv.x; ws[b][lc + 1][lr] = wv.y; ws[b][lc + 2][lr] = wv.z; ws[b][lc + 3][lr] = wv.w;
     };
-    float acc[TM][4] = {};
+    float acc[TM][4] = {}, few[TM][4] = {};            // few: SHORT, the sum of up to four steps
+    auto add = [](float (&sum)[TM][4], const float (&v)[TM][4]) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sum[i][j] = __fadd_rn(sum[i][j], v[i][j]);
+    };
     fetch(kbeg);
     put(0);
     __syncthreads();
-    int buf = 0;
+    int buf = 0, n_few = 0;
     for (int k0 = kbeg; k0 < kend; k0 += 16, buf ^= 1) {
         const bool more = k0 + 16 < kend;
         if (more) fetch(k0 + 16);
+        auto chain = [&](int kb, int n, float (&sum)[TM][4]) {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            float av[TM];
+            for (int k = kb; k < kb + n; ++k) {
+                float av[TM];
 #pragma unroll
-            for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4 *>(&av[i]) = *reinterpret_cast<const float4 *>(&xs[buf][k][tm + i]);
-            const float4 b = *reinterpret_cast<const float4 *>(&ws[buf][k][tn]);
-            const float bv[4] = {b.x, b.y, b.z, b.w};
+                for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4 *>(&av[i]) = *reinterpret_cast<const float4 *>(&xs[buf][k][tm + i]);
+                const float4 b = *reinterpret_cast<const float4 *>(&ws[buf][k][tn]);
+                const float bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
+                for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+                    for (int j = 0; j < 4; ++j) sum[i][j] = fmaf(av[i], bv[j], sum[i][j]);
+            }
+        };
+        if (SHORT) {
+            float half[2][TM][4] = {};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float four[TM][4] = {};
+                chain(8 * h, 4, half[h]);
+                chain(8 * h + 4, 4, four);
+                add(half[h], four);
+            }
+            add(half[0], half[1]);
+            add(few, half[0]);
+            if (++n_few == 4) {
+                add(acc, few);
+                n_few = 0;
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) few[i][j] = 0.f;
+            }
+        } else {
+            chain(0, 16, acc);
         }
         if (more) put(buf ^ 1);                        // its last readers passed the barrier below one step ago
         __syncthreads();
     }
+    if (SHORT) add(acc, few);
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -241,8 +277,9 @@ __global__ void __launch_bounds__(256) router_logits_gemm_kernel(const float *__
             if (t0 + tm + i < T && e0 + tn + j < E) out[(size_t)(t0 + tm + i) * E + e0 + tn + j] = acc[i][j];
 }
 
-// part != nullptr: the logits are the sum of `ksplit` partial matrices part[z][T, E], added in the order z = 0, 1, ...
-__global__ void __launch_bounds__(128) router_select_kernel(float *logits, const float *part, int ksplit,
+// part != nullptr: the logits are the sum of `ksplit` (a power of two up to ROUTER_MAX_SPLIT) partial matrices part[z][T, E],
+// added in the order z = 0, 1, ..., or as a tree (for the logits of the SHORT form above)
+__global__ void __launch_bounds__(128) router_select_kernel(float *logits, const float *part, int ksplit, bool tree,
                                                             const float *bias, int32_t *ids, float *weights, int T,
                                                             RouterSpec sp) {
     extern __shared__ float rsel[];
@@ -254,9 +291,20 @@ __global__ void __launch_bounds__(128) router_select_kernel(float *logits, const
     float *row = logits + (size_t)t * sp.E;
     if (part) {
         for (int e = lane; e < sp.E; e += 32) {
-            float v = part[(size_t)t * sp.E + e];
-            for (int z = 1; z < ksplit; ++z) v = __fadd_rn(v, part[((size_t)z * T + t) * sp.E + e]);
-            row[e] = v;
+            if (tree) {
+                float v[ROUTER_MAX_SPLIT];
+#pragma unroll
+                for (int z = 0; z < ROUTER_MAX_SPLIT; ++z) v[z] = z < ksplit ? part[((size_t)z * T + t) * sp.E + e] : 0.f;
+#pragma unroll
+                for (int w = 1; w < ROUTER_MAX_SPLIT; w *= 2)
+#pragma unroll
+                    for (int z = 0; z < ROUTER_MAX_SPLIT; z += 2 * w) v[z] = __fadd_rn(v[z], v[z + w]);
+                row[e] = v[0];
+            } else {
+                float v = part[(size_t)t * sp.E + e];
+                for (int z = 1; z < ksplit; ++z) v = __fadd_rn(v, part[((size_t)z * T + t) * sp.E + e]);
+                row[e] = v;
+            }
         }
         __syncwarp();
     }
@@ -277,14 +325,15 @@ int launch_router_prefill(const RouterArgs &a, cudaStream_t st) {
     float *dst = ksplit > 1 ? a.logits_part : a.logits;
     // 128-token tiles once they still are one and a half CTAs per SM
     const int wide = ((a.E + 63) / 64) * ((a.T + 127) / 128) * ksplit;
-    const int bt = 2 * wide >= 3 * a.n_sm ? 128 : 64;
-    int rc = launch_pdl(bt == 128 ? router_logits_gemm_kernel<8> : router_logits_gemm_kernel<4>,
+    const bool sh = a.T <= ROUTER_SHORT_TOKENS;
+    const int bt = !sh && 2 * wide >= 3 * a.n_sm ? 128 : 64;
+    int rc = launch_pdl(bt == 128 ? router_logits_gemm_kernel<8, false> : sh ? router_logits_gemm_kernel<4, true> : router_logits_gemm_kernel<4, false>,
                         dim3((a.E + 63) / 64, (a.T + bt - 1) / bt, ksplit), dim3(256), 0, st, a.x, a.wr, dst, a.T, a.D, a.E,
                         ksplit) == cudaSuccess ? ZMOE_OK : ZMOE_ERR_CUDA;
     RouterSpec sp{a.E, a.K, a.gating, a.normalize, a.weight_scale, a.n_groups, a.n_groups_used};
     if (!rc)
         rc = launch_pdl(router_select_kernel, dim3((a.T + 3) / 4), dim3(128), (size_t)8 * a.E * sizeof(float), st,
-                        a.logits, (const float *)(ksplit > 1 ? a.logits_part : nullptr), ksplit, a.bias, a.ids, a.weights,
+                        a.logits, (const float *)(ksplit > 1 ? a.logits_part : nullptr), ksplit, sh, a.bias, a.ids, a.weights,
                         a.T, sp) == cudaSuccess ? ZMOE_OK : ZMOE_ERR_CUDA;
     if (!rc && a.want_q8x) rc = launch_quantize_rows(a.x, a.D, a.q8x, a.T, a.D, a.q8_layout, st);
     if (!rc) rc = launch_plan_from_ids(a.ids, a.T * a.K, a.E, a.plan, a.nrt_gu, a.nrt_dn, st);

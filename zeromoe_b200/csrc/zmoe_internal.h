@@ -66,12 +66,20 @@ struct RouterArgs {
     unsigned long long *stats = nullptr;   // phase timers of the decode router (builds with ZMOE_GEMM_STATS), or null
 };
 constexpr int ROUTER_MAX_SPLIT = 16;
-// Batches above this many tokens take the tiled router.  A CTA per (expert, 4 tokens) reads every activation row E times
-// and grows with the batch; the tiles split k until they fill the chip, but are four launches for one.  A route call, decode
-// against tiled, us: hidden 4096, 128 experts: 96 tokens 34 / 37, 128 tokens 47 / 37, 256 tokens 84 / 40; hidden 7168, 256
-// experts: 96 tokens 66 / 59, 256 tokens 163 / 96.
-constexpr int ROUTER_TILED_TOKENS = 96;
+// The tiled router or the decode router.  The decode router's CTA per (expert, 4 tokens) reads every activation row E times, so it
+// grows with T * E; the tiles split k up to sixteen ways, so they take as long as D / 16 products and three more launches whatever
+// the batch is.  A route call, decode against tiled, us: hidden 2048, 128 experts: 97 tokens 30 / 24, 256 61 / 27; 7168, 256
+// experts: 97 66 / 44, 256 150 / 66; 4096, 64 experts: 97 23 / 27, 128 27 / 28, 256 43 / 27; 7168, 64 experts: 97 26 / 36,
+// 160 37 / 37; 4096, 32 experts: 160 22 / 24, 256 29 / 25; 4096, 8 experts: 256 18 / 24.  Both have the same short sums up to
+// ROUTER_SHORT_TOKENS; larger batches take the tiles alone, with longer ones.
+constexpr int ROUTER_TILED_TOKENS = 96, ROUTER_SHORT_TOKENS = 256;
 constexpr int ROUTER_TILED_EXPERTS = 1536;   // the tiled router's selection holds this many in shared memory
+constexpr int ROUTER_DECODE_HIDDEN = 8192;   // the decode router holds a row of this many elements in registers
+inline bool router_takes_tiles(long T, long D, long E) {
+    if (T > ROUTER_SHORT_TOKENS) return true;
+    if (T <= ROUTER_TILED_TOKENS || E > ROUTER_TILED_EXPERTS) return false;
+    return 5 * T * E > 8 * D || D > ROUTER_DECODE_HIDDEN;
+}
 inline long router_part_rows(long max_tokens) {
     const long split = ROUTER_MAX_SPLIT * (max_tokens < 1024 ? max_tokens : 1024);
     return split > 4 * max_tokens ? split : 4 * max_tokens;
