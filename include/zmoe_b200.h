@@ -411,6 +411,13 @@ int zmoe_block_isums(int type, const void *w_dev, const float *x_dev, int32_t *i
 int zmoe_block_isums_pairs(int type, const void *w_dev, const float *x_dev, int32_t *sums_dev, int pairs, int I,
                            void *stream);
 
+/* the attention of a long prompt, as zmoe_decoder_step runs it over tiles of query rows, on its own: qkv_dev f32
+ * [T, (H + 2 KV) * head_dim] (q rotated; its k and v columns are not read), k_dev / v_dev f16 [max_ctx][KV * head_dim] that
+ * hold the T tokens' own rows too, pos_dev the position of the first token; out_dev f32 [T, H * head_dim].
+ * head_dim 64 or 128, H a multiple of KV, H / KV <= 32. */
+int zmoe_attention_rows(const float *qkv_dev, const void *k_dev, const void *v_dev, float *out_dev, const int *pos_dev,
+                        int T, int H, int KV, int head_dim, int max_ctx, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

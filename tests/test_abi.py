@@ -38,6 +38,11 @@ def test_argument_validation_needs_no_device():
     assert L.zmoe_ctx_set_path(None, 0) == -1
     assert L.zmoe_quantize_q8_K(None, None, 1, 256, lib.Q4_K, None) == -1
     assert L.zmoe_block_isums(99, None, None, None, None, 1, 256, None) == -1
+    assert L.zmoe_attention_rows(None, None, None, None, None, 1, 8, 2, 128, 64, None) == -1
+    p = C.c_void_p(256)                       # refused before anything is read: no such head size, no such grouping
+    assert L.zmoe_attention_rows(p, p, p, p, p, 1, 8, 2, 96, 64, None) == -3
+    assert L.zmoe_attention_rows(p, p, p, p, p, 1, 8, 3, 128, 64, None) == -3
+    assert L.zmoe_attention_rows(p, p, p, p, p, 1, 33, 1, 128, 64, None) == -3
     assert L.zmoe_reserve(4, 100) == -1
     assert L.zmoe_ctx_bad_counts(None, None, 0) == -1
     assert L.zmoe_gemm_min_pairs_per_expert() == 24

@@ -564,13 +564,15 @@ __global__ void __launch_bounds__(256) attention_merge_q8_0_kernel(const float *
 // The same for many tokens at once (a prompt): a CTA takes 64 query rows of one KV head (64 / G tokens times the G heads of
 // the group), walks the keys in tiles of 64 and keeps its output rows in registers, so that a K or V row is fetched once
 // per 64 query rows instead of once per token (attention_kernel reads each key's row with one lane, 16 bytes at a time, for
-// every token: 370 + 38 us with the merge at 512 tokens of 32 heads of 128, against 131 here).  f32 throughout, as there: the products are
+// every token: 370 + 38 us with the merge at 512 tokens of 32 heads of 128, against 136 here).  f32 throughout, as there: the products are
 // bound by the FMA pipe and by shared memory (4 x 4 scores and 4 x HD / 16 outputs per thread).  K and V share one
-// buffer, which leaves room for two CTAs per SM: one loads while the other multiplies.
+// buffer, which leaves room for two CTAs per SM: one loads while the other multiplies.  The weighted sum of V is added up
+// in ATTN_SPLITS shares of the keys and the shares then, as there: one chain over all keys was 2.7 times as far from 64 bits at
+// 512 keys, and more with each key.
 // ---------------------------------------------------------------------------
 constexpr int AP_ROWS = 64, AP_KEYS = 64, AP_PP = AP_KEYS + 4;
 template <int HD>
-constexpr size_t attention_prompt_smem() { return ((size_t)(AP_ROWS + AP_KEYS) * (HD + 4) + (size_t)AP_ROWS * AP_PP) * sizeof(float); }
+constexpr size_t attention_prompt_smem() { return ((size_t)(AP_ROWS + AP_KEYS) * (HD + 4) + (size_t)AP_ROWS * (AP_PP + 3)) * sizeof(float); }
 
 template <int HD>
 __global__ void __launch_bounds__(256, 2) attention_prompt_kernel(const float *__restrict__ qkv, const __half *__restrict__ kc,
@@ -580,6 +582,10 @@ __global__ void __launch_bounds__(256, 2) attention_prompt_kernel(const float *_
     constexpr int PITCH = HD + 4, NV = HD / 64;   // NV: float4 of an output row per thread
     extern __shared__ __align__(16) float ap_s[];
     float *qs = ap_s, *kv = qs + AP_ROWS * PITCH, *ps = kv + AP_KEYS * PITCH;
+    // per row, written by the first of its sixteen threads (registers are short): the keys it sees; the sum of weights of
+    // the shares that are complete; what the maximum has taken from those since
+    float *l_s = ps + AP_ROWS * AP_PP, *since_s = l_s + AP_ROWS;
+    int *nk_s = reinterpret_cast<int *>(since_s + AP_ROWS);
     pdl_wait_prior_grid();
     pdl_launch_dependents();
     const int G = H / KV, TQ = AP_ROWS / G;
@@ -593,19 +599,26 @@ __global__ void __launch_bounds__(256, 2) attention_prompt_kernel(const float *_
         if (r < TQ * G && t < T) v = *reinterpret_cast<const float4 *>(qkv + (size_t)t * ld + (size_t)(kvh * G + r % G) * HD + 4 * c);
         *reinterpret_cast<float4 *>(qs + r * PITCH + 4 * c) = v;
     }
-    int nk[4];                                    // keys each of this thread's rows sees
-    float m[4], l[4], acc[4][NV][4];
+    if (tid < AP_ROWS) {
+        nk_s[tid] = min(p0 + t0 + tid / G + 1, max_ctx);
+        l_s[tid] = 0.f;
+        since_s[tid] = 1.f;
+    }
+    // acc: weighted sum of V of the complete shares, for the maximum at that time; as, ls: of the current one, with its sum
+    // of weights, for the maximum m
+    float m[4], ls[4], acc[4][NV][4], as[4][NV][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        nk[i] = min(p0 + t0 + (4 * ty + i) / G + 1, max_ctx);
         m[i] = -CUDART_INF_F;
-        l[i] = 0.f;
+        ls[i] = 0.f;
 #pragma unroll
         for (int h = 0; h < NV; ++h)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][h][j] = 0.f;
+            for (int j = 0; j < 4; ++j) acc[i][h][j] = as[i][h][j] = 0.f;
     }
     const int kmax = min(p0 + min(t0 + TQ, T), max_ctx);     // keys any row of the tile sees
+    const int share = ((kmax + AP_KEYS - 1) / AP_KEYS + ATTN_SPLITS - 1) / ATTN_SPLITS * AP_KEYS;   // keys of a share: whole tiles
+    int share_end = share;
     auto load = [&](const __half *src, int k0) {
         for (int i = tid; i < AP_KEYS * (HD / 8); i += 256) {
             const int r = i / (HD / 8), c = i % (HD / 8);
@@ -646,10 +659,11 @@ __global__ void __launch_bounds__(256, 2) attention_prompt_kernel(const float *_
         // running-maximum softmax; a row's sixteen threads are half a warp
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
+            const int nk = nk_s[4 * ty + i];
             float cm = -CUDART_INF_F;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                s[i][j] = k0 + tx + 16 * j < nk[i] ? s[i][j] * scale : -CUDART_INF_F;
+                s[i][j] = k0 + tx + 16 * j < nk ? s[i][j] * scale : -CUDART_INF_F;
                 cm = fmaxf(cm, s[i][j]);
             }
 #pragma unroll
@@ -659,18 +673,19 @@ __global__ void __launch_bounds__(256, 2) attention_prompt_kernel(const float *_
             float sum = 0.f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float pr = k0 + tx + 16 * j < nk[i] ? expf(s[i][j] - mn) : 0.f;
+                const float pr = k0 + tx + 16 * j < nk ? expf(s[i][j] - mn) : 0.f;
                 ps[(4 * ty + i) * AP_PP + tx + 16 * j] = pr;
                 sum += pr;
             }
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            l[i] = l[i] * corr + sum;
+            ls[i] = ls[i] * corr + sum;
+            if (tx == 0) since_s[4 * ty + i] *= corr;
             m[i] = mn;
 #pragma unroll
             for (int h = 0; h < NV; ++h)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][h][j] *= corr;
+                for (int j = 0; j < 4; ++j) as[i][h][j] *= corr;
         }
         __syncthreads();
         // outputs of rows 4 ty + i, dimensions 64 h + 4 tx ..
@@ -687,20 +702,41 @@ __global__ void __launch_bounds__(256, 2) attention_prompt_kernel(const float *_
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float pe = e == 0 ? pr[i].x : e == 1 ? pr[i].y : e == 2 ? pr[i].z : pr[i].w;
-                        acc[i][h][0] = fmaf(pe, v.x, acc[i][h][0]);
-                        acc[i][h][1] = fmaf(pe, v.y, acc[i][h][1]);
-                        acc[i][h][2] = fmaf(pe, v.z, acc[i][h][2]);
-                        acc[i][h][3] = fmaf(pe, v.w, acc[i][h][3]);
+                        as[i][h][0] = fmaf(pe, v.x, as[i][h][0]);
+                        as[i][h][1] = fmaf(pe, v.y, as[i][h][1]);
+                        as[i][h][2] = fmaf(pe, v.z, as[i][h][2]);
+                        as[i][h][3] = fmaf(pe, v.w, as[i][h][3]);
                     }
                 }
             }
+        }
+        if (k0 + AP_KEYS >= share_end || k0 + AP_KEYS >= kmax) {
+            share_end += share;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float since = since_s[4 * ty + i];
+#pragma unroll
+                for (int h = 0; h < NV; ++h)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        acc[i][h][j] = fmaf(acc[i][h][j], since, as[i][h][j]);
+                        as[i][h][j] = 0.f;
+                    }
+                __syncwarp();                     // all sixteen have read
+                if (tx == 0) {
+                    l_s[4 * ty + i] = fmaf(l_s[4 * ty + i], since, ls[i]);
+                    since_s[4 * ty + i] = 1.f;
+                }
+                ls[i] = 0.f;
+            }
+            __syncwarp();
         }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int r = 4 * ty + i, t = t0 + r / G;
         if (r >= TQ * G || t >= T) continue;
-        const float inv = 1.0f / l[i];
+        const float inv = 1.0f / l_s[r];
 #pragma unroll
         for (int h = 0; h < NV; ++h)
             *reinterpret_cast<float4 *>(out + ((size_t)t * H + kvh * G + r % G) * HD + 64 * h + 4 * tx) =
@@ -801,6 +837,17 @@ int launch_q8_0_mm(float *y, int ldy, const void *w, const int8_t *xq, const flo
                          (size_t)O * rb, xq, xd, S, I, O, accumulate));
 }
 
+template <int HD>
+int launch_attention_prompt(const float *qkv, const __half *kc, const __half *vc, float *out, const int *pos, int T, int H, int KV,
+                            float scale, int max_ctx, cudaStream_t st) {
+    const int TQ = AP_ROWS / (H / KV);
+    auto fn = attention_prompt_kernel<HD>;
+    if (raise_dynamic_smem(reinterpret_cast<const void *>(fn), attention_prompt_smem<HD>()) != ZMOE_OK) return ZMOE_ERR_CUDA;
+    count_launches(1);
+    return cu(launch_pdl(fn, dim3((T + TQ - 1) / TQ, KV), dim3(256), attention_prompt_smem<HD>(), st, qkv, kc, vc, out, pos, T, H, KV,
+                         scale, max_ctx));
+}
+
 // Attention of T tokens, its rows quantised to Q8_0 (aq, ad): by query tiles where those are enough CTAs for half of the chip (a tile walks all keys on its
 // own, and the number of earlier positions is not known here); below that, keys split over CTAs token by token.
 template <int HD>
@@ -808,11 +855,7 @@ int launch_attention(const float *qkv, const __half *kc, const __half *vc, float
                      int KV, float scale, int max_ctx, int8_t *aq, float *ad, cudaStream_t st) {
     const int G = H / KV, TQ = AP_ROWS / G, tiles = (T + TQ - 1) / TQ;
     if (tiles * KV >= device_sm_count() / 2) {
-        auto fn = attention_prompt_kernel<HD>;
-        if (raise_dynamic_smem(reinterpret_cast<const void *>(fn), attention_prompt_smem<HD>()) != ZMOE_OK) return ZMOE_ERR_CUDA;
-        count_launches(1);
-        const int rc = cu(launch_pdl(fn, dim3(tiles, KV), dim3(256), attention_prompt_smem<HD>(), st, qkv, kc, vc, out, pos, T,
-                                     H, KV, scale, max_ctx));
+        const int rc = launch_attention_prompt<HD>(qkv, kc, vc, out, pos, T, H, KV, scale, max_ctx, st);
         return rc ? rc : launch_quantize_q8_0(out, H * HD, aq, ad, T, H * HD, st);
     }
     count_launches(2);
@@ -989,6 +1032,17 @@ int zmoe_decoder_step(zmoe_decoder *dec, const int32_t *tokens_dev, int T, void 
     if (!rc) rc = cu(launch_pdl(argmax_kernel, dim3(1), dim3(1024), 0, st, (const float *)dec->logits, d.vocab, dec->next, dec->pos, T));
     count_launches(1);
     return rc;
+}
+
+int zmoe_attention_rows(const float *qkv_dev, const void *k_dev, const void *v_dev, float *out_dev, const int *pos_dev, int T, int H,
+                        int KV, int head_dim, int max_ctx, void *stream) {
+    if (!qkv_dev || !k_dev || !v_dev || !out_dev || !pos_dev || T <= 0 || H <= 0 || KV <= 0 || max_ctx <= 0) return ZMOE_ERR_ARG;
+    if ((head_dim != 64 && head_dim != 128) || H % KV || H / KV > 32) return ZMOE_ERR_SHAPE;
+    const __half *k = static_cast<const __half *>(k_dev), *v = static_cast<const __half *>(v_dev);
+    const float scale = 1.0f / sqrtf((float)head_dim);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return head_dim == 128 ? launch_attention_prompt<128>(qkv_dev, k, v, out_dev, pos_dev, T, H, KV, scale, max_ctx, st)
+                           : launch_attention_prompt<64>(qkv_dev, k, v, out_dev, pos_dev, T, H, KV, scale, max_ctx, st);
 }
 
 int zmoe_decoder_read(zmoe_decoder *dec, int32_t *next_token_host, int32_t *pos_host, float *logits_host, int n_logits) {
