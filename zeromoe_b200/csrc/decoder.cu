@@ -19,6 +19,7 @@
 #include <cmath>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "quant_units.cuh"
@@ -619,6 +620,7 @@ __global__ void __launch_bounds__(256, 2) attention_prompt_kernel(const float *_
     const int kmax = min(p0 + min(t0 + TQ, T), max_ctx);     // keys any row of the tile sees
     const int share = ((kmax + AP_KEYS - 1) / AP_KEYS + ATTN_SPLITS - 1) / ATTN_SPLITS * AP_KEYS;   // keys of a share: whole tiles
     int share_end = share;
+    const int first_seen = min(p0 + t0 + 1, max_ctx);        // keys every row of the tile sees
     auto load = [&](const __half *src, int k0) {
         for (int i = tid; i < AP_KEYS * (HD / 8); i += 256) {
             const int r = i / (HD / 8), c = i % (HD / 8);
@@ -688,28 +690,37 @@ __global__ void __launch_bounds__(256, 2) attention_prompt_kernel(const float *_
                 for (int j = 0; j < 4; ++j) as[i][h][j] *= corr;
         }
         __syncthreads();
-        // outputs of rows 4 ty + i, dimensions 64 h + 4 tx ..
+        // Outputs of rows 4 ty + i, dimensions 64 h + 4 tx ..  In a tile with keys that some row does not see (masked) such a
+        // key's V does not enter the row at all: its weight is zero, but zero times an infinity is not.
+        auto weigh = [&](auto form) {
+            constexpr bool masked = decltype(form)::value;
+            int seen[4];                          // keys of this tile that row 4 ty + i sees
+#pragma unroll
+            for (int i = 0; i < 4; ++i) seen[i] = masked ? nk_s[4 * ty + i] - k0 : AP_KEYS;
 #pragma unroll 2
-        for (int k = 0; k < AP_KEYS; k += 4) {
-            float4 pr[4];
+            for (int k = 0; k < AP_KEYS; k += 4) {
+                float4 pr[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) pr[i] = *reinterpret_cast<const float4 *>(ps + (4 * ty + i) * AP_PP + k);
+                for (int i = 0; i < 4; ++i) pr[i] = *reinterpret_cast<const float4 *>(ps + (4 * ty + i) * AP_PP + k);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
+                for (int e = 0; e < 4; ++e) {
 #pragma unroll
-                for (int h = 0; h < NV; ++h) {
-                    const float4 v = *reinterpret_cast<const float4 *>(kv + (k + e) * PITCH + 64 * h + 4 * tx);
+                    for (int h = 0; h < NV; ++h) {
+                        const float4 v = *reinterpret_cast<const float4 *>(kv + (k + e) * PITCH + 64 * h + 4 * tx);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float pe = e == 0 ? pr[i].x : e == 1 ? pr[i].y : e == 2 ? pr[i].z : pr[i].w;
-                        as[i][h][0] = fmaf(pe, v.x, as[i][h][0]);
-                        as[i][h][1] = fmaf(pe, v.y, as[i][h][1]);
-                        as[i][h][2] = fmaf(pe, v.z, as[i][h][2]);
-                        as[i][h][3] = fmaf(pe, v.w, as[i][h][3]);
+                        for (int i = 0; i < 4; ++i) {
+                            if (masked && k + e >= seen[i]) continue;
+                            const float pe = e == 0 ? pr[i].x : e == 1 ? pr[i].y : e == 2 ? pr[i].z : pr[i].w;
+                            as[i][h][0] = fmaf(pe, v.x, as[i][h][0]);
+                            as[i][h][1] = fmaf(pe, v.y, as[i][h][1]);
+                            as[i][h][2] = fmaf(pe, v.z, as[i][h][2]);
+                            as[i][h][3] = fmaf(pe, v.w, as[i][h][3]);
+                        }
                     }
                 }
             }
-        }
+        };
+        if (k0 + AP_KEYS > first_seen) weigh(std::true_type()); else weigh(std::false_type());
         if (k0 + AP_KEYS >= share_end || k0 + AP_KEYS >= kmax) {
             share_end += share;
 #pragma unroll
