@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(32 * MM_WARPS) q8_0_matmul_kernel(float *__res
             if (at + 16 <= w_end16) {
                 v = *reinterpret_cast<const uint4 *>(w + at);
             } else {   // the last bytes of the tensor
-                uint8_t tmp[16];
+                __align__(16) uint8_t tmp[16];
                 for (int i = 0; i < 16; ++i) tmp[i] = at + i < w_bytes ? w[at + i] : 0;
                 v = *reinterpret_cast<uint4 *>(tmp);
             }
