@@ -846,6 +846,32 @@ def test_hook_mul_mat_id_chunked_kernel(zlib, oracle, dev, qtype, I, O):
             assert np.all(np.isnan(got[3, 2]))
 
 
+@pytest.mark.parametrize("qtype", TYPES)
+@pytest.mark.parametrize("I,O", [(512, 40), (1536, 64), (4096, 40)])
+def test_hook_mul_mat_id_several_pairs_exact(zlib, oracle, dev, qtype, I, O):
+    """super-scales that are a power of two and activations that Q8_K represents exactly: every product and partial sum is a
+    multiple of one power of two and below 2^24 of it, so whatever the order the f32 result is the exact one, bit for bit.  Experts
+    hold about seven pairs each (the tensor-core consumer path of every format)."""
+    import torch
+    E, K, T = 3, 2, 11
+    rng = synth.rng_for(37, qtype, I)
+    w = synth.expert_weights(qtype, E, O, I, rng)
+    blocks = w.reshape(-1, synth.BLOCK_BYTES[qtype])
+    for off in synth._HALF_FIELDS[qtype]:
+        blocks[:, off:off + 2] = np.array([0.0625], dtype=np.float16).view(np.uint8)
+    x = synth.exact_activations(T, I, rng)
+    ids = np.stack([rng.permutation(E)[:K] for _ in range(T)]).astype(np.int32)
+    ref = np.stack([[oracle.dequantize(qtype, w[e], I).astype(np.float64) @ x[t] for e in ids[t]] for t in range(T)])
+    unit = 0.0625 / (8 if qtype == synth.IQ2_XXS else 1)
+    assert np.array_equal(ref, np.round(ref / unit) * unit) and np.abs(ref).max() < unit * 2 ** 23
+    wd, xd, ids_d = to_dev(w, dev), to_dev(x, dev), to_dev(ids, dev)
+    y = torch.full((T, K, O), 7.0, device=dev)
+    args = _hook_tensors(zlib, qtype, wd, 0, I, O, E, w[0].size, xd, K, T, False, ids_d, y)
+    assert zlib.load().zmoe_f32_quant_hook(*[C.byref(t) for t in args], None, True)
+    _sync()
+    assert np.array_equal(y.cpu().numpy(), ref.astype(np.float32))
+
+
 @pytest.mark.parametrize("T", [1, 19])
 def test_hook_mul_mat_id_strided_slab(zlib, oracle, dev, T):
     """gate|up|down slabs per expert viewed in place: each projection equals the planar
