@@ -9,21 +9,22 @@
 // rows and the same 128 up rows; otherwise rows m0..m0+127 and m0+128..m0+255 of one matrix)
 // against up to 160 pairs; both halves multiply the same activation tile, which halves the
 // activation traffic per flop.
-//   warp 17    loader of the weights: copies the raw quantised super-blocks of the tile's 256 rows, one
+//   warp 0     issues tcgen05.mma (M = 128 weight rows, N = pairs, K = 16 per instruction, A from tensor memory, B from
+//              shared memory) for both halves; tcgen05.commit releases the operand slots.
+//   warp 1     loader of the weights: copies the raw quantised super-blocks of the tile's 256 rows, one
 //              super-block column (256 k) at a time, into a ring in shared memory with tiled copies on the TMA
 //              engine (no multicast), completion on mbarriers.  Rows that are
 //              not multiples of 16 bytes are addressed G rows at a time (G * row bytes is one): G
 //              copies per 128 rows, one per position of a row inside its group.
-//   warp 18    loader of the activations: one tiled copy per 64 k of the rows gathered into expert order, into a
+//   warp 2     loader of the activations: one tiled copy per 64 k of the rows gathered into expert order, into a
 //              ring of its own.
-//   warps 0-15 converters, two groups of eight: a thread reads 64 consecutive weights of one row from shared memory,
+//   warp 3     idle: makes the first converter's number a multiple of four.
+//   warps 4-19 converters, two groups of eight: a thread reads 64 consecutive weights of one row from shared memory,
 //              converts them to fp16 in 32 registers and stores them as its lane of the A operand in tensor memory.
 //              The groups take alternate k-steps, so that one group's loads and conversion overlap the other's
 //              waits, and a group converts before it waits for its operand slot.  The same warps drain the
 //              accumulators of a finished tile (tcgen05.ld, SwiGLU in DUAL mode, f32 stores) while the first k-steps
 //              of the next tile already lie in tensor memory.
-//   warp 16    issues tcgen05.mma (M = 128 weight rows, N = pairs, K = 16 per instruction, A from tensor memory, B from
-//              shared memory) for both halves; tcgen05.commit releases the operand slots.
 //
 // What bounds it.  A from tensor memory: with both operands in shared memory the fp16 weights cost a store and a read there
 // (16 KB each per half tile and k-step), and raw blocks, activations, stores and operand reads together needed more
@@ -35,7 +36,7 @@
 // weight is converted once per pair block).  Measured on one B200 against both operands in shared memory, two slots, 256
 // pairs: 700 tokens of 4096 / 1536, 128 experts, Q2_K gate and up 730 -> 423 us, Q3_K down 422 -> 263; 4096 tokens
 // of IQ2_XXS, skewed load, 1486 -> 1181 and 747 -> 621; 8192 tokens of 7168 / 2048, 256 experts, Q4_K, with a shared
-// expert 6264 -> 4833 and 3080 -> 2633.
+// expert 6264 -> 4776 and 3080 -> 2623.
 // Activations arrive already rounded through Q8_K (value = d * q) as fp16, each row divided by a
 // power of two that brings its largest value near 2^13 (undone exactly in the epilogue), so the
 // result follows the reference CPU path's activation quantisation and cannot overflow fp16;
@@ -57,7 +58,7 @@ constexpr int GEMM_BK = 64;         // k per step: one 128-byte swizzle row of f
 constexpr int GEMM_NB = 4;          // activation slots
 constexpr int GEMM_NRAW = 3;        // raw super-block slots
 constexpr int GEMM_CWARPS = 16;     // converter warps: two groups of eight
-constexpr int GEMM_CW0 = 4;          // first of them; warps 0-2 issue MMAs and copies, warp 3 rounds the CTA up and leaves at once
+constexpr int GEMM_CW0 = 4;          // first of them; warps 0-2 issue MMAs and copies, warp 3 only waits at the last barrier
 constexpr int GEMM_THREADS = 32 * (GEMM_CW0 + GEMM_CWARPS);
 constexpr int GEMM_NA = 3;          // weight slots in tensor memory, 2 x 32 columns each
 constexpr int GEMM_A_COL = 2 * GEMM_BN;   // tensor-memory column of the first of them
@@ -114,7 +115,7 @@ struct GemmParams {
 #endif
 
 // Activation tile maps with boxes of 32, 64, .. 160 rows (a tile loads the smallest box that covers
-// its pairs, so an expert with few pairs does not pull 256 rows through L2 for every k-step) and the
+// its pairs, so an expert with few pairs does not pull 160 rows through L2 for every k-step) and the
 // byte maps [E][O / G][G * rb] of the weight tensors with a box of 128 / G row groups x one raw row pitch.
 struct GemmMaps {
     alignas(64) CUtensorMap box[GEMM_NBOX];

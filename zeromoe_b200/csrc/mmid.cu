@@ -154,7 +154,6 @@ static KernelFn pick_type(int type, int lpr, int upl, bool mma) {
 // The multi-token path splits a tile into 16-row pieces and each piece's row into slices of whole
 // half super-blocks, one slice per warp; it needs every output of a tile to find a thread.
 static bool mma_split(int type, const MmidGeom &g, int I, bool dual, int *ks, int *hpw) {
-    if (type != Q2_K && type != Q3_K && type != Q4_K && type != IQ2_XXS) return false;
     if (g.R % 16 != 0) return false;
     // rows must start on word boundaries, the same for every lane of a fragment load (IQ2_XXS reads any even address)
     if (type != IQ2_XXS && ((I / QK_K) * block_bytes(type)) % 4 != 0) return false;
@@ -250,7 +249,7 @@ int launch_mma_isums(int type, const void *w, const uint8_t *q8, int *out, int I
     case Q2_K: fn = mma_isums_kernel<Q2_K>; break;
     case Q3_K: fn = mma_isums_kernel<Q3_K>; break;
     case Q4_K: fn = mma_isums_kernel<Q4_K>; break;
-    default: return ZMOE_ERR_TYPE;   // no tensor-core consumer path for the type
+    default: return ZMOE_ERR_TYPE;   // IQ2_XXS: mma_rows has no dump of its sums; whole products with exact inputs pin them
     }
     if (raise_dynamic_smem(reinterpret_cast<const void *>(fn), 200 * 1024) != ZMOE_OK) return ZMOE_ERR_CUDA;
     fn<<<1, 32, smem, st>>>(static_cast<const uint8_t *>(w), q8, out, I, pairs, q8s);

@@ -274,12 +274,10 @@ __device__ __forceinline__ void bsum_pair_planes(uint4 w, uint32_t &hi, uint32_t
          ((uint32_t)((s3 >> 7) & 255) << 24);
 }
 
-template <int TYPE> struct MmaPath { static constexpr bool kHas = false; static constexpr int kGrain = 1; };
 // kGrain: half super-blocks a warp's slice must be a multiple of
-template <> struct MmaPath<Q2_K> { static constexpr bool kHas = true; static constexpr int kGrain = 2; };
-template <> struct MmaPath<Q3_K> { static constexpr bool kHas = true; static constexpr int kGrain = 1; };
-template <> struct MmaPath<IQ2_XXS> { static constexpr bool kHas = true; static constexpr int kGrain = 1; };
-template <> struct MmaPath<Q4_K> { static constexpr bool kHas = true; static constexpr int kGrain = 2; };
+template <int TYPE> struct MmaPath { static constexpr int kGrain = 1; };
+template <> struct MmaPath<Q2_K> { static constexpr int kGrain = 2; };
+template <> struct MmaPath<Q4_K> { static constexpr int kGrain = 2; };
 
 // Rows g and g+8 of a 16-row slice against the item's pairs over half-blocks [hb0, hb1): the f32 sums of
 // (row g, pair 2c), (row g, pair 2c+1), (row g+8, pair 2c), (row g+8, pair 2c+1) are added into f0 (tile0)

@@ -23,7 +23,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // ---- operand descriptors --------------------------------------------------------------
 // K-major 16-bit tile stored as rows of 64 elements (128 bytes) with the 128-byte swizzle:
@@ -40,9 +39,6 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
     d |= (uint64_t)2 << 61;
     return d;
 }
-__host__ __device__ constexpr uint32_t swz128_offset(int r, int k) {
-    return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((((k >> 3) ^ (r & 7)) & 7) << 4) + (k & 7) * 2);
-}
 
 // instruction descriptor, kind::f16: f32 accumulate (bits 4-5 = 1), A and B fp16 (bits 7-9 and
 // 10-12 = 0; 1 would be bf16), both K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at
@@ -58,17 +54,7 @@ __device__ __forceinline__ bool elect_one() {
     return one != 0;
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by one thread
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                          uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// The same with A in tensor memory: lane = row of A, a 32-bit column holds two consecutive k, so a k-step of 16
+// D[tmem] (+)= A[tmem] * B[smem]; issued by one thread.  A: lane = row, a 32-bit column holds two consecutive k, so a k-step of 16
 // advances the address by 8 columns
 __device__ __forceinline__ void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                              uint32_t accumulate) {
