@@ -135,8 +135,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) router_decode_kernel(const Rou
                a.plan.freq, a.plan.aoffs, a.plan.antok, a.nrt_gu, a.nrt_dn, a.plan.pos, a.plan.mt_gu, a.plan.mt_dn};
     // the routing scratch at the start of dyn is free again: 2 * NW * E words, NW * E of them for the planner's counts
     const int nfill = plan_runs(a.T * a.K, NW);
-    if (nfill == 1) build_plan_cta<PLAN_ONE_RUN>(a.ids, a.T * a.K, a.E, po, cnt_s, pre_s, ids_s, nullptr, 1);
-    else build_plan_cta<PLAN_RUNS>(a.ids, a.T * a.K, a.E, po, cnt_s, pre_s, ids_s, reinterpret_cast<int *>(dyn), nfill);
+    build_plan_cta<PLAN_RUNS, false>(a.ids, a.T * a.K, a.E, po, cnt_s, pre_s, ids_s, reinterpret_cast<int *>(dyn), nfill);
     if (tid == 0 && n_tg > 1) a.ticket[0] = 0u;
 #ifdef ZMOE_GEMM_STATS
     // phases of the CTA that ends the kernel, in ns: logits + quantise, ticket, routing, ticket, plan; calls

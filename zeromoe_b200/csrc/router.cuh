@@ -171,7 +171,10 @@ __host__ __device__ inline int plan_runs(int P, int most) {
 // nfill * E ints, nfill a number of the CTA's warps.
 // ids: [T*K] (entries outside [0,E) are skipped: negative = inactive route,
 // reference backends/ggml/mmid_route_skip.hpp:60-67).
-template <PlanFill FILL>
+// AHEAD: the runs' loads are on their way before they are used.  The decode router takes PLAN_RUNS without it for any number of
+// pairs: with a second fill in that kernel a layer of 2048 / 768 with 64 tokens took 139 us instead of 134, although the
+// router alone was no slower (16 tokens of 4096 / 1536 gained 1 us of 172).
+template <PlanFill FILL, bool AHEAD = true>
 __device__ __forceinline__ void build_plan_cta(const int32_t *ids, int P, int E, const PlanOut &po, int *cnt_s, int *pre_s,
                                                int *ids_s, int *wcnt_s, int nfill) {
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
@@ -191,12 +194,13 @@ __device__ __forceinline__ void build_plan_cta(const int32_t *ids, int P, int E,
         p_hi = warp < nfill ? min(P, p_lo + run_len) : p_lo;
         for (int i = tid; i < nfill * E; i += nt) wcnt_s[i] = 0;
         __syncthreads();
-        for (int p0 = p_lo + lane; p0 < p_hi; p0 += 128) {
-            int e[4];                                  // four loads on their way at once
+        constexpr int W = AHEAD ? 4 : 1;               // loads on their way at once
+        for (int p0 = p_lo + lane; p0 < p_hi; p0 += 32 * W) {
+            int e[W];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) e[i] = p0 + 32 * i < p_hi ? ids[p0 + 32 * i] : -1;
+            for (int i = 0; i < W; ++i) e[i] = p0 + 32 * i < p_hi ? ids[p0 + 32 * i] : -1;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < W; ++i) {
                 if (ids_s && p0 + 32 * i < p_hi) ids_s[p0 + 32 * i] = e[i];
                 if (e[i] >= 0 && e[i] < E) atomicAdd(&wcnt_s[warp * E + e[i]], 1);
             }
@@ -281,10 +285,10 @@ __device__ __forceinline__ void build_plan_cta(const int32_t *ids, int P, int E,
     // one warp for all pairs P / 32 of them.)
     const int *src = ids_s ? ids_s : ids;
     int *cur = FILL == PLAN_ONE_RUN ? pre_s : wcnt_s + warp * E;
-    int ahead = p_lo + lane < p_hi ? src[p_lo + lane] : -1;    // the next step's load flies during this step
+    int ahead = AHEAD && p_lo + lane < p_hi ? src[p_lo + lane] : -1;   // the next step's load flies during this step
     for (int p0 = p_lo; p0 < p_hi; p0 += 32) {
-        const int p = p0 + lane, e = ahead;
-        ahead = p + 32 < p_hi ? src[p + 32] : -1;
+        const int p = p0 + lane, e = AHEAD ? ahead : p < p_hi ? src[p] : -1;
+        if (AHEAD) ahead = p + 32 < p_hi ? src[p + 32] : -1;
         const bool on = e >= 0 && e < E;
         const unsigned peers = __match_any_sync(0xffffffffu, on ? e : -1 - lane);
         const int leader = __ffs(peers) - 1;
