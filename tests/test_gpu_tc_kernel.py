@@ -1,0 +1,89 @@
+"""The integer tensor-core MUL_MAT_ID kernel (csrc/mmid_tc.cuh) at the sizes where it can go wrong: pairs per expert around its tiles of
+16 columns and its limit of 64 per item, rows of an odd number of super-blocks (a raw chunk that is half full, groups of two, four
+and eight rows per copy), gate and up of one type or two."""
+import numpy as np
+import pytest
+
+from helpers import REL_TO_NORM, TYPES, rel_to_norm, to_dev
+from zeromoe_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+COUNTS = [1, 8, 15, 16, 17, 33, 48, 49, 64, 65, 0, 97, 2]      # pairs of each expert
+
+
+def _layer(zlib, dev, types, D, F, T, rng):
+    E = len(COUNTS)
+    w = [synth.expert_weights(t, E, o, i, rng) for t, o, i in ((types[0], F, D), (types[1], F, D), (types[2], D, F))]
+    ctx = zlib.Context(T, D, F, E, 1)
+    return ctx, zlib.Layer(ctx, D, F, E, 1, types, *[to_dev(a, dev) for a in w]), w
+
+
+def _ffn(zlib, dev, ctx, layer, x, ids, path):
+    import torch
+    T = x.shape[0]
+    out = torch.full((T, x.shape[1]), float("nan"), device=dev)
+    ctx.set_path(path)
+    layer.set_routes(to_dev(x, dev), to_dev(ids, dev), to_dev(np.ones((T, 1), np.float32), dev))
+    layer.expert_ffn(out)
+    torch.cuda.synchronize()
+    ctx.check()
+    return out.cpu().numpy(), ctx.act(T, layer.d_ff)
+
+
+@pytest.mark.parametrize("types", [(t, t, d) for t in (synth.Q2_K, synth.Q3_K, synth.IQ2_XXS) for d in TYPES if t == d or t == synth.Q2_K] +
+                         [(synth.Q2_K, synth.Q4_K, synth.Q3_K), (synth.IQ2_XXS, synth.Q3_K, synth.Q4_K), (synth.Q4_K, synth.Q4_K, synth.IQ2_XXS)])
+@pytest.mark.parametrize("D,F", [(1024, 768), (1280, 512), (256, 1536)])
+def test_pairs_per_expert(zlib, oracle, dev, types, D, F):
+    rng = synth.rng_for(71, D, F, *types)
+    T = sum(COUNTS)
+    ids = rng.permutation(np.repeat(np.arange(len(COUNTS)), COUNTS)).astype(np.int32).reshape(T, 1)
+    x = synth.activations(T, D, rng)
+    ctx, layer, w = _layer(zlib, dev, types, D, F, T, rng)
+    got, act = _ffn(zlib, dev, ctx, layer, x, ids, 1)
+    # a row does not depend on the others of its expert: the same bytes in other columns and items
+    order = rng.permutation(T)
+    moved, act_moved = _ffn(zlib, dev, ctx, layer, x[order], ids[order], 1)
+    if synth.Q4_K not in types[:2]:                  # (the other kernel adds up an expert's last pair alone in another order)
+        assert np.array_equal(act_moved.view(np.uint32), act[order].view(np.uint32))
+        if types[2] != synth.Q4_K:
+            assert np.array_equal(moved.view(np.uint32), got[order].view(np.uint32))
+    some = np.sort(rng.permutation(T)[:11])
+    # the same integers pair by pair, added up in f32 in another order: at most 32 roundings of 2^-24 apart per gate and up value.  In
+    # the output an 8-bit step of the SwiGLU rows more, where such a difference moves a value across a rounding boundary.
+    one, act_one = _ffn(zlib, dev, ctx, layer, x, ids, 3)
+    assert rel_to_norm(act, act_one) < 2e-6
+    assert rel_to_norm(got, one) < REL_TO_NORM
+    ref = oracle.moe_ffn(oracle.make_layer(D, F, len(COUNTS), 1, types, *w), x[some], ids[some], np.ones((len(some), 1), np.float32))
+    assert rel_to_norm(got[some], ref) < REL_TO_NORM
+
+
+@pytest.mark.parametrize("qtype", [synth.Q2_K, synth.Q3_K, synth.IQ2_XXS])
+def test_largest_integers(zlib, dev, qtype):
+    """blocks of the largest and smallest quants and scales against activations of +-127: integer sums at the ends of their ranges.
+    Scales are powers of two, so the only roundings are those of sums above 2^24 (two f32 roundings per gate and up value)."""
+    import torch
+    D = F = 512
+    rng = synth.rng_for(72, qtype)
+    T, E, bb = 40, 2, synth.BLOCK_BYTES[qtype]
+    b = synth.random_blocks(qtype, E * F * (D // 256), rng).reshape(-1, bb)
+    b[::2] = 0xFF
+    b[1::4] = 0x00
+    for a in {synth.Q2_K: (80, 82), synth.Q3_K: (108,), synth.IQ2_XXS: (0,)}[qtype]:
+        b[:, a:a + 2] = np.frombuffer(np.float16(2.0 ** -6).tobytes(), np.uint8)
+    w = to_dev(b.reshape(E, F, -1), dev)
+    wd = to_dev(synth.expert_weights(qtype, E, D, F, rng), dev)
+    x = rng.choice([-127.0, 127.0], size=(T, D)).astype(np.float32)
+    x[::3] = 127.0
+    ids = (np.arange(T) % E).astype(np.int32).reshape(T, 1)
+    acts = []
+    for path in (1, 3):
+        ctx = zlib.Context(T, D, F, E, 1)
+        ctx.set_path(path)
+        layer = zlib.Layer(ctx, D, F, E, 1, (qtype,) * 3, w, w, wd)
+        layer.set_routes(to_dev(x, dev), to_dev(ids, dev), to_dev(np.ones((T, 1), np.float32), dev))
+        layer.expert_ffn(torch.empty((T, D), device=dev))
+        torch.cuda.synchronize()
+        ctx.check()
+        acts.append(ctx.act(T, F))
+    np.testing.assert_allclose(acts[0], acts[1], rtol=1e-6, atol=0)

@@ -132,22 +132,23 @@ struct zmoe_ctx {
     cudaStream_t host_stream = nullptr;
     int *err_host = nullptr;   // pinned mirror of err: the host entry reads the flag with the same sync as its output
     int routed_t = -1;  // tokens of the current route table
-    bool plan_small = false;  // the current plan's items are those of the layer's `small` kernel set
+    int plan_path = 0;        // `path` when the current plan was made: the kernels it was made for depend on it
 };
 
 struct zmoe_layer {
     zmoe_ctx *ctx;
     zmoe_layer_desc d;
-    // Geometries, tile maps and item spaces of the decode kernels.  Two sets: `big` (the K-chunked kernel where
-    // the shapes allow it) and `small` (the kernel whose whole CTA works on one 16-row item: shorter latency
-    // when there are fewer items than warp sets to give them to).  The plan of a call is built for one of them.
+    // Geometries, tile maps and item spaces of the decode kernels.  Three sets: `big` (the K-chunked kernel where
+    // the shapes allow it), `small` (the kernel whose whole CTA works on one 16-row item: shorter latency
+    // when there are fewer items than warp sets to give them to) and `tc` (integers on the tensor cores).  The plan of a call is
+    // built for one of them per projection (call_geom).
     struct Proj {
         MmidGeom g_gu, g_gate1, g_dn;
         CUtensorMap tm_gate, tm_up, tm_down;
         bool has_tm_gu = false, has_tm_dn = false;
         int nrt_gu = 0, nrt_dn = 0;
         int mt_gu = 4, mt_dn = 4;   // pairs per item of the two projections
-    } big, small;
+    } big, small, tc;
     bool dual;
     size_t bytes_gate, bytes_up, bytes_down;
 };
@@ -166,6 +167,41 @@ int layer_route_table(zmoe_layer *L, const int32_t **ids_dev, const float **weig
 zmoe_ctx *layer_context(zmoe_layer *L) { return L ? L->ctx : nullptr; }
 int context_path(const zmoe_ctx *c) { return c ? c->path : 0; }
 }  // namespace zmoe
+
+// The kernel of one projection of a call of T tokens: the integer tensor-core kernel (mmid_tc.cuh) from so many pairs per expert on,
+// on average, that its one conversion of a weight for up to 64 pairs pays; below, the kernels that convert it for up to eight (six) pairs
+// and keep more of the machine busy with few.  A layer of 4096 / 1536, 128 experts, us, that kernel against those before it:
+//   IQ2_XXS  8 tokens 247 / 265, 61 547 / 853, 256 688 / 2641; 2048 / 768: 8 tokens 96 / 111, 40 175 / 303, 200 228 / 1022
+//   Q3_K     (gate and up have no chunk geometry at 4096) 24 tokens 383 / 401, 61 499 / 717, 256 647 / 2172
+//   Q2_K gate and up, Q3_K down  61 tokens 312 / 312 (neither taken), 100 348 / 383 (down), 230 569 / 704 (both), 350 665 / 1000
+static bool takes_tc(int type, const MmidGeom &other, long P, int E) {
+    switch (type) {
+    case IQ2_XXS: return 2 * P >= E;
+    case Q3_K: return other.v2 ? P >= 5L * E : 2 * P >= 3L * E;
+    case Q2_K: return P >= 14L * E;
+    default: return false;
+    }
+}
+
+struct CallGeom {
+    const zmoe_layer::Proj *gu, *dn;    // the sets the two projections' kernels come from
+    int mt_gu, mt_dn, nrt_gu, nrt_dn;   // pairs per item, row tiles per expert
+};
+// the kernels of a call of T tokens.  path: what the context was set to when the routes were made
+static CallGeom call_geom(const zmoe_layer *L, int T, int path) {
+    const long P = (long)T * L->d.topk;
+    const int E = L->d.n_experts;
+    CallGeom g;
+    g.gu = g.dn = P <= kSmallCallPairs ? &L->small : &L->big;
+    if (P > kSmallCallPairs && path != 3) {
+        if (L->tc.has_tm_gu && takes_tc(L->d.gate.type, L->big.g_gu, P, E) && takes_tc(L->d.up.type, L->dual ? L->big.g_gu : L->big.g_gate1, P, E)) g.gu = &L->tc;
+        if (L->tc.has_tm_dn && takes_tc(L->d.down.type, L->big.g_dn, P, E)) g.dn = &L->tc;
+    }
+    g.mt_gu = g.gu->mt_gu; g.mt_dn = g.dn->mt_dn; g.nrt_gu = g.gu->nrt_gu; g.nrt_dn = g.dn->nrt_dn;
+    if (g.gu == &L->tc) g.mt_gu = tc_maxtok(T);
+    if (g.dn == &L->tc) g.mt_dn = tc_maxtok(T);
+    return g;
+}
 
 extern "C" {
 
@@ -299,6 +335,19 @@ static int build_proj(const zmoe_layer_desc &d, bool dual, bool allow_v2, zmoe_l
     return ZMOE_OK;
 }
 
+// the same for the integer tensor-core kernel: which of the two item spaces have it
+static void build_tc(const zmoe_layer_desc &d, bool dual, zmoe_layer::Proj *P) {
+    const int D = d.d_model, F = d.d_ff, E = d.n_experts;
+    auto rb = [](int type, int I) { return (I / QK_K) * block_bytes(type); };
+    P->has_tm_gu = tc_geometry(d.gate.type, D, F, dual, &P->g_gu) == ZMOE_OK && tc_geometry(d.up.type, D, F, dual, &P->g_gate1) == ZMOE_OK &&
+                   make_tc_map(&P->tm_gate, d.gate.data_dev, E, F, rb(d.gate.type, D), d.gate.expert_stride, P->g_gu.pitch, P->g_gu.g_log2) == ZMOE_OK &&
+                   make_tc_map(&P->tm_up, d.up.data_dev, E, F, rb(d.up.type, D), d.up.expert_stride, P->g_gate1.pitch, P->g_gate1.g_log2) == ZMOE_OK;
+    P->has_tm_dn = tc_geometry(d.down.type, F, D, false, &P->g_dn) == ZMOE_OK &&
+                   make_tc_map(&P->tm_down, d.down.data_dev, E, D, rb(d.down.type, F), d.down.expert_stride, P->g_dn.pitch, P->g_dn.g_log2) == ZMOE_OK;
+    if (P->has_tm_gu) P->nrt_gu = (F + P->g_gu.R - 1) / P->g_gu.R;
+    if (P->has_tm_dn) P->nrt_dn = (D + P->g_dn.R - 1) / P->g_dn.R;
+}
+
 int zmoe_layer_create(zmoe_ctx *ctx, const zmoe_layer_desc *desc, zmoe_layer **out) {
     if (!ctx || !desc || !out) return ZMOE_ERR_ARG;
     const zmoe_layer_desc &d = *desc;
@@ -329,10 +378,7 @@ int zmoe_layer_create(zmoe_ctx *ctx, const zmoe_layer_desc *desc, zmoe_layer **o
         delete L;
         return rc;
     }
-    if (rc) {
-        delete L;
-        return rc;
-    }
+    build_tc(d, L->dual, &L->tc);
     *out = L;
     return ZMOE_OK;
 }
@@ -378,10 +424,10 @@ int zmoe_route(zmoe_layer *L, const float *x_dev, int T, void *stream) {
     a.q8_layout = q8_layout_of(L->d.gate.type);
     a.plan = c->plan.b;
     a.stats = gemm_stats_buffer(0);
-    c->plan_small = (long)T * L->d.topk <= kSmallCallPairs;
-    const zmoe_layer::Proj &ps = c->plan_small ? L->small : L->big;
-    a.plan.mt_gu = ps.mt_gu; a.plan.mt_dn = ps.mt_dn;
-    a.nrt_gu = ps.nrt_gu; a.nrt_dn = ps.nrt_dn;
+    c->plan_path = c->path;
+    const CallGeom cg = call_geom(L, T, c->path);
+    a.plan.mt_gu = cg.mt_gu; a.plan.mt_dn = cg.mt_dn;
+    a.nrt_gu = cg.nrt_gu; a.nrt_dn = cg.nrt_dn;
     a.ticket = c->ticket;
     a.logits_part = c->logits_part;
     a.logits_part_rows = router_part_rows(c->max_t) * c->max_e / L->d.n_experts;
@@ -414,12 +460,12 @@ static int set_routes_impl(zmoe_layer *L, const float *x_dev, const int32_t *ids
     if (!takes_gemm(L, T)) rc = quantize_input(L, x_dev, T, st);   // the tensor-core path quantises while it gathers
     // the planner takes the routes in (copy, window mapping) before it groups them: one launch
     PlanBuffers pb = c->plan.b;
-    c->plan_small = (long)P <= kSmallCallPairs;
-    const zmoe_layer::Proj &ps = c->plan_small ? L->small : L->big;
-    pb.mt_gu = ps.mt_gu; pb.mt_dn = ps.mt_dn;
+    c->plan_path = c->path;
+    const CallGeom cg = call_geom(L, T, c->path);
+    pb.mt_gu = cg.mt_gu; pb.mt_dn = cg.mt_dn;
     if (!rc)
         rc = launch_plan_ingest(ids_dev, weights_dev, c->ids, c->weights, (int)P, L->d.n_experts, first_expert, window,
-                                pb, ps.nrt_gu, ps.nrt_dn, st, ids_ld ? L->d.topk : 0, ids_ld, w_ld);
+                                pb, cg.nrt_gu, cg.nrt_dn, st, ids_ld ? L->d.topk : 0, ids_ld, w_ld);
     if (!rc) { g_launches += 1; c->routed_t = T; c->x_last = x_dev; }
     return rc;
 }
@@ -503,7 +549,9 @@ int zmoe_expert_ffn_events(zmoe_layer *L, float *out_dev, int T, int accumulate,
         rc = quantize_input(L, c->x_last, T, st);
         if (rc) return rc;
     }
-    const zmoe_layer::Proj &ps = c->plan_small ? L->small : L->big;   // the set the plan was built for
+    const CallGeom cg = call_geom(L, T, c->plan_path);       // what the plan was built for
+    m.plan.mt_gu = cg.mt_gu; m.plan.mt_dn = cg.mt_dn;
+    const zmoe_layer::Proj &ps = *cg.gu, &pd = *cg.dn;
     if (ev_before) cudaEventRecord(static_cast<cudaEvent_t>(ev_before), st);
     if (L->dual) {
         m.type = d.gate.type; m.dual = true;
@@ -524,11 +572,11 @@ int zmoe_expert_ffn_events(zmoe_layer *L, float *out_dev, int T, int accumulate,
         m.I = d.d_model; m.O = d.d_ff; m.q8 = c->q8x; m.xdiv = d.topk; m.ldy = d.d_ff; m.down = false;
         m.type = d.up.type; m.w0 = d.up.data_dev; m.stride0 = d.up.expert_stride; m.total0 = L->bytes_up; m.y = ubuf;
         if (q8_layout_of(d.up.type) != q8_layout_of(d.gate.type)) m.q8 = c->q8x2;
-        m.tm0 = ps.g_gate1.v2 && ps.g_gate1.tiled ? &ps.tm_up : nullptr;
+        m.tm0 = ps.g_gate1.tc || (ps.g_gate1.v2 && ps.g_gate1.tiled) ? &ps.tm_up : nullptr;
         rc = launch_mmid(m, ps.g_gate1, st);
         m.q8 = c->q8x;
         m.type = d.gate.type; m.w0 = d.gate.data_dev; m.stride0 = d.gate.expert_stride; m.total0 = L->bytes_gate; m.y = gbuf;
-        m.tm0 = ps.g_gu.v2 && ps.g_gu.tiled ? &ps.tm_gate : nullptr;
+        m.tm0 = ps.g_gu.tc || (ps.g_gu.v2 && ps.g_gu.tiled) ? &ps.tm_gate : nullptr;
         if (!rc) rc = launch_mmid(m, ps.g_gu, st);
         m.tm0 = nullptr;
         if (!rc) {
@@ -548,8 +596,8 @@ int zmoe_expert_ffn_events(zmoe_layer *L, float *out_dev, int T, int accumulate,
         m.q8 = c->q8act; m.xdiv = 1;
         m.y = c->ydown; m.ldy = d.d_model;
         m.down = true;
-        if (ps.has_tm_dn) m.tm0 = &ps.tm_down;
-        rc = launch_mmid(m, ps.g_dn, st);
+        if (pd.has_tm_dn) m.tm0 = &pd.tm_down;
+        rc = launch_mmid(m, pd.g_dn, st);
     }
     if (!rc) rc = launch_combine(out_dev, c->ydown, c->weights, c->ids, T, d.topk, d.d_model, d.n_experts, accumulate, st);
     g_launches += 3;

@@ -301,6 +301,21 @@ int make_chunk_map(CUtensorMap *m, const void *base, int E, int O, int rb, size_
     return r == CUDA_SUCCESS ? ZMOE_OK : ZMOE_ERR_CUDA;
 }
 
+int make_tc_map(CUtensorMap *m, const void *base, int E, int O, int rb, size_t expert_stride, int pitch, int g_log2) {
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return ZMOE_ERR_CUDA;
+    const int G = 1 << g_log2;
+    if ((G * rb) % 16 || expert_stride % 16 || pitch % 16 || pitch > 256 || O % G || g_log2 > 3) return ZMOE_ERR_SHAPE;
+    const cuuint64_t dims[3] = {(cuuint64_t)G * rb, (cuuint64_t)(O / G), (cuuint64_t)E};
+    const cuuint64_t strides[2] = {(cuuint64_t)G * rb, (cuuint64_t)expert_stride};
+    const cuuint32_t box[3] = {(cuuint32_t)pitch, (cuuint32_t)(64 / G), 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? ZMOE_OK : ZMOE_ERR_CUDA;
+}
+
 int launch_gemm_sm100(const GemmLaunch &L, cudaStream_t st) {
     if (!gemm_sm100_supported(L.type, L.I, L.O)) return ZMOE_ERR_SHAPE;
     GemmFn fn = nullptr;

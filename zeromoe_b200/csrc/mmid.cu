@@ -257,6 +257,7 @@ int launch_mma_isums(int type, const void *w, const uint8_t *q8, int *out, int I
 }
 
 int launch_mmid(const MmidLaunch &L, const MmidGeom &g, cudaStream_t st) {
+    if (g.tc) return launch_mmid_tc(L, g, st);
     if (g.v2) return launch_mmid2(L, g, st);
     int mma_ks = 0, mma_hpw = 0;
     const bool mma = L.multi && mma_split(L.type, g, L.I, L.dual, &mma_ks, &mma_hpw);

@@ -1,0 +1,96 @@
+// mmid_tc.cu -- geometry and launch of the integer tensor-core MUL_MAT_ID kernel.
+#include <mutex>
+#include <set>
+
+#include "mmid_tc.cuh"
+#include "zmoe_internal.h"
+
+namespace zmoe {
+
+int tc_maxtok(int T) {
+    const int room = T <= 0 ? 16 : (T + 15) & ~15;
+    return room < TC_BN ? room : TC_BN;
+}
+
+int tc_geometry(int type, int I, int O, bool dual, MmidGeom *g) {
+    const int bb = block_bytes(type);
+    if (bb == 0 || type == Q4_K) return ZMOE_ERR_TYPE;
+    if (I <= 0 || O <= 0 || I % QK_K) return ZMOE_ERR_SHAPE;
+    const int nb = I / QK_K, rb = nb * bb;
+    int gl = 0;
+    while (((rb << gl) & 15) != 0) ++gl;              // rb is even: at most three
+    if (O % (1 << gl)) return ZMOE_ERR_SHAPE;
+    // two super-blocks per raw chunk: the window that holds a chunk of any row of
+    // a group, from the 16-byte boundary at or below its start, an odd number of 16-byte pieces wide so that 128-bit loads of
+    // consecutive rows fall into different banks
+    const int cbl = nb == 1 ? 0 : 1, cbytes = bb << cbl;
+    int step = 16;                                    // every offset is a multiple of it
+    while ((rb | cbytes) % step) step /= 2;
+    int pitch = (cbytes + 16 - step + 15) & ~15;
+    if ((pitch / 16) % 2 == 0) pitch += 16;
+    *g = MmidGeom();
+    g->tc = 1; g->g_log2 = gl; g->cb_log2 = cbl; g->pitch = pitch;
+    g->R = dual ? 64 : 128;
+    g->maxtok = TC_BN;
+    return ZMOE_OK;
+}
+
+using KernelTcFn = void (*)(const TcParams);
+
+static bool tc_regs_ok(KernelTcFn fn) {
+    static std::mutex mu;
+    static std::set<KernelTcFn> seen;
+    std::lock_guard<std::mutex> lock(mu);
+    if (seen.count(fn)) return true;
+    cudaFuncAttributes at;
+    if (cudaFuncGetAttributes(&at, fn) != cudaSuccess || at.numRegs != TC_REGS) return false;
+    seen.insert(fn);
+    return true;
+}
+
+int launch_mmid_tc(const MmidLaunch &L, const MmidGeom &g, cudaStream_t st) {
+    KernelTcFn fn = nullptr;
+    switch (L.type) {
+    case Q2_K: fn = L.dual ? mmid_tc_kernel<Q2_K, true> : mmid_tc_kernel<Q2_K, false>; break;
+    case Q3_K: fn = L.dual ? mmid_tc_kernel<Q3_K, true> : mmid_tc_kernel<Q3_K, false>; break;
+    case IQ2_XXS: fn = L.dual ? mmid_tc_kernel<IQ2_XXS, true> : mmid_tc_kernel<IQ2_XXS, false>; break;
+    default: return ZMOE_ERR_TYPE;
+    }
+    if ((reinterpret_cast<size_t>(L.w0) & 15) || (L.dual && (reinterpret_cast<size_t>(L.w1) & 15))) return ZMOE_ERR_ALIGN;
+    if (!L.tm0 || (L.dual && !L.tm1)) return ZMOE_ERR_ARG;
+    const int mt = L.down ? L.plan.mt_dn : L.plan.mt_gu;
+    if (mt < 1 || mt > TC_BN) return ZMOE_ERR_ARG;
+    TcParams p;
+    p.bnr = (mt + 15) & ~15;
+    p.mt = mt;
+    p.nbuf = p.bnr <= 32 ? 4 : 2;   // what the accumulator columns hold (TcGeom::kAcc)
+    // 227 KB per CTA less the kernel's static arrays; the raw stages take what the activation slots leave
+    const int avail = 227 * 1024 - (L.type == IQ2_XXS ? 48 : 35) * 1024;
+    const int fixed = 1024 + TC_NB * p.bnr * (256 + 32) + 128 + 64;
+    p.nraw = (avail - fixed) / (128 * g.pitch);
+    if (p.nraw > TC_MAXRAW) p.nraw = TC_MAXRAW;
+    if (p.nraw < 2) return ZMOE_ERR_SHAPE;
+    if (raise_dynamic_smem(reinterpret_cast<const void *>(fn), (size_t)avail) != ZMOE_OK) return ZMOE_ERR_CUDA;
+    // the roles' register shares are drawn from the launch's: a build that has fewer would wait for them without end
+    if (!tc_regs_ok(fn)) return ZMOE_ERR_CUDA;
+    p.I = L.I; p.O = L.O;
+    p.rb = (L.I / QK_K) * block_bytes(L.type);
+    p.g_log2 = g.g_log2; p.cb_log2 = g.cb_log2; p.pitch = g.pitch;
+    p.q8 = L.q8;
+    p.q8_stride = q8row_stride(L.I);
+    p.xdiv = L.xdiv;
+    p.y = L.y; p.ldy = L.ldy;
+    p.plan.hdr = L.plan.hdr; p.plan.active = L.plan.active; p.plan.offs = L.plan.offs; p.plan.slot = L.plan.slot;
+    p.plan.item_offs = L.down ? L.plan.item_offs_dn : L.plan.item_offs_gu;
+    p.plan.aoffs = L.plan.aoffs; p.plan.antok = L.plan.antok; p.plan.cap_e = L.plan.cap_e;
+    p.hdr_items = L.down ? 2 : 1;
+    p.clamp = L.clamp; p.clamp_fused = L.clamp_fused;
+    p.err = L.err;
+    p.bad = L.dual ? L.bad : nullptr;
+    p.tm0 = *L.tm0;
+    p.tm1 = L.dual ? *L.tm1 : *L.tm0;
+    return launch_pdl(fn, dim3(L.n_sm), dim3(TC_THREADS), (size_t)fixed + (size_t)p.nraw * 128 * g.pitch, st, p) == cudaSuccess
+               ? ZMOE_OK : ZMOE_ERR_CUDA;
+}
+
+}  // namespace zmoe

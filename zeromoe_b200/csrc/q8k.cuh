@@ -51,9 +51,15 @@ __device__ __forceinline__ void quantize_block_q8k(const float *__restrict__ src
     *reinterpret_cast<uint2 *>(row_out + q8row_elem_off(layout, b, 8 * lane)) = packed;
     int s = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
     s += __shfl_xor_sync(0xffffffffu, s, 1);
-    if ((lane & 1) == 0)
-        *reinterpret_cast<int16_t *>(row_out + q8_bs_off(b) + 2 * (lane >> 1)) = (int16_t)s;
-    if (lane == 0) *reinterpret_cast<float *>(row_out + q8_d_off(b)) = d;
+    const int g = lane >> 1;
+    if ((lane & 1) == 0) {
+        *reinterpret_cast<int16_t *>(row_out + q8_bs_off(b) + 2 * g) = (int16_t)s;
+        *reinterpret_cast<__half *>(row_out + q8_bs16_off(layout, b, g)) = __int2half_rn(s);
+    }
+    int all = s;
+#pragma unroll
+    for (int off = 2; off < 32; off <<= 1) all += __shfl_xor_sync(0xffffffffu, all, off);
+    if (lane == 0) *reinterpret_cast<uint2 *>(row_out + q8_d_off(b)) = make_uint2(__float_as_uint(d), (uint32_t)(128 * all));
 }
 
 }  // namespace zmoe

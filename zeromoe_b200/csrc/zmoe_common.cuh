@@ -21,7 +21,7 @@ __host__ __device__ constexpr int block_bytes(int type) {
 // ---------------------------------------------------------------------------
 // Packed activation rows.  One Q8_K-quantised row of I elements is stored block by
 // block, every super-block a record of 368 bytes:
-//   [ 4 units x 80 bytes | float d (padded to 16 B) | int16 bsums[16] ]
+//   [ 4 units x 80 bytes | float d, int 128 * sum (padded to 16 B) | int16 bsums[16] ]
 // so that one bulk copy brings a row -- or the slice of a row that a chunk of weight
 // blocks meets -- to shared memory.
 // Same numbers as the 292-byte ggml block (reference backends/cpu/kernels_cpu.cpp:22-26),
@@ -42,6 +42,12 @@ enum Q8Layout : int { Q8_LINEAR = 0, Q8_PLANAR = 1 };
 __host__ __device__ inline int q8_unit_off(int u) { return (u >> 2) * Q8_BLOCK_STRIDE + (u & 3) * Q8_UNIT_STRIDE; }
 __host__ __device__ inline int q8_d_off(int b) { return b * Q8_BLOCK_STRIDE + Q8_BLOCK_D; }
 __host__ __device__ inline int q8_bs_off(int b) { return b * Q8_BLOCK_STRIDE + Q8_BLOCK_BS; }
+// What the integer tensor-core kernel wants of a block lies in the padding: group sum g (of sixteen) once more as fp16, eight behind each of
+// the first two units, in the order that kernel's A operand has them; and 128 times the block's sum as an int behind d.
+__host__ __device__ inline int q8_bs16_off(int layout, int b, int g) {
+    const int at = layout == Q8_PLANAR ? (g & 4) | ((g & 1) << 1) | ((g >> 1) & 1) : g & 7;
+    return b * Q8_BLOCK_STRIDE + (g >> 3) * Q8_UNIT_STRIDE + 64 + 2 * at;
+}
 __host__ __device__ inline int q8row_stride(int I) { return (I / QK_K) * Q8_BLOCK_STRIDE; }
 __host__ __device__ constexpr int q8_layout_of(int type) { return (type == Q2_K || type == Q3_K) ? Q8_PLANAR : Q8_LINEAR; }
 // byte offset inside the packed row of element e (0..255) of super-block b

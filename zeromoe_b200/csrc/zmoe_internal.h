@@ -101,12 +101,21 @@ struct MmidGeom {
     int q8s_l = 0;         // bytes between the pairs' activation slices in shared memory
     int maxtok = 4;        // pairs per item (8 where the K-chunked kernel has the tensor-core path and the stages fit)
     int tiled = 0;         // chunks come through tiled maps (make_chunk_map); 0: rows are copied whole as one run
+    // tensor-core kernel (mmid_tc.cuh): tc_geometry fills these, R (rows of one matrix per item) and pitch
+    int tc = 0, g_log2 = 0, cb_log2 = 0;
 };
 // allow_v2: the caller passes maps made by make_chunk_map where g->tiled is set
 int mmid_geometry(int type, int I, int O, bool dual, MmidGeom *g, bool allow_v2 = false);
 // Map of a [E][O rows][rb bytes] weight tensor whose box is 32 rows of `pitch` bytes starting at any multiple of 16
 // bytes inside a row: bytes past the end of a row and rows past the last arrive as zeros.
 int make_chunk_map(CUtensorMap *m, const void *base, int E, int O, int rb, size_t expert_stride, int pitch);
+
+// Geometry of the integer tensor-core kernel for experts that hold several pairs; its maps come from make_tc_map.
+int tc_geometry(int type, int I, int O, bool dual, MmidGeom *g);
+// most pairs per item of that kernel, for calls of T tokens: what a call's plan is built with
+int tc_maxtok(int T);
+// Map of a [E][O rows][rb bytes] weight tensor, G = 2^g_log2 rows at a time (G * rb a multiple of 16): box of 64 / G groups x `pitch` bytes
+int make_tc_map(CUtensorMap *m, const void *base, int E, int O, int rb, size_t expert_stride, int pitch, int g_log2);
 
 struct MmidLaunch {
     int type;
@@ -139,6 +148,7 @@ int launch_widen_bf16(const void *src, float *dst, long n, int n_sm, cudaStream_
 // g[t] = sigmoid(w . x[t]) for T rows of D floats (D a multiple of 4)
 int launch_token_gate(const float *x, const float *w, float *g, int T, int D, cudaStream_t st);
 int launch_mmid(const MmidLaunch &L, const MmidGeom &g, cudaStream_t st);
+int launch_mmid_tc(const MmidLaunch &L, const MmidGeom &g, cudaStream_t st);
 // s32 sums of the tensor-core consumer path: out[16 rows][4 pair slots][I / 256][2]
 int launch_mma_isums(int type, const void *w, const uint8_t *q8, int *out, int I, int pairs, cudaStream_t st);
 
