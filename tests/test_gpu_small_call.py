@@ -1,0 +1,56 @@
+"""Calls of very few pairs, which run a whole MoE layer as one cooperative kernel (csrc/moe_small.cuh), against the router and the experts
+called one after the other: the same routes, the same integers, sums in another f32 order, and the same state left behind."""
+import numpy as np
+import pytest
+
+from helpers import REL_TO_NORM, rel_to_norm, to_dev
+from zeromoe_b200 import synth
+
+pytestmark = pytest.mark.gpu
+Q2, Q3, Q4 = synth.Q2_K, synth.Q3_K, synth.Q4_K
+
+
+@pytest.mark.parametrize("D,F,E,K,T,types,gating", [
+    (2048, 768, 128, 8, 1, (Q4, Q4, Q4), 0),      # the benchmark's small layer
+    (2048, 768, 128, 8, 2, (Q2, Q2, Q3), 0),
+    (256, 256, 3, 2, 1, (Q3, Q3, Q2), 1),         # one super-block per row, fewer experts and outputs than CTAs
+    (512, 1280, 250, 6, 5, (Q4, Q4, Q3), 1),      # rows of Q3_K on odd 2-byte offsets, experts that two tokens share
+    (768, 512, 9, 9, 3, (Q3, Q3, Q4), 0),         # more than eight experts per token, all of them chosen
+    (1024, 256, 16, 1, 16, (Q2, Q2, Q2), 0),      # as many tokens as warps
+])
+def test_one_kernel_against_separate_calls(zlib, dev, D, F, E, K, T, types, gating):
+    import torch
+    rng = synth.rng_for(81, D, F, E, T)
+    w = [to_dev(synth.expert_weights(t, E, o, i, rng), dev) for t, o, i in ((types[0], F, D), (types[1], F, D), (types[2], D, F))]
+    wr = to_dev(synth.router_weights(E, D, rng, sigma=D ** -0.5), dev)
+    bias = to_dev((rng.standard_normal(E) * 0.1).astype(np.float32), dev)
+    x = to_dev(synth.activations(T, D, rng), dev)
+    ctx = zlib.Context(T, D, F, E, K)
+    layer = zlib.Layer(ctx, D, F, E, K, types, *w, router_w=wr, router_bias=bias, gating=gating, weights_scale=1.5)
+    n0 = zlib.load().zmoe_kernel_launches()
+    seen = []
+    for one in (True, False):
+        out = torch.full((T, D), float("nan"), device=dev)
+        if one:
+            layer.forward(x, out)
+            assert zlib.load().zmoe_kernel_launches() == n0 + 1
+        else:
+            layer.route(x)
+            layer.expert_ffn(out)
+        torch.cuda.synchronize()
+        ctx.check()
+        ids, wts = ctx.routes(T, K)
+        seen.append((out.cpu().numpy(), ids, wts, ctx.probs(T, E), ctx.act(T * K, F), ctx.expert_freq(E)))
+        if one:
+            # the plan it leaves serves the experts once more
+            again = torch.ones((T, D), device=dev)
+            layer.expert_ffn(again, accumulate=1)
+            torch.cuda.synchronize()
+            ctx.check()
+            assert rel_to_norm(again.cpu().numpy() - 1.0, seen[0][0]) < REL_TO_NORM
+    a, b = seen
+    assert np.array_equal(a[1], b[1]) and np.array_equal(a[5], b[5])
+    for i in (2, 3):
+        np.testing.assert_allclose(a[i], b[i], rtol=2e-5, atol=1e-7)      # logits of up to 2048 products in another order
+    assert rel_to_norm(a[4], b[4]) < 2e-6
+    assert rel_to_norm(a[0], b[0]) < REL_TO_NORM                          # an 8-bit step of an act value now and then

@@ -128,6 +128,7 @@ struct zmoe_ctx {
     int *bad = nullptr;        // [2] NaN / Inf inputs seen by the fused SwiGLU epilogues
     int *queue = nullptr;      // [4] item tickets of the decode matmuls (two per projection; every launch leaves them zero)
     unsigned *ticket = nullptr;
+    unsigned *small_bar = nullptr;  // [2] grid-barrier counters of the one-kernel layer (every launch leaves them zero)
     float *x_stage = nullptr, *out_stage = nullptr;  // device staging of the host entry
     cudaStream_t host_stream = nullptr;
     int *err_host = nullptr;   // pinned mirror of err: the host entry reads the flag with the same sync as its output
@@ -154,6 +155,17 @@ struct zmoe_layer {
 };
 // calls with at most this many pairs take the `small` set
 static const int kSmallCallPairs = 8;
+// Calls of the whole layer that run as one kernel (moe_small.cuh): the pairs' experts hold at most this many bytes, and no IQ2_XXS, whose
+// one-pair dot is bound by its table lookups.  One kernel saves about 12 us of launches and plans, and its rows come a little slower
+// than those of the kernels it stands for.  us per layer, one kernel / five launches: Q4_K 2048 / 768: one token (21 MB) 23 / 31, two (42 MB)
+// 34 / 39, four (85 MB) 55 / 54; Q2_K and Q3_K 4096 / 1536, one token (55 MB) 44 / 42; Q4_K 7168 / 2048, one token (198 MB) 122 / 102.
+static const size_t kFusedCallBytes = (size_t)48 << 20;
+static bool takes_fused(const zmoe_layer_desc &d, int T) {
+    const size_t gu = (size_t)d.d_ff * (d.d_model / QK_K) * (block_bytes(d.gate.type) + block_bytes(d.up.type));
+    const size_t dn = (size_t)d.d_model * (d.d_ff / QK_K) * block_bytes(d.down.type);
+    if (d.n_experts > 256 || d.n_groups > 1) return false;             // what its router holds in registers
+    return d.gate.type != IQ2_XXS && d.down.type != IQ2_XXS && (size_t)T * d.topk * (gu + dn) <= kFusedCallBytes;
+}
 
 namespace zmoe {
 int layer_route_table(zmoe_layer *L, const int32_t **ids_dev, const float **weights_dev, int *n_experts) {
@@ -237,6 +249,7 @@ int zmoe_ctx_create(int max_tokens, int max_d_model, int max_d_ff, int max_exper
     rc |= dev_alloc(&c->bad, 2);
     rc |= dev_alloc(&c->queue, 4);
     rc |= dev_alloc(&c->ticket, 1 + ROUTER_MAX_GROUPS);
+    rc |= dev_alloc(&c->small_bar, 2);
     rc |= dev_alloc(&c->x_stage, (size_t)max_tokens * max_d_model);
     rc |= dev_alloc(&c->out_stage, (size_t)max_tokens * max_d_model);
     rc |= ok(cudaStreamCreateWithFlags(&c->host_stream, cudaStreamNonBlocking));
@@ -246,6 +259,7 @@ int zmoe_ctx_create(int max_tokens, int max_d_model, int max_d_ff, int max_exper
         rc |= ok(cudaMemset(c->bad, 0, 2 * sizeof(int)));
         rc |= ok(cudaMemset(c->queue, 0, 4 * sizeof(int)));
         rc |= ok(cudaMemset(c->ticket, 0, (1 + ROUTER_MAX_GROUPS) * sizeof(unsigned)));
+        rc |= ok(cudaMemset(c->small_bar, 0, 2 * sizeof(unsigned)));
         rc |= ok(cudaMemset(c->plan.b.hdr, 0, 4 * sizeof(int)));
         rc |= ok(cudaMemset(c->zero_ids, 0, (size_t)max_tokens * sizeof(int32_t)));
         // 1.0f = 0x3f800000: fill through a host staging vector (done once)
@@ -272,7 +286,7 @@ void zmoe_ctx_destroy(zmoe_ctx *c) {
     cudaFree(c->zero_ids); cudaFree(c->one_w); cudaFree(c->gate_s);
     cudaFree(c->xq_f16); cudaFree(c->actq_f16); cudaFree(c->xscale); cudaFree(c->actscale);
     cudaFree(c->q8x); cudaFree(c->q8x2); cudaFree(c->act); cudaFree(c->act2); cudaFree(c->q8act); cudaFree(c->ydown);
-    cudaFree(c->logits); cudaFree(c->logits_part); cudaFree(c->ids); cudaFree(c->weights); cudaFree(c->err); cudaFree(c->bad); cudaFree(c->queue); cudaFree(c->ticket);
+    cudaFree(c->logits); cudaFree(c->logits_part); cudaFree(c->ids); cudaFree(c->weights); cudaFree(c->err); cudaFree(c->bad); cudaFree(c->queue); cudaFree(c->ticket); cudaFree(c->small_bar);
     cudaFree(c->x_stage); cudaFree(c->out_stage);
     c->plan.release();
     if (c->host_stream) cudaStreamDestroy(c->host_stream);
@@ -396,24 +410,26 @@ static bool takes_gemm(const zmoe_layer *L, int T) {
     return gemm_ok && (c->path == 2 || (c->path == 0 && P >= (long)kGemmMinPairsPerExpert * d.n_experts));
 }
 
+// how the quantiser writes rows that meet weights of `type`
+static int q8_rows_for(int type, bool on_tc) { return q8_layout_of(type) | (on_tc ? Q8_FOR_TC : 0); }
+
 // packed Q8_K rows of the layer input for the decode kernels (both unit layouts where gate and up differ)
 static int quantize_input(zmoe_layer *L, const float *x_dev, int T, cudaStream_t st) {
     zmoe_ctx *c = L->ctx;
-    int rc = launch_quantize_rows(x_dev, L->d.d_model, c->q8x, T, L->d.d_model, q8_layout_of(L->d.gate.type), st);
+    const bool on_tc = call_geom(L, T, c->plan_path).gu == &L->tc;
+    int rc = launch_quantize_rows(x_dev, L->d.d_model, c->q8x, T, L->d.d_model, q8_rows_for(L->d.gate.type, on_tc), st);
     g_launches += 1;
     if (!rc && q8_layout_of(L->d.up.type) != q8_layout_of(L->d.gate.type)) {
-        rc = launch_quantize_rows(x_dev, L->d.d_model, c->q8x2, T, L->d.d_model, q8_layout_of(L->d.up.type), st);
+        rc = launch_quantize_rows(x_dev, L->d.d_model, c->q8x2, T, L->d.d_model, q8_rows_for(L->d.up.type, on_tc), st);
         g_launches += 1;
     }
     if (!rc) c->q8x_valid = true;
     return rc;
 }
 
-int zmoe_route(zmoe_layer *L, const float *x_dev, int T, void *stream) {
-    if (!L || !x_dev || T <= 0) return ZMOE_ERR_ARG;
+// the arguments of a router launch for T tokens; sets the kernel set that the plan is built for
+static RouterArgs router_args(zmoe_layer *L, const float *x_dev, int T) {
     zmoe_ctx *c = L->ctx;
-    if (T > c->max_t) return ZMOE_ERR_CAPACITY;
-    if (!L->d.router_w_dev) return ZMOE_ERR_STATE;
     RouterArgs a;
     a.x = x_dev; a.wr = L->d.router_w_dev; a.bias = L->d.router_bias_dev;
     a.T = T; a.D = L->d.d_model; a.E = L->d.n_experts; a.K = L->d.topk;
@@ -421,17 +437,26 @@ int zmoe_route(zmoe_layer *L, const float *x_dev, int T, void *stream) {
     a.weight_scale = L->d.weights_scale;
     a.n_groups = L->d.n_groups; a.n_groups_used = L->d.n_groups_used;
     a.logits = c->logits; a.ids = c->ids; a.weights = c->weights; a.q8x = c->q8x;
-    a.q8_layout = q8_layout_of(L->d.gate.type);
     a.plan = c->plan.b;
     a.stats = gemm_stats_buffer(0);
     c->plan_path = c->path;
     const CallGeom cg = call_geom(L, T, c->path);
+    a.q8_layout = q8_rows_for(L->d.gate.type, cg.gu == &L->tc);
     a.plan.mt_gu = cg.mt_gu; a.plan.mt_dn = cg.mt_dn;
     a.nrt_gu = cg.nrt_gu; a.nrt_dn = cg.nrt_dn;
     a.ticket = c->ticket;
     a.logits_part = c->logits_part;
     a.logits_part_rows = router_part_rows(c->max_t) * c->max_e / L->d.n_experts;
     a.n_sm = c->n_sm;
+    return a;
+}
+
+int zmoe_route(zmoe_layer *L, const float *x_dev, int T, void *stream) {
+    if (!L || !x_dev || T <= 0) return ZMOE_ERR_ARG;
+    zmoe_ctx *c = L->ctx;
+    if (T > c->max_t) return ZMOE_ERR_CAPACITY;
+    if (!L->d.router_w_dev) return ZMOE_ERR_STATE;
+    RouterArgs a = router_args(L, x_dev, T);
     const bool big = router_takes_tiles(T, a.D, a.E);
     // the tensor-core path quantises the rows itself while it gathers them: the large-batch router then skips q8x
     a.want_q8x = !(big && takes_gemm(L, T));
@@ -439,8 +464,8 @@ int zmoe_route(zmoe_layer *L, const float *x_dev, int T, void *stream) {
                  : launch_router_decode(a, static_cast<cudaStream_t>(stream));
     g_launches += big ? (a.want_q8x ? 4 : 3) : 1;
     c->q8x_valid = a.want_q8x;
-    if (!rc && a.want_q8x && q8_layout_of(L->d.up.type) != a.q8_layout) {
-        rc = launch_quantize_rows(x_dev, L->d.d_model, c->q8x2, T, L->d.d_model, q8_layout_of(L->d.up.type),
+    if (!rc && a.want_q8x && q8_layout_of(L->d.up.type) != q8_layout_of(L->d.gate.type)) {
+        rc = launch_quantize_rows(x_dev, L->d.d_model, c->q8x2, T, L->d.d_model, q8_rows_for(L->d.up.type, (a.q8_layout & Q8_FOR_TC) != 0),
                                   static_cast<cudaStream_t>(stream));
         g_launches += 1;
     }
@@ -457,10 +482,10 @@ static int set_routes_impl(zmoe_layer *L, const float *x_dev, const int32_t *ids
     const size_t P = (size_t)T * L->d.topk;
     int rc = 0;
     c->q8x_valid = false;
+    c->plan_path = c->path;
     if (!takes_gemm(L, T)) rc = quantize_input(L, x_dev, T, st);   // the tensor-core path quantises while it gathers
     // the planner takes the routes in (copy, window mapping) before it groups them: one launch
     PlanBuffers pb = c->plan.b;
-    c->plan_path = c->path;
     const CallGeom cg = call_geom(L, T, c->path);
     pb.mt_gu = cg.mt_gu; pb.mt_dn = cg.mt_dn;
     if (!rc)
@@ -586,7 +611,7 @@ int zmoe_expert_ffn_events(zmoe_layer *L, float *out_dev, int T, int accumulate,
         g_launches += 3;
     }
     if (ev_after) cudaEventRecord(static_cast<cudaEvent_t>(ev_after), st);
-    if (!rc) rc = launch_quantize_rows(c->act, d.d_ff, c->q8act, P, d.d_ff, q8_layout_of(d.down.type), st);
+    if (!rc) rc = launch_quantize_rows(c->act, d.d_ff, c->q8act, P, d.d_ff, q8_rows_for(d.down.type, &pd == &L->tc), st);
     if (!rc) {
         m.type = d.down.type; m.dual = false;
         m.w0 = d.down.data_dev; m.w1 = nullptr;
@@ -627,9 +652,7 @@ int zmoe_dense_ffn_gated(zmoe_layer *L, const float *x_dev, const float *gate_w_
 }
 
 int zmoe_moe_forward(zmoe_layer *L, const float *x_dev, float *out_dev, int T, void *stream) {
-    int rc = zmoe_route(L, x_dev, T, stream);
-    if (!rc) rc = zmoe_expert_ffn(L, out_dev, T, 0, stream);
-    return rc;
+    return zmoe::layer_forward(L, x_dev, out_dev, T, 0, stream);
 }
 
 int zmoe_moe_forward_bf16(zmoe_layer *L, const void *x_bf16_dev, float *out_dev, int T, void *stream) {
@@ -657,6 +680,7 @@ int zmoe_moe_forward_host(zmoe_layer *L, const float *x_host, float *out_host, i
     if (!rc && *c->err_host) {
         cudaMemset(c->err, 0, sizeof(int));
         cudaMemset(c->queue, 0, 4 * sizeof(int));   // a launch that gave up may have left its tickets behind
+        cudaMemset(c->small_bar, 0, 2 * sizeof(unsigned));
         rc = ZMOE_ERR_DEVICE_WAIT;
     }
     return rc;
@@ -707,6 +731,7 @@ int zmoe_ctx_check(zmoe_ctx *c) {
     if (e) {
         cudaMemset(c->err, 0, sizeof(int));
         cudaMemset(c->queue, 0, 4 * sizeof(int));   // a launch that gave up may have left its tickets behind
+        cudaMemset(c->small_bar, 0, 2 * sizeof(unsigned));
         return ZMOE_ERR_DEVICE_WAIT;
     }
     return ZMOE_OK;
@@ -731,6 +756,47 @@ int zmoe_debug_gemm_cycles(uint64_t *counters32_host) {
 uint64_t zmoe_kernel_launches(void) { return g_launches.load(); }
 
 }  // extern "C"
+
+bool zmoe::layer_small_args(zmoe_layer *L, const float *x_dev, float *out_dev, int T, int accumulate, RouterArgs *r, SmallLaunch *s) {
+    const zmoe_layer_desc &d = L->d;
+    if (T > L->ctx->max_t || !d.router_w_dev || !L->dual || L->ctx->path >= 2 || !takes_fused(d, T) ||
+        !moe_small_supported(d.gate.type, d.down.type, T, d.d_model, d.d_ff, d.n_experts, d.topk))
+        return false;
+    zmoe_ctx *c = L->ctx;
+    *r = router_args(L, x_dev, T);
+    s->type_gu = d.gate.type; s->type_dn = d.down.type; s->F = d.d_ff;
+    s->w_gate = d.gate.data_dev; s->w_up = d.up.data_dev; s->w_down = d.down.data_dev;
+    s->stride_gate = d.gate.expert_stride; s->stride_up = d.up.expert_stride; s->stride_down = d.down.expert_stride;
+    s->total_gate = L->bytes_gate; s->total_up = L->bytes_up; s->total_down = L->bytes_down;
+    s->clamp = d.swiglu_clamp; s->clamp_fused = d.swiglu_clamp_fused;
+    s->act = c->act; s->out = out_dev; s->accumulate = accumulate;
+    s->err = c->err; s->bad = c->bad; s->bar = c->small_bar;
+    return true;
+}
+
+void zmoe::layer_small_done(zmoe_layer *L, const float *x_dev, int T) {
+    zmoe_ctx *c = L->ctx;
+    c->plan_path = c->path;
+    c->q8x_valid = true;
+    c->routed_t = T;
+    c->x_last = x_dev;
+}
+
+int zmoe::layer_forward(zmoe_layer *L, const float *x_dev, float *out_dev, int T, int accumulate, void *stream) {
+    RouterArgs r;
+    SmallLaunch s;
+    if (L && x_dev && out_dev && T > 0 && layer_small_args(L, x_dev, out_dev, T, accumulate, &r, &s)) {
+        const int rc = launch_moe_small(r, s, static_cast<cudaStream_t>(stream));
+        if (!rc) {
+            g_launches += 1;
+            layer_small_done(L, x_dev, T);
+        }
+        return rc;
+    }
+    int rc = zmoe_route(L, x_dev, T, stream);
+    if (!rc) rc = zmoe_expert_ffn(L, out_dev, T, accumulate, stream);
+    return rc;
+}
 
 // ---------------------------------------------------------------------------
 // per-device scratch of the handle-free entry points

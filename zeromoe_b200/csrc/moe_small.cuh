@@ -1,0 +1,413 @@
+// moe_small.cuh -- a whole MoE layer of very few (token, expert) pairs inside one cooperative kernel: router, top-k, gate / up,
+// SwiGLU, down, weighted sum.
+//
+// Same arithmetic as the five launches it stands for (router_decode_kernel, mmid_kernel twice, quantize_rows_kernel,
+// combine_kernel; reference core/moe_router_service.cpp:1409-1474, core/batched_dispatch_pipeline.cpp:1833-1921,
+// models/graph/moe_routed_ggml.hpp:198-215).  With a pair or two per expert and a few megabytes of weights those launches were bound by
+// their chain: each waits for the one before it to drain, reads its plan, fills its pipeline and drains again.  Here one CTA per SM
+// runs through the phases with grid-wide barriers between them (a cooperative launch, so all CTAs are resident):
+//   1  the CTA's experts' logits for all tokens; the tokens' rows quantised to Q8_K, by every CTA for itself
+//   -- barrier --
+//   2  top-k, by every CTA for itself, one warp per token; then gate / up: a warp takes row r of a pair, its bytes copied to shared
+//      memory by 16-byte asynchronous copies, several rows ahead
+//   -- barrier, with the first down rows already on their way --
+//   3  the pairs' SwiGLU rows quantised, by every CTA for itself; then down: a warp takes output element d of a token, eight lane groups
+//      multiply the rows d of its K experts at once, and the weighted sum in k order needs no other warp
+// Afterwards the context holds what the separate launches leave there: routes, probabilities, SwiGLU rows, quantised input, plan.
+// What other CTAs wrote in the same launch is read past the L1 cache.  Every wait is bounded; on expiry the error flag is raised and
+// the CTA goes on without waiting.
+#pragma once
+
+#include "mmid.cuh"
+#include "q8k.cuh"
+#include "router.cuh"
+
+namespace zmoe {
+
+constexpr int SMALL_WARPS = 16, SMALL_THREADS = 32 * SMALL_WARPS;
+constexpr int SMALL_PAIRS = 32;      // most pairs of a call
+
+// A selection score as an integer that orders like it, 0 for none (a NaN); -0 counts as 0 and -inf is a candidate
+__device__ __forceinline__ unsigned score_key(float s) {
+    const unsigned u = __float_as_uint(__fadd_rn(s, 0.f));
+    return isnan(s) ? 0u : (u >> 31) ? ~u : u | 0x80000000u;
+}
+
+// route_token_warp for up to 256 experts in one group, in registers: lane l holds experts l, l + 32, ..  A round is two integer reductions
+// over the warp and a new look of one lane at its eight scores.  (In the decode router the same form made the calls slower, 66 -> 70 us
+// for a layer of 4096 / 1536 with three tokens, by what it adds to that kernel's code and registers.)
+__device__ __forceinline__ void route_token_regs(const RouterSpec &sp, const float *row_in, float *probs_out, const float *bias,
+                                                 int32_t *ids, float *weights, float *prob_s, int lane) {
+    const int E = sp.E, K = sp.K;
+    float pr[8];
+    unsigned key[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) pr[i] = lane + 32 * i < E ? row_in[lane + 32 * i] : -CUDART_INF_F;
+    if (sp.gating == 0) {
+        float mx = -CUDART_INF_F;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx = fmaxf(mx, pr[i]);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (lane + 32 * i < E) {
+                pr[i] = expf(pr[i] - mx);
+                sum += pr[i];
+            }
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        const float inv = 1.0f / sum;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) pr[i] *= inv;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (lane + 32 * i < E) pr[i] = gate_scalar(pr[i], sp.gating);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int e = lane + 32 * i;
+        key[i] = 0u;
+        if (e < E) {
+            prob_s[e] = pr[i];
+            if (probs_out) probs_out[e] = pr[i];
+            key[i] = score_key(pr[i] + (bias ? bias[e] : 0.f));
+        }
+    }
+    __syncwarp();
+    // the lane's best, the first on a tie
+    unsigned bk;
+    int bi;
+    auto look = [&]() {
+        bk = 0u;
+        bi = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (key[i] > bk) { bk = key[i]; bi = i; }
+    };
+    look();
+    float sum_w = 0.f, mine = 0.f;
+    int my_id = 0;
+    for (int k = 0; k < K; ++k) {
+        const unsigned m = __reduce_max_sync(0xffffffffu, bk);
+        const unsigned win = m == 0u ? 0u : __reduce_min_sync(0xffffffffu, bk == m ? (unsigned)(lane + 32 * bi) : 0xffffffffu);
+        const float w = prob_s[win];
+        if (lane == (int)(win & 31u)) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i == (int)(win >> 5)) key[i] = 0u;      // taken
+            look();
+        }
+        if (lane == k) { mine = w; my_id = (int)win; }
+        sum_w += w;
+    }
+    if (sp.normalize) mine *= 1.0f / fmaxf(sum_w, 6.103515625e-5f);
+    if (sp.weight_scale != 0.0f) mine *= sp.weight_scale;
+    if (lane < K) {
+        ids[lane] = my_id;
+        weights[lane] = mine;
+    }
+}
+
+struct SmallArgs {
+    const float *x, *wr, *bias;
+    int T, D, F, E, K;
+    RouterSpec sp;
+    const uint8_t *wg, *wu, *wd;
+    size_t sg, su, sd, tg, tu, td;   // bytes between experts, bytes of the tensors
+    int rb_gu, rb_dn;
+    float clamp;
+    int clamp_fused;
+    float *logits;                   // [T, E]; probabilities afterwards
+    int32_t *ids;
+    float *weights;
+    uint8_t *q8x;
+    float *act, *out;
+    int accumulate;
+    PlanOut plan;
+    int *err, *bad;
+    unsigned *bar;                   // [2] arrivals and departures, zero between launches
+    int depth_gu, depth_dn;          // rows (pairs of rows, K rows) a warp has on their way
+    int stage;                       // bytes of a warp's staging area
+};
+
+struct SmallLaunch;
+struct RouterArgs;
+SmallArgs small_args(const RouterArgs &r, const SmallLaunch &L);   // all but the staging geometry
+
+// a CTA's shared memory
+struct SmallShared {
+    uint32_t stage;                  // this warp's staging area
+    uint8_t *q8x, *q8f;              // packed rows of the input [T] and of the SwiGLU output [T * K]
+    float *prob;                     // probabilities and selection scores, 2 E floats per token
+    int *ids;                        // [SMALL_PAIRS]
+    float *w;                        // [SMALL_PAIRS]
+    float *part;                     // [SMALL_WARPS]
+    Iq2Tables tb;
+};
+
+// grid-wide barrier number `n` (1, 2, ...) of a cooperative launch
+__device__ __forceinline__ void small_grid_barrier(unsigned *bar, int *err, unsigned n) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        const unsigned want = n * gridDim.x;
+        bool ok = false;
+        for (unsigned i = 0; i < (1u << 20) && !ok; ++i) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            ok = v >= want;
+        }
+        if (!ok) atomicExch(err, 21);
+    }
+    __syncthreads();
+}
+// the last CTA to leave resets the counters for the next launch
+__device__ __forceinline__ void small_leave(unsigned *bar) {
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(bar + 1, 1u) == gridDim.x - 1) {
+            bar[0] = 0u;
+            bar[1] = 0u;
+        }
+    }
+}
+
+// `bytes` bytes at byte `at` of a tensor of `total` bytes go to dst, keeping their offset from a 16-byte boundary.  dst has room for
+// bytes + 32; only whole 16-byte pieces of the tensor are read, but for its last, which may be short.
+__device__ __forceinline__ void small_stage(uint32_t dst, const uint8_t *w, size_t total, size_t at, int bytes, int lane) {
+    const int off = (int)(at & 15);
+    const size_t g0 = at - off;
+    const int n = (off + bytes + 15) >> 4;
+    for (int c = lane; c < n; c += 32) {
+        const size_t g = g0 + 16 * (size_t)c;
+        const int have = g + 16 <= total ? 16 : (int)(total - g);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 16 * c), "l"(w + g), "r"(have) : "memory");
+    }
+}
+__device__ __forceinline__ void small_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// at most n groups of copies still on their way (n up to 3)
+__device__ __forceinline__ void small_wait(int n) {
+    if (n <= 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else if (n == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else if (n == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else asm volatile("cp.async.wait_group 3;" ::: "memory");
+    __syncwarp();
+}
+
+__device__ __forceinline__ void small_prefetch_router(const SmallArgs &a) {
+    for (int e = blockIdx.x; e < a.E; e += gridDim.x)
+        for (int i = threadIdx.x; i < a.D / 32; i += SMALL_THREADS)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(a.wr + (size_t)e * a.D + 32 * i));
+}
+
+// phase 1.  x: the tokens' rows [T][D], in global or shared memory
+template <int GU>
+__device__ __forceinline__ void small_logits(const SmallArgs &a, const SmallShared &s, const float *x) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.D;
+    for (int e = blockIdx.x; e < a.E; e += gridDim.x) {
+        const float4 *wr = reinterpret_cast<const float4 *>(a.wr + (size_t)e * D);
+        for (int t = 0; t < a.T; ++t) {
+            const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)t * D);
+            float v = 0.f;
+            for (int i = tid; i < D / 4; i += SMALL_THREADS) {
+                const float4 w = __ldg(wr + i), u = xr[i];
+                v = fmaf(w.x, u.x, v); v = fmaf(w.y, u.y, v); v = fmaf(w.z, u.z, v); v = fmaf(w.w, u.w, v);
+            }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+            if (lane == 0) s.part[warp] = v;
+            __syncthreads();
+            if (warp == 0) {
+                float sum = lane < SMALL_WARPS ? s.part[lane] : 0.f;
+#pragma unroll
+                for (int off = SMALL_WARPS / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+                if (lane == 0) a.logits[(size_t)t * a.E + e] = sum;
+            }
+            __syncthreads();
+        }
+    }
+    const int nb = D / QK_K, str = q8row_stride(D);
+    for (int i = warp; i < a.T * nb; i += SMALL_WARPS)
+        quantize_block_q8k(x + (size_t)(i / nb) * D + QK_K * (i % nb), s.q8x + (i / nb) * str, D, i % nb, lane, q8_layout_of(GU) | Q8_FOR_TC);
+}
+
+// phase 2: routes, then SwiGLU(gate, up) of the warp's rows into a.act
+template <int GU>
+__device__ __forceinline__ void small_gate_up(const SmallArgs &a, const SmallShared &s) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.D, F = a.F, E = a.E, K = a.K;
+    if (warp < a.T) {
+        float *const prob = s.prob + 2 * E * warp, *const sel = prob + E;
+        for (int e = lane; e < E; e += 32) sel[e] = __ldcg(a.logits + (size_t)warp * E + e);
+        __syncwarp();
+        route_token_regs(a.sp, sel, nullptr, a.bias, s.ids + warp * K, s.w + warp * K, prob, lane);
+    }
+    __syncthreads();
+    const int gw = blockIdx.x * SMALL_WARPS + warp, W = gridDim.x * SMALL_WARPS;
+    const int n_units = a.T * K * F, room = (a.rb_gu + 47) & ~15, str = q8row_stride(D), U = D / 64;
+    auto fetch = [&](int u, int slot) {
+        if (u < n_units) {
+            const int p = u / F, e = s.ids[p];
+            const size_t at = (size_t)(u - p * F) * a.rb_gu;
+            small_stage(s.stage + (uint32_t)(2 * slot * room), a.wg, a.tg, (size_t)e * a.sg + at, a.rb_gu, lane);
+            small_stage(s.stage + (uint32_t)((2 * slot + 1) * room), a.wu, a.tu, (size_t)e * a.su + at, a.rb_gu, lane);
+        }
+        small_commit();
+    };
+    for (int i = 0; i < a.depth_gu; ++i) fetch(gw + i * W, i);
+    float keep_g = 0.f, keep_u = 0.f;
+    int n_done = 0, slot = 0;
+    for (int u = gw; u < n_units; u += W, ++n_done) {
+        small_wait(a.depth_gu - 1);
+        const int p = u / F, r = u - p * F, e = s.ids[p];
+        const uint32_t bg = s.stage + (uint32_t)(2 * slot * room) + (uint32_t)(((size_t)e * a.sg + (size_t)r * a.rb_gu) & 15);
+        const uint32_t bu = s.stage + (uint32_t)((2 * slot + 1) * room) + (uint32_t)(((size_t)e * a.su + (size_t)r * a.rb_gu) & 15);
+        const uint32_t row = smem_u32(s.q8x) + (uint32_t)((p / K) * str);
+        float g = 0.f, v = 0.f;
+        for (int k = lane; k < U; k += 32) {
+            UnitAct ua;
+            load_unit_act<GU>(row, D, k, ua);
+            int is, ms;
+            float d, dm;
+            unit_dot<GU>(bg + (uint32_t)((k >> 2) * QTraits<GU>::kBytes), k & 3, ua, s.tb, is, ms, d, dm);
+            g = fmaf(d * ua.d, (float)is, g);
+            if (QTraits<GU>::kHasMin) g = fmaf(-(dm * ua.d), (float)ms, g);
+            unit_dot<GU>(bu + (uint32_t)((k >> 2) * QTraits<GU>::kBytes), k & 3, ua, s.tb, is, ms, d, dm);
+            v = fmaf(d * ua.d, (float)is, v);
+            if (QTraits<GU>::kHasMin) v = fmaf(-(dm * ua.d), (float)ms, v);
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            g += __shfl_xor_sync(0xffffffffu, g, off);
+            v += __shfl_xor_sync(0xffffffffu, v, off);
+        }
+        // lane i keeps the i-th row's sums: SwiGLU runs once for all rows (once per 32)
+        if (lane == (n_done & 31)) { keep_g = g; keep_u = v; }
+        __syncwarp();
+        fetch(u + a.depth_gu * W, slot);
+        slot = slot + 1 == a.depth_gu ? 0 : slot + 1;
+        if (u + W >= n_units || (n_done & 31) == 31) {
+            const int at = u + (lane - (n_done & 31)) * W;
+            if (lane <= (n_done & 31)) {
+                const float sc = GU == IQ2_XXS ? 0.125f : 1.f, gg = keep_g * sc, uu = keep_u * sc;
+                count_bad(a.bad, gg, uu);
+                a.act[at] = swiglu_f(gg, uu, a.clamp, a.clamp_fused);     // unit u is element u of [T * K][F]
+            }
+        }
+    }
+    small_wait(0);
+}
+
+// the first down rows of the warp on their way (before the barrier that completes a.act)
+__device__ __forceinline__ void small_fetch_down(const SmallArgs &a, const SmallShared &s, int u, int slot) {
+    const int D = a.D, K = a.K, room = (a.rb_dn + 47) & ~15, lane = threadIdx.x & 31;
+    if (u < a.T * D) {
+        const int t = u / D, d = u - t * D;
+        for (int k = 0; k < K; ++k)
+            small_stage(s.stage + (uint32_t)((slot * K + k) * room), a.wd, a.td, (size_t)s.ids[t * K + k] * a.sd + (size_t)d * a.rb_dn, a.rb_dn, lane);
+    }
+    small_commit();
+}
+__device__ __forceinline__ void small_prefetch_down(const SmallArgs &a, const SmallShared &s) {
+    const int gw = blockIdx.x * SMALL_WARPS + (threadIdx.x >> 5), W = gridDim.x * SMALL_WARPS;
+    for (int i = 0; i < a.depth_dn; ++i) small_fetch_down(a, s, gw + i * W, i);
+}
+
+// phase 3 (after small_prefetch_down and the barrier)
+template <int DN>
+__device__ __forceinline__ void small_down(const SmallArgs &a, const SmallShared &s) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.D, F = a.F, K = a.K, P = a.T * K;
+    const int nb = F / QK_K, str = q8row_stride(F), U = F / 64, room = (a.rb_dn + 47) & ~15;
+    for (int i = warp; i < P * nb; i += SMALL_WARPS)
+        quantize_block_q8k<true>(a.act + (size_t)(i / nb) * F + QK_K * (i % nb), s.q8f + (i / nb) * str, F, i % nb, lane, q8_layout_of(DN));
+    __syncthreads();
+    const int gw = blockIdx.x * SMALL_WARPS + warp, W = gridDim.x * SMALL_WARPS;
+    int slot = 0;
+    for (int u = gw; u < a.T * D; u += W) {
+        small_wait(a.depth_dn - 1);
+        const int t = u / D, d = u - t * D;
+        float acc = 0.f;
+        for (int k0 = 0; k0 < K; k0 += 8) {
+            const int k = k0 + (lane >> 2);
+            float v = 0.f;
+            if (k < K) {
+                const int p = t * K + k;
+                const uint32_t blk = s.stage + (uint32_t)((slot * K + k) * room) + (uint32_t)(((size_t)s.ids[p] * a.sd + (size_t)d * a.rb_dn) & 15);
+                const uint32_t row = smem_u32(s.q8f) + (uint32_t)(p * str);
+#pragma unroll 1
+                for (int i = lane & 3; i < U; i += 4) {
+                    UnitAct ua;
+                    load_unit_act<DN>(row, F, i, ua);
+                    int is, ms;
+                    float dw, dm;
+                    unit_dot<DN>(blk + (uint32_t)((i >> 2) * QTraits<DN>::kBytes), i & 3, ua, s.tb, is, ms, dw, dm);
+                    v = fmaf(dw * ua.d, (float)is, v);
+                    if (QTraits<DN>::kHasMin) v = fmaf(-(dm * ua.d), (float)ms, v);
+                }
+            }
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            if (DN == IQ2_XXS) v *= 0.125f;
+            // separately rounded products and sums in k order
+            for (int j = 0; j < 8 && k0 + j < K; ++j) {
+                const float pr = __fmul_rn(s.w[t * K + k0 + j], __shfl_sync(0xffffffffu, v, 4 * j));
+                acc = k0 + j == 0 ? pr : __fadd_rn(acc, pr);
+            }
+        }
+        if (lane == 0) a.out[u] = a.accumulate ? __fadd_rn(__ldcg(a.out + u), acc) : acc;
+        __syncwarp();
+        small_fetch_down(a, s, u + a.depth_dn * W, slot);
+        slot = slot + 1 == a.depth_dn ? 0 : slot + 1;
+    }
+    small_wait(0);
+}
+
+// what the separate launches leave in the context; called by all threads of one CTA, after the second barrier
+__device__ __forceinline__ void small_leave_state(const SmallArgs &a, const SmallShared &s) {
+    const int tid = threadIdx.x, E = a.E, P = a.T * a.K;
+    for (int i = tid; i < a.T * q8row_stride(a.D) / 16; i += SMALL_THREADS)
+        reinterpret_cast<uint4 *>(a.q8x)[i] = reinterpret_cast<const uint4 *>(s.q8x)[i];
+    for (int i = tid; i < a.T * E; i += SMALL_THREADS) a.logits[i] = s.prob[2 * E * (i / E) + i % E];
+    for (int i = tid; i < P; i += SMALL_THREADS) { a.ids[i] = s.ids[i]; a.weights[i] = s.w[i]; }
+    __syncthreads();
+    int *const cnt = reinterpret_cast<int *>(s.prob);
+    build_plan_cta<PLAN_ONE_RUN>(s.ids, P, E, a.plan, cnt, cnt + E + 1, nullptr, nullptr, 1);
+    __syncthreads();
+}
+
+template <int GU, int DN>
+__global__ void __launch_bounds__(SMALL_THREADS, 1) moe_small_kernel(const SmallArgs a) {
+    // a staging area per warp | packed input rows | packed SwiGLU rows | probabilities and scores
+    extern __shared__ __align__(128) uint8_t dyn[];
+    __shared__ float s_part[SMALL_WARPS], s_w[SMALL_PAIRS];
+    __shared__ int s_ids[SMALL_PAIRS];
+    constexpr bool IQ = GU == IQ2_XXS || DN == IQ2_XXS;
+    __shared__ __align__(8) uint64_t iq2_grid[IQ ? 256 : 1], iq2_sign[IQ ? 128 : 1];
+    SmallShared s;
+    s.stage = smem_u32(dyn) + (uint32_t)((threadIdx.x >> 5) * a.stage);
+    s.q8x = dyn + SMALL_WARPS * a.stage;
+    s.q8f = s.q8x + a.T * q8row_stride(a.D);
+    s.prob = reinterpret_cast<float *>(s.q8f + a.T * a.K * q8row_stride(a.F));
+    s.ids = s_ids; s.w = s_w; s.part = s_part;
+    s.tb.grid = smem_u32(iq2_grid); s.tb.signs = smem_u32(iq2_sign);
+    small_prefetch_router(a);
+    if (IQ) iq2_fill_tables(iq2_grid, iq2_sign);
+    pdl_wait_prior_grid();
+    pdl_launch_dependents();
+    small_logits<GU>(a, s, a.x);
+    small_grid_barrier(a.bar, a.err, 1);
+    small_gate_up<GU>(a, s);
+    small_prefetch_down(a, s);
+    small_grid_barrier(a.bar, a.err, 2);
+    small_down<DN>(a, s);
+    if (blockIdx.x == gridDim.x - 1) {
+        __syncthreads();
+        small_leave_state(a, s);
+    }
+    small_leave(a.bar);
+}
+
+}  // namespace zmoe

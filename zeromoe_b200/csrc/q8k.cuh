@@ -12,11 +12,14 @@
 
 namespace zmoe {
 
-// src: 256 floats of block b of the row; row_out: packed row base
+// src: 256 floats of block b of the row; row_out: packed row base.  L2: src was written by other CTAs of the same launch
+// and is read past the L1 cache
+template <bool L2 = false>
 __device__ __forceinline__ void quantize_block_q8k(const float *__restrict__ src, uint8_t *__restrict__ row_out,
-                                                   int I, int b, int lane, int layout) {
-    const float4 v0 = *reinterpret_cast<const float4 *>(src + 8 * lane);
-    const float4 v1 = *reinterpret_cast<const float4 *>(src + 8 * lane + 4);
+                                                   int I, int b, int lane, int layout_and) {
+    const int layout = layout_and & Q8_PLANAR;
+    const float4 *s4 = reinterpret_cast<const float4 *>(src + 8 * lane);
+    const float4 v0 = L2 ? __ldcg(s4) : s4[0], v1 = L2 ? __ldcg(s4 + 1) : s4[1];
     const float x[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     // first occurrence of the largest |x| wins (strict >), as the scalar loop does
     float amax = 0.f, mx = 0.f;
@@ -52,14 +55,15 @@ __device__ __forceinline__ void quantize_block_q8k(const float *__restrict__ src
     int s = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     const int g = lane >> 1;
-    if ((lane & 1) == 0) {
-        *reinterpret_cast<int16_t *>(row_out + q8_bs_off(b) + 2 * g) = (int16_t)s;
-        *reinterpret_cast<__half *>(row_out + q8_bs16_off(layout, b, g)) = __int2half_rn(s);
-    }
-    int all = s;
+    if ((lane & 1) == 0) *reinterpret_cast<int16_t *>(row_out + q8_bs_off(b) + 2 * g) = (int16_t)s;
+    if (lane == 0) *reinterpret_cast<float *>(row_out + q8_d_off(b)) = d;
+    if (layout_and & Q8_FOR_TC) {
+        if ((lane & 1) == 0) *reinterpret_cast<__half *>(row_out + q8_bs16_off(layout, b, g)) = __int2half_rn(s);
+        int all = s;
 #pragma unroll
-    for (int off = 2; off < 32; off <<= 1) all += __shfl_xor_sync(0xffffffffu, all, off);
-    if (lane == 0) *reinterpret_cast<uint2 *>(row_out + q8_d_off(b)) = make_uint2(__float_as_uint(d), (uint32_t)(128 * all));
+        for (int off = 2; off < 32; off <<= 1) all += __shfl_xor_sync(0xffffffffu, all, off);
+        if (lane == 0) *reinterpret_cast<int *>(row_out + q8_d_off(b) + 4) = 128 * all;
+    }
 }
 
 }  // namespace zmoe

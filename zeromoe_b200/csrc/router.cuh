@@ -57,7 +57,7 @@ __device__ __forceinline__ void warp_argmax(float &v, int &i) {
 
 // One warp routes one token.  row: logits in (global), probs out (global, may
 // alias row).  prob_s / sel_s: per-warp shared scratch of E floats each.
-__device__ void route_token_warp(const RouterSpec &sp, const float *row_in, float *probs_out, const float *bias,
+static __device__ void route_token_warp(const RouterSpec &sp, const float *row_in, float *probs_out, const float *bias,
                                  int32_t *ids, float *weights, float *prob_s, float *sel_s, int lane) {
     const int E = sp.E, K = sp.K;
     if (sp.gating == 0) {

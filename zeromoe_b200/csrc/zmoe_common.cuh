@@ -38,6 +38,7 @@ constexpr int Q8_BLOCK_STRIDE = 4 * Q8_UNIT_STRIDE + 16 + 32;   // 368
 constexpr int Q8_BLOCK_D = 4 * Q8_UNIT_STRIDE;                  // d of the block
 constexpr int Q8_BLOCK_BS = Q8_BLOCK_D + 16;                    // its sixteen group sums
 enum Q8Layout : int { Q8_LINEAR = 0, Q8_PLANAR = 1 };
+constexpr int Q8_FOR_TC = 2;   // beside the layout of a row to be quantised: with what the integer tensor-core kernel wants in the padding
 // byte offsets inside a packed row: unit u = 4b + sub, d and group sums of block b
 __host__ __device__ inline int q8_unit_off(int u) { return (u >> 2) * Q8_BLOCK_STRIDE + (u & 3) * Q8_UNIT_STRIDE; }
 __host__ __device__ inline int q8_d_off(int b) { return b * Q8_BLOCK_STRIDE + Q8_BLOCK_D; }

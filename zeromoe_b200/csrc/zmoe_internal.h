@@ -29,6 +29,8 @@ int noalloc_take_error(int *out);
 // device pointers of the route table a layer's context currently holds, and the layer's expert count
 int layer_route_table(zmoe_layer *layer, const int32_t **ids_dev, const float **weights_dev, int *n_experts);
 zmoe_ctx *layer_context(zmoe_layer *layer);
+// out (+)= MoE(x) for T tokens: the router and the experts in one kernel where the call is small enough, else zmoe_route and zmoe_expert_ffn
+int layer_forward(zmoe_layer *layer, const float *x_dev, float *out_dev, int T, int accumulate, void *stream);
 int context_path(const zmoe_ctx *ctx);
 
 // device-resident routing plan buffers
@@ -198,6 +200,51 @@ int launch_combine(float *out, const float *y, const float *w, const int32_t *id
                    int accumulate, cudaStream_t st);
 int launch_block_isums(int type, const void *w, const uint8_t *q8, int32_t *isum, int32_t *msum, int rows, int I,
                        cudaStream_t st);
+
+// a whole layer of very few pairs in one cooperative kernel (moe_small.cuh)
+struct SmallLaunch {
+    int type_gu, type_dn, F;
+    const void *w_gate, *w_up, *w_down;
+    size_t stride_gate, stride_up, stride_down, total_gate, total_up, total_down;
+    float clamp;
+    int clamp_fused;
+    float *act, *out;
+    int accumulate;
+    int *err, *bad;
+    unsigned *bar;         // [2] zero-initialised, left at zero
+};
+bool moe_small_supported(int gu, int dn, int T, int D, int F, int E, int K);
+int launch_moe_small(const RouterArgs &r, const SmallLaunch &L, cudaStream_t st);
+
+// router and launch arguments of that kernel for a call of T tokens of a layer; false where the call does not take it
+bool layer_small_args(zmoe_layer *layer, const float *x_dev, float *out_dev, int T, int accumulate, RouterArgs *r, SmallLaunch *s);
+// host state of the layer's context after such a call
+void layer_small_done(zmoe_layer *layer, const float *x_dev, int T);
+
+// one token through a decoder in one cooperative kernel (decoder_step.cuh)
+struct DecoderStep;
+struct DecoderStepDesc {
+    int n_layers;
+    const float *const *attn_norm, *const *ffn_norm;
+    const void *const *wqkv, *const *wo;
+    zmoe_layer *const *moe;
+    const void *embd, *head;
+    const float *out_norm;
+    int D, H, KV, HD, vocab, max_ctx, splits;
+    float eps, theta_scale, scale;
+    float *h, *xn, *qkv, *part, *logits, *ad;
+    int8_t *aq;
+    void *kc, *vc;
+    int *pos;
+    int32_t *next;
+    unsigned *sync;        // decoder_step_sync_words(KV) zero-initialised words, 8-byte aligned, left at zero
+};
+int decoder_step_sync_words(int KV);
+// null where the decoder's shapes or layers do not allow it
+DecoderStep *decoder_step_create(const DecoderStepDesc &d);
+void decoder_step_destroy(DecoderStep *s);
+// ZMOE_ERR_STATE where a layer's context is set to a path that the kernel does not follow: the caller takes the separate launches
+int decoder_step_launch(DecoderStep *s, const int32_t *token_dev, cudaStream_t st);
 
 // launch helper: programmatic dependent launch attribute on every kernel of the chain
 template <typename... KArgs, typename... Args>
