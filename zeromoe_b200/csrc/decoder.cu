@@ -901,8 +901,10 @@ struct zmoe_decoder {
     int8_t *aq = nullptr;
     float *ad = nullptr;
     __half *kc = nullptr, *vc = nullptr;     // [layers][max_ctx][KV * hd]
-    int *pos = nullptr;
+    int *pos = nullptr;                      // followed by the step kernel's synchronisation words: a reset clears both
+    size_t pos_words = 1;
     int32_t *next = nullptr;
+    DecoderStep *step = nullptr;             // one-token steps in one kernel, where the shapes allow it
 };
 
 extern "C" {
@@ -942,6 +944,7 @@ void launch_q8_0_matmul(float *y, const float *x, const void *weights, int S, in
 
 void zmoe_decoder_destroy(zmoe_decoder *dec) {
     if (!dec) return;
+    decoder_step_destroy(dec->step);
     cudaFree(dec->h); cudaFree(dec->xn); cudaFree(dec->qkv); cudaFree(dec->ao); cudaFree(dec->logits); cudaFree(dec->apart);
     cudaFree(dec->aq); cudaFree(dec->ad); cudaFree(dec->kc); cudaFree(dec->vc); cudaFree(dec->pos); cudaFree(dec->next);
     delete dec;
@@ -982,19 +985,32 @@ int zmoe_decoder_create(const zmoe_decoder_desc *desc, zmoe_decoder **out) {
     bad |= A(&dec->apart, T * d.n_heads * ATTN_SPLITS * (d.head_dim + 2));
     bad |= A(&dec->aq, T * widest); bad |= A(&dec->ad, T * widest / 32);
     bad |= A(&dec->kc, kv); bad |= A(&dec->vc, kv);
-    bad |= A(&dec->pos, 1); bad |= A(&dec->next, 1);
-    if (!bad) bad |= cudaMemset(dec->pos, 0, sizeof(int)) != cudaSuccess || cudaMemset(dec->next, 0, sizeof(int32_t)) != cudaSuccess;
+    dec->pos_words = 2 + (size_t)decoder_step_sync_words(d.n_kv_heads);
+    bad |= A(&dec->pos, dec->pos_words); bad |= A(&dec->next, 1);
+    if (!bad) bad |= cudaMemset(dec->pos, 0, dec->pos_words * sizeof(int)) != cudaSuccess || cudaMemset(dec->next, 0, sizeof(int32_t)) != cudaSuccess;
     if (bad) {
         zmoe_decoder_destroy(dec);
         return ZMOE_ERR_CUDA;
     }
+    DecoderStepDesc sd = {};
+    sd.n_layers = d.n_layers;
+    sd.attn_norm = dec->attn_norm.data(); sd.ffn_norm = dec->ffn_norm.data(); sd.wqkv = dec->wqkv.data(); sd.wo = dec->wo.data();
+    sd.moe = dec->moe.data();
+    sd.embd = d.tok_embd; sd.head = d.lm_head; sd.out_norm = d.out_norm_w;
+    sd.D = d.d_model; sd.H = d.n_heads; sd.KV = d.n_kv_heads; sd.HD = d.head_dim; sd.vocab = d.vocab; sd.max_ctx = d.max_ctx;
+    sd.splits = ATTN_SPLITS;
+    sd.eps = d.rms_eps; sd.theta_scale = powf(d.rope_theta, -2.0f / (float)d.head_dim); sd.scale = 1.0f / sqrtf((float)d.head_dim);
+    sd.h = dec->h; sd.xn = dec->xn; sd.qkv = dec->qkv; sd.part = dec->apart; sd.logits = dec->logits; sd.aq = dec->aq; sd.ad = dec->ad;
+    sd.kc = dec->kc; sd.vc = dec->vc; sd.pos = dec->pos; sd.next = dec->next;
+    sd.sync = reinterpret_cast<unsigned *>(dec->pos) + 2;
+    dec->step = decoder_step_create(sd);     // null: the separate launches
     *out = dec;
     return ZMOE_OK;
 }
 
 int zmoe_decoder_reset(zmoe_decoder *dec, void *stream) {
     if (!dec) return ZMOE_ERR_ARG;
-    return cu(cudaMemsetAsync(dec->pos, 0, sizeof(int), static_cast<cudaStream_t>(stream)));
+    return cu(cudaMemsetAsync(dec->pos, 0, dec->pos_words * sizeof(int), static_cast<cudaStream_t>(stream)));
 }
 
 int zmoe_decoder_step(zmoe_decoder *dec, const int32_t *tokens_dev, int T, void *stream) {
@@ -1006,6 +1022,10 @@ int zmoe_decoder_step(zmoe_decoder *dec, const int32_t *tokens_dev, int T, void 
         tokens_dev = dec->next;             // the token the previous step produced
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (T == 1 && dec->step) {
+        const int one = decoder_step_launch(dec->step, tokens_dev, st);
+        if (one != ZMOE_ERR_STATE) return one;
+    }
     const int D = d.d_model, H = d.n_heads, KV = d.n_kv_heads, hd = d.head_dim, QO = H * hd;
     const size_t kv_layer = (size_t)d.max_ctx * KV * hd;
     const float scale = 1.0f / sqrtf((float)hd);
@@ -1030,8 +1050,7 @@ int zmoe_decoder_step(zmoe_decoder *dec, const int32_t *tokens_dev, int T, void 
         if (!rc) rc = launch_q8_0_mm(dec->h, D, dec->wo[l], dec->aq, dec->ad, T, QO, D, 1, st);
         // ---- MoE block: h += MoE(rmsnorm(h)) ----
         if (!rc) rc = launch_rmsnorm_rows(dec->xn, dec->h, dec->ffn_norm[l], T, D, d.rms_eps, st);
-        if (!rc) rc = zmoe_route(dec->moe[l], dec->xn, T, stream);
-        if (!rc) rc = zmoe_expert_ffn(dec->moe[l], dec->h, T, 1, stream);
+        if (!rc) rc = layer_forward(dec->moe[l], dec->xn, dec->h, T, 1, stream);
     }
     // ---- output head on the last token, greedy sampling ----
     if (!rc) {
