@@ -20,6 +20,7 @@ constexpr int ROUTER_THREADS = 256;
 constexpr int ROUTER_MAXV = 8;     // float4 per thread: rows up to 8192 elements
 constexpr int ROUTER_IDS_SMEM = 2048;  // pairs whose ids the planner mirrors in shared memory
 
+template <bool TC>
 __global__ void __launch_bounds__(ROUTER_THREADS) router_decode_kernel(const RouterArgs a) {
     extern __shared__ __align__(16) uint8_t dyn[];
     __shared__ unsigned s_ticket;
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) router_decode_kernel(const Rou
     const int nb = a.D / QK_K, stride = q8row_stride(a.D);
     for (int idx = blockIdx.x * NW + warp; idx < a.T * nb; idx += gridDim.x * NW) {
         const int t = idx / nb, b = idx % nb;
-        quantize_block_q8k(a.x + (size_t)t * a.D + QK_K * b, a.q8x + (size_t)t * stride, a.D, b, lane, a.q8_layout);
+        quantize_block_q8k<false, TC>(a.x + (size_t)t * a.D + QK_K * b, a.q8x + (size_t)t * stride, a.D, b, lane, a.q8_layout);
     }
     // Two levels of tickets: the last of the E CTAs of a token group routes that group's tokens (one warp per
     // token) while other groups are still computing logits; the last group to finish builds the plan.
@@ -154,11 +155,15 @@ int launch_router_decode(const RouterArgs &a, cudaStream_t st) {
     const size_t smem = (size_t)2 * (ROUTER_THREADS / 32) * a.E * sizeof(float) + (size_t)2 * (a.E + 1) * sizeof(int) +
                         (a.T * a.K <= ROUTER_IDS_SMEM ? (size_t)a.T * a.K * sizeof(int) : 0);
     if (smem > 200 * 1024) return ZMOE_ERR_SHAPE;
-    if (raise_dynamic_smem(reinterpret_cast<const void *>(router_decode_kernel), 200 * 1024) != ZMOE_OK)
+    // q8_layout: unit layout, and Q8_FOR_TC where the rows meet the integer tensor-core kernel
+    RouterArgs b = a;
+    b.q8_layout = a.q8_layout & Q8_PLANAR;
+    auto fn = a.q8_layout & Q8_FOR_TC ? router_decode_kernel<true> : router_decode_kernel<false>;
+    if (raise_dynamic_smem(reinterpret_cast<const void *>(fn), 200 * 1024) != ZMOE_OK)
         return ZMOE_ERR_CUDA;
     const long grid = (long)a.E * ((a.T + ROUTER_TPB - 1) / ROUTER_TPB);
     if (grid > 0x7fffffffL) return ZMOE_ERR_SHAPE;
-    return launch_pdl(router_decode_kernel, dim3((unsigned)grid), dim3(ROUTER_THREADS), smem, st, a) == cudaSuccess
+    return launch_pdl(fn, dim3((unsigned)grid), dim3(ROUTER_THREADS), smem, st, b) == cudaSuccess
                ? ZMOE_OK
                : ZMOE_ERR_CUDA;
 }
@@ -438,6 +443,7 @@ int launch_plan_dense(int S, const PlanBuffers &plan, int nrt, cudaStream_t st) 
 // Q8_K row quantiser (one warp per super-block) and the test-side repack to
 // ggml's 292-byte blocks
 // ------------------------------------------------------------------------
+template <bool TC>
 __global__ void __launch_bounds__(256) quantize_rows_kernel(const float *x, int ldx, uint8_t *q8, int rows, int I,
                                                             int layout) {
     pdl_wait_prior_grid();
@@ -446,7 +452,7 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const float *x, int 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int idx = blockIdx.x * 8 + warp; idx < rows * nb; idx += gridDim.x * 8) {
         const int r = idx / nb, b = idx % nb;
-        quantize_block_q8k(x + (size_t)r * ldx + QK_K * b, q8 + (size_t)r * stride, I, b, lane, layout);
+        quantize_block_q8k<false, TC>(x + (size_t)r * ldx + QK_K * b, q8 + (size_t)r * stride, I, b, lane, layout);
     }
 }
 
@@ -456,7 +462,8 @@ int launch_quantize_rows(const float *x, int ldx, uint8_t *q8, int rows, int I, 
     long grid = (blocks + 7) / 8;
     const long cap = 8L * device_sm_count();
     if (grid > cap) grid = cap;
-    return launch_pdl(quantize_rows_kernel, dim3((unsigned)grid), dim3(256), 0, st, x, ldx, q8, rows, I, layout) == cudaSuccess
+    return launch_pdl(layout & Q8_FOR_TC ? quantize_rows_kernel<true> : quantize_rows_kernel<false>, dim3((unsigned)grid), dim3(256), 0, st,
+                      x, ldx, q8, rows, I, layout & Q8_PLANAR) == cudaSuccess
                ? ZMOE_OK
                : ZMOE_ERR_CUDA;
 }

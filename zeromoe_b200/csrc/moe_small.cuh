@@ -232,7 +232,7 @@ __device__ __forceinline__ void small_logits(const SmallArgs &a, const SmallShar
     }
     const int nb = D / QK_K, str = q8row_stride(D);
     for (int i = warp; i < a.T * nb; i += SMALL_WARPS)
-        quantize_block_q8k(x + (size_t)(i / nb) * D + QK_K * (i % nb), s.q8x + (i / nb) * str, D, i % nb, lane, q8_layout_of(GU) | Q8_FOR_TC);
+        quantize_block_q8k<false, true>(x + (size_t)(i / nb) * D + QK_K * (i % nb), s.q8x + (i / nb) * str, D, i % nb, lane, q8_layout_of(GU));
 }
 
 // phase 2: routes, then SwiGLU(gate, up) of the warp's rows into a.act

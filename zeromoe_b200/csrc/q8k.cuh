@@ -14,10 +14,10 @@ namespace zmoe {
 
 // src: 256 floats of block b of the row; row_out: packed row base.  L2: src was written by other CTAs of the same launch
 // and is read past the L1 cache
-template <bool L2 = false>
+// TC: with what the integer tensor-core kernel wants in the padding (a template: as a run-time branch it cost every decode router call 0.6 us)
+template <bool L2 = false, bool TC = false>
 __device__ __forceinline__ void quantize_block_q8k(const float *__restrict__ src, uint8_t *__restrict__ row_out,
-                                                   int I, int b, int lane, int layout_and) {
-    const int layout = layout_and & Q8_PLANAR;
+                                                   int I, int b, int lane, int layout) {
     const float4 *s4 = reinterpret_cast<const float4 *>(src + 8 * lane);
     const float4 v0 = L2 ? __ldcg(s4) : s4[0], v1 = L2 ? __ldcg(s4 + 1) : s4[1];
     const float x[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
@@ -57,7 +57,7 @@ __device__ __forceinline__ void quantize_block_q8k(const float *__restrict__ src
     const int g = lane >> 1;
     if ((lane & 1) == 0) *reinterpret_cast<int16_t *>(row_out + q8_bs_off(b) + 2 * g) = (int16_t)s;
     if (lane == 0) *reinterpret_cast<float *>(row_out + q8_d_off(b)) = d;
-    if (layout_and & Q8_FOR_TC) {
+    if (TC) {
         if ((lane & 1) == 0) *reinterpret_cast<__half *>(row_out + q8_bs16_off(layout, b, g)) = __int2half_rn(s);
         int all = s;
 #pragma unroll
