@@ -791,7 +791,7 @@ int zmoe::layer_forward(zmoe_layer *L, const float *x_dev, float *out_dev, int T
             g_launches += 1;
             layer_small_done(L, x_dev, T);
         }
-        return rc;
+        if (rc != ZMOE_ERR_STATE) return rc;
     }
     int rc = zmoe_route(L, x_dev, T, stream);
     if (!rc) rc = zmoe_expert_ffn(L, out_dev, T, accumulate, stream);

@@ -134,7 +134,8 @@ int decoder_step_launch(DecoderStep *s, const int32_t *token_dev, cudaStream_t s
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, s->fn, a) != cudaSuccess) return ZMOE_ERR_CUDA;
+    const int rc = cooperative_status(cudaLaunchKernelEx(&cfg, s->fn, a));
+    if (rc) return rc;
     count_launches(1);
     for (zmoe_layer *L : s->leaving) layer_small_done(L, a.xn, 1);
     return ZMOE_OK;

@@ -85,7 +85,7 @@ int launch_moe_small(const RouterArgs &r, const SmallLaunch &L, cudaStream_t st)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, fn, a) == cudaSuccess ? ZMOE_OK : ZMOE_ERR_CUDA;
+    return cooperative_status(cudaLaunchKernelEx(&cfg, fn, a));
 }
 
 }  // namespace zmoe

@@ -20,6 +20,7 @@
 
 #include "mmid.cuh"
 #include "q8k.cuh"
+#define ZMOE_PLAN_ONLY
 #include "router.cuh"
 
 namespace zmoe {

@@ -55,9 +55,10 @@ __device__ __forceinline__ void warp_argmax(float &v, int &i) {
     }
 }
 
+#ifndef ZMOE_PLAN_ONLY   // one source file compiles the router itself; the others take the types and the planner
 // One warp routes one token.  row: logits in (global), probs out (global, may
 // alias row).  prob_s / sel_s: per-warp shared scratch of E floats each.
-static __device__ void route_token_warp(const RouterSpec &sp, const float *row_in, float *probs_out, const float *bias,
+__device__ void route_token_warp(const RouterSpec &sp, const float *row_in, float *probs_out, const float *bias,
                                  int32_t *ids, float *weights, float *prob_s, float *sel_s, int lane) {
     const int E = sp.E, K = sp.K;
     if (sp.gating == 0) {
@@ -151,6 +152,8 @@ static __device__ void route_token_warp(const RouterSpec &sp, const float *row_i
             for (int k = 0; k < K; ++k) weights[k] *= sp.weight_scale;
     }
 }
+
+#endif
 
 // How the planner fills an expert's list.  Up to 128 pairs one warp takes them all (a single run: its counts are the totals and
 // its cursors the experts' offsets, which saves a pass and a barrier: 8 tokens of 8 among 128 experts, quantiser and planner

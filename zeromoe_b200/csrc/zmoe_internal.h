@@ -214,7 +214,16 @@ struct SmallLaunch {
     unsigned *bar;         // [2] zero-initialised, left at zero
 };
 bool moe_small_supported(int gu, int dn, int T, int D, int F, int E, int K);
+// ZMOE_ERR_STATE where the device cannot hold the whole grid at once (the caller takes the separate launches)
 int launch_moe_small(const RouterArgs &r, const SmallLaunch &L, cudaStream_t st);
+// status of a cooperative launch: ZMOE_ERR_STATE, with the error cleared, where it was refused for its size
+inline int cooperative_status(cudaError_t e) {
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+        cudaGetLastError();
+        return ZMOE_ERR_STATE;
+    }
+    return e == cudaSuccess ? ZMOE_OK : ZMOE_ERR_CUDA;
+}
 
 // router and launch arguments of that kernel for a call of T tokens of a layer; false where the call does not take it
 bool layer_small_args(zmoe_layer *layer, const float *x_dev, float *out_dev, int T, int accumulate, RouterArgs *r, SmallLaunch *s);
@@ -243,7 +252,8 @@ int decoder_step_sync_words(int KV);
 // null where the decoder's shapes or layers do not allow it
 DecoderStep *decoder_step_create(const DecoderStepDesc &d);
 void decoder_step_destroy(DecoderStep *s);
-// ZMOE_ERR_STATE where a layer's context is set to a path that the kernel does not follow: the caller takes the separate launches
+// ZMOE_ERR_STATE where a layer's context is set to a path that the kernel does not follow, or the device cannot hold the whole grid at once:
+// the caller takes the separate launches
 int decoder_step_launch(DecoderStep *s, const int32_t *token_dev, cudaStream_t st);
 
 // launch helper: programmatic dependent launch attribute on every kernel of the chain
