@@ -2,6 +2,7 @@
 // the tcgen05 grouped GEMM.
 #include <map>
 #include <mutex>
+#include <set>
 #include <utility>
 
 #include "gemm_sm100.cuh"
@@ -191,11 +192,38 @@ int launch_q8_roundtrip_f16(const float *x, int ldx, void *out_f16, float *scale
                : ZMOE_ERR_CUDA;
 }
 
-bool gemm_sm100_supported(int type, int I, int O) {
-    return block_bytes(type) != 0 && I > 0 && O > 0 && I % QK_K == 0 && O % GEMM_BM == 0;
+using GemmFn = void (*)(const GemmParams, const GemmMaps);
+
+static GemmFn pick_gemm(int type, bool dual) {
+    switch (type) {
+    case Q2_K: return dual ? gemm_sm100_kernel<Q2_K, true> : gemm_sm100_kernel<Q2_K, false>;
+    case Q3_K: return dual ? gemm_sm100_kernel<Q3_K, true> : gemm_sm100_kernel<Q3_K, false>;
+    case Q4_K: return dual ? gemm_sm100_kernel<Q4_K, true> : gemm_sm100_kernel<Q4_K, false>;
+    case IQ2_XXS: return dual ? gemm_sm100_kernel<IQ2_XXS, true> : gemm_sm100_kernel<IQ2_XXS, false>;
+    }
+    return nullptr;
 }
 
-using GemmFn = void (*)(const GemmParams, const GemmMaps);
+// The roles' register shares are drawn from the launch's: a build that has fewer would wait for them without end.
+static bool gemm_regs_ok(GemmFn fn) {
+    static std::mutex mu;
+    static std::set<GemmFn> seen;
+    std::lock_guard<std::mutex> lock(mu);
+    if (seen.count(fn)) return true;
+    cudaFuncAttributes at;
+    if (cudaFuncGetAttributes(&at, fn) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (at.numRegs != GEMM_REGS) return false;
+    seen.insert(fn);
+    return true;
+}
+
+bool gemm_sm100_supported(int type, int I, int O) {
+    return block_bytes(type) != 0 && I > 0 && O > 0 && I % QK_K == 0 && O % GEMM_BM == 0 && pick_gemm(type, true) &&
+           gemm_regs_ok(pick_gemm(type, true)) && gemm_regs_ok(pick_gemm(type, false));
+}
 
 // Cycle counters of the instrumented build (see GSTAT_* in gemm_sm100.cuh): two sets of 16 counters on the
 // current device, the first for gate / up launches, the second for down launches; null in normal builds.
@@ -318,14 +346,7 @@ int make_tc_map(CUtensorMap *m, const void *base, int E, int O, int rb, size_t e
 
 int launch_gemm_sm100(const GemmLaunch &L, cudaStream_t st) {
     if (!gemm_sm100_supported(L.type, L.I, L.O)) return ZMOE_ERR_SHAPE;
-    GemmFn fn = nullptr;
-    switch (L.type) {
-    case Q2_K: fn = L.dual ? gemm_sm100_kernel<Q2_K, true> : gemm_sm100_kernel<Q2_K, false>; break;
-    case Q3_K: fn = L.dual ? gemm_sm100_kernel<Q3_K, true> : gemm_sm100_kernel<Q3_K, false>; break;
-    case Q4_K: fn = L.dual ? gemm_sm100_kernel<Q4_K, true> : gemm_sm100_kernel<Q4_K, false>; break;
-    case IQ2_XXS: fn = L.dual ? gemm_sm100_kernel<IQ2_XXS, true> : gemm_sm100_kernel<IQ2_XXS, false>; break;
-    default: return ZMOE_ERR_TYPE;
-    }
+    const GemmFn fn = pick_gemm(L.type, L.dual);
     const int pitch = gemm_raw_pitch(L.type);
     const size_t smem = (size_t)GEMM_NB * GEMM_BN * GEMM_BK * 2 + (size_t)GEMM_NRAW * 2 * GEMM_BM * pitch + 1024;
     if (raise_dynamic_smem(reinterpret_cast<const void *>(fn), smem) != ZMOE_OK) return ZMOE_ERR_CUDA;

@@ -9,8 +9,8 @@
 // rows and the same 128 up rows; otherwise rows m0..m0+127 and m0+128..m0+255 of one matrix)
 // against up to 160 pairs; both halves multiply the same activation tile, which halves the
 // activation traffic per flop.
-//   warp 0     issues tcgen05.mma (M = 128 weight rows, N = pairs, K = 16 per instruction, A from tensor memory, B from
-//              shared memory) for both halves; tcgen05.commit releases the operand slots.
+//   warps 0, 3 issue tcgen05.mma (M = 128 weight rows, N = pairs, K = 16 per instruction, A from tensor memory, B from
+//              shared memory), a half tile each; tcgen05.commit releases the operand slots.
 //   warp 1     loader of the weights: copies the raw quantised super-blocks of the tile's 256 rows, one
 //              super-block column (256 k) at a time, into a ring in shared memory with tiled copies on the TMA
 //              engine (no multicast), completion on mbarriers.  Rows that are
@@ -18,13 +18,12 @@
 //              copies per 128 rows, one per position of a row inside its group.
 //   warp 2     loader of the activations: one tiled copy per 64 k of the rows gathered into expert order, into a
 //              ring of its own.
-//   warp 3     idle: makes the first converter's number a multiple of four.
-//   warps 4-19 converters, two groups of eight: a thread reads 64 consecutive weights of one row from shared memory,
-//              converts them to fp16 in 32 registers and stores them as its lane of the A operand in tensor memory.
-//              The groups take alternate k-steps, so that one group's loads and conversion overlap the other's
-//              waits, and a group converts before it waits for its operand slot.  The same warps drain the
-//              accumulators of a finished tile (tcgen05.ld, SwiGLU in DUAL mode, f32 stores) while the first k-steps
-//              of the next tile already lie in tensor memory.
+//   warps 4-19 converters, two groups of eight: a thread reads 128 consecutive weights of one row from shared memory,
+//              converts 64 at a time to fp16 in 32 registers and stores them as its lane of the A operand in tensor memory.
+//              The groups take alternate k-steps (each has a half of the super-block), so that one group's loads and conversion
+//              overlap the other's waits.  A group converts before it waits for its operand slot, hands a stored step over halfway
+//              through the conversion of the next one, and loads its next half before it needs it.
+//   warps 20-23 drain the accumulators of a finished tile (tcgen05.ld, SwiGLU in DUAL mode, f32 stores).
 //
 // What bounds it.  A from tensor memory: with both operands in shared memory the fp16 weights cost a store and a read there
 // (16 KB each per half tile and k-step), and raw blocks, activations, stores and operand reads together needed more
@@ -33,10 +32,12 @@
 // (commit, wait, tcgen05.st, wait, issue) takes longer than the MMAs of one other slot.  Tiles of at most
 // 80 pairs use half of the accumulator columns and alternate between two buffers, so that the
 // drain of one overlaps the MMAs of the next.  Below about 100 pairs the converters' instruction issue is the limit (every
-// weight is converted once per pair block).  Measured on one B200 against both operands in shared memory, two slots, 256
-// pairs: 700 tokens of 4096 / 1536, 128 experts, Q2_K gate and up 730 -> 423 us, Q3_K down 422 -> 263; 4096 tokens
-// of IQ2_XXS, skewed load, 1486 -> 1181 and 747 -> 621; 8192 tokens of 7168 / 2048, 256 experts, Q4_K, with a shared
-// expert 6264 -> 4776 and 3080 -> 2623.
+// weight is converted once per pair block): 64 % of the issue slots at 44 pairs, the integer pipe half busy.
+// Measured on one B200, layers of 128 experts, us per layer with all its launches, this form against one where sixteen
+// warps converted 64 weights at a time and drained as well and one warp issued all MMAs: 4096 / 1536, Q2_K gate and up, Q3_K down, 512 tokens
+// 759 -> 565, 700 785 -> 594, 1024 831 -> 658; IQ2_XXS 700 tokens 836 -> 650; Q3_K 700 919 -> 683; Q4_K 2048 / 768 512 tokens 247 -> 204;
+// 4096 tokens of IQ2_XXS, skewed load, 2357 -> 2255; 8192 tokens of 7168 / 2048, 256 experts, Q4_K, with a shared expert 10 270 -> 9 710.
+// Of that the converters' instructions gave a third, the drain's own warps (before, 16 to 30 % of a converter's time) more than half.
 // Activations arrive already rounded through Q8_K (value = d * q) as fp16, each row divided by a
 // power of two that brings its largest value near 2^13 (undone exactly in the epilogue), so the
 // result follows the reference CPU path's activation quantisation and cannot overflow fp16;
@@ -58,12 +59,16 @@ constexpr int GEMM_BK = 64;         // k per step: one 128-byte swizzle row of f
 constexpr int GEMM_NB = 4;          // activation slots
 constexpr int GEMM_NRAW = 3;        // raw super-block slots
 constexpr int GEMM_CWARPS = 16;     // converter warps: two groups of eight
-constexpr int GEMM_CW0 = 4;          // first of them; warps 0-2 issue MMAs and copies, warp 3 only waits at the last barrier
-constexpr int GEMM_THREADS = 32 * (GEMM_CW0 + GEMM_CWARPS);
+constexpr int GEMM_CW0 = 4;          // first of them, a multiple of four
+constexpr int GEMM_DW0 = GEMM_CW0 + GEMM_CWARPS;   // first of the four drain warps
+constexpr int GEMM_THREADS = 32 * (GEMM_DW0 + 4);
 constexpr int GEMM_NA = 3;          // weight slots in tensor memory, 2 x 32 columns each
 constexpr int GEMM_A_COL = 2 * GEMM_BN;   // tensor-memory column of the first of them
 constexpr int GEMM_NBOX = GEMM_BN / 32;   // activation boxes of 32, 64, .. 160 rows
 constexpr int GEMM_MAX_ACTIVE = 512;
+// registers per thread: of the launch, and of the warpgroups' roles, which add up to six times the launch's
+constexpr int GEMM_REGS = 80, GEMM_REGS_CONV = 88, GEMM_REGS_DRAIN = 80, GEMM_REGS_MISC = 48;
+static_assert(4 * GEMM_REGS_CONV + GEMM_REGS_DRAIN + GEMM_REGS_MISC == 6 * GEMM_REGS, "registers");
 
 // bytes between the raw copies of consecutive rows in shared memory: room for one super-block plus its
 // offset from the 16-byte boundary the copy starts on, and a multiple of 16 that is 16 or 48 modulo 128
@@ -98,7 +103,7 @@ struct GemmParams {
 // ZMOE_GEMM_STATS=1 in the environment): one thread per role of CTA 0 adds up clock64() differences around
 // its waits and its work and stores the sums when the kernel ends.  Slots: 0 k-steps, 1 converter
 // wait for raw blocks, 2 load + convert, 3 drain, 4 wait for an operand slot, 5 store + arrive,
-// 6 MMA wait for weights, 7 MMA wait for activations, 8 MMA wait for the accumulators, 9 tiles,
+// 6 MMA wait for operands, 7 drain wait for the accumulators, 8 MMA wait for the accumulators, 9 tiles,
 // 10 MMA issue.
 #ifdef ZMOE_GEMM_STATS
 #define GSTAT_DECL unsigned long long gs_t0 = 0, gs_acc[5] = {0, 0, 0, 0, 0}; const bool gs_on = blockIdx.x == 0 && p.stats != nullptr
@@ -134,12 +139,15 @@ template <int TYPE, bool DUAL>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    // a_*: weight slots in tensor memory; b_*: activation slots; acc_*: accumulator buffers, by tile parity
-    __shared__ __align__(8) uint64_t a_full[GEMM_NA], a_empty[GEMM_NA], b_full[GEMM_NB], b_empty[GEMM_NB], raw_full[GEMM_NRAW],
-        raw_empty[GEMM_NRAW], acc_full[2], acc_empty[2];
+    // K-step j of the CTA's run (counted through its tiles) uses entry j % GEMM_NB of two rings: in_full, all that its MMAs wait for (the
+    // weights from eight converter warps, the activations), and done, its MMAs (of both issuers) have finished: its operand slots can be
+    // refilled.  No waiter can be a whole ring behind: each arrives on the in_full of a later k-step first.
+    // raw_*: raw super-block slots; acc_*: accumulator buffers, by tile parity
+    __shared__ __align__(8) uint64_t in_full[GEMM_NB], done[GEMM_NB], raw_full[GEMM_NRAW], raw_empty[GEMM_NRAW], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
-    __shared__ int s_tile_offs[GEMM_MAX_ACTIVE + 1];
-    __shared__ __align__(16) uint2 grid_s[TYPE == IQ2_XXS ? 256 * IQ2_TABLE_COPIES : 2];
+    __shared__ int s_tile_offs[GEMM_MAX_ACTIVE + 1], s_active[GEMM_MAX_ACTIVE], s_aoffs[GEMM_MAX_ACTIVE], s_antok[GEMM_MAX_ACTIVE];
+    __shared__ int2 s_col[4][GEMM_BN];                       // per drain warp: scale (as bits) and pair of a tile's columns
+    __shared__ __align__(16) uint4 grid_s[TYPE == IQ2_XXS ? 256 * IQ2_TABLE_COPIES : 1];
 
     // 1024-byte alignment of the activation tiles (required by the 128-byte swizzle)
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -153,17 +161,13 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
-        for (int s = 0; s < GEMM_NA; ++s) {
-            mbar_init(&a_full[s], GEMM_CWARPS / 2);     // one arrival per warp of the group
-            mbar_init(&a_empty[s], 1);
-        }
         for (int s = 0; s < 2; ++s) {
-            mbar_init(&acc_full[s], 1);
-            mbar_init(&acc_empty[s], GEMM_CWARPS);
+            mbar_init(&acc_full[s], 2);                 // a commit of each issuer
+            mbar_init(&acc_empty[s], 4);
         }
         for (int s = 0; s < GEMM_NB; ++s) {
-            mbar_init(&b_full[s], 1);                   // the loader's expect_tx arrival
-            mbar_init(&b_empty[s], 1);
+            mbar_init(&in_full[s], GEMM_CWARPS / 2 + 1);   // one arrival per warp of the group, the loader's expect_tx arrival
+            mbar_init(&done[s], 2);
         }
         for (int s = 0; s < GEMM_NRAW; ++s) {
             mbar_init(&raw_full[s], 1);
@@ -182,6 +186,11 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
     const int n_active = min(p.hdr[0], GEMM_MAX_ACTIVE);
     const int mstep = DUAL ? GEMM_BM : 2 * GEMM_BM;          // rows of one matrix a tile covers
     const int mblocks = (p.O + mstep - 1) / mstep;
+    for (int i = tid; i < n_active; i += GEMM_THREADS) {
+        s_active[i] = p.active[i];
+        s_aoffs[i] = p.aoffs[i];
+        s_antok[i] = p.antok[i];
+    }
     if (warp == 0) {
         // prefix sums of the tiles per active expert, 32 experts at a time
         int run = 0;
@@ -207,22 +216,27 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
     const int nblk = p.I / QK_K;
     bool alive = true;
 
+    // which expert, rows and pairs a tile has; called by whole warps
     auto tile_info = [&](int tile, int &e, int &m0, int &p0, int &np) {
+        // last a with s_tile_offs[a] <= tile: the lanes probe 32 points of the range at once
         int lo = 0, hi = n_active - 1;
         while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (s_tile_offs[mid] <= tile) lo = mid; else hi = mid - 1;
+            const int step = (hi - lo + 31) >> 5, probe = min(hi, lo + (lane + 1) * step);
+            const int k = __popc(__ballot_sync(0xffffffffu, s_tile_offs[probe] <= tile));   // probes increase: a prefix of the lanes
+            const int nlo = k == 0 ? lo : min(hi, lo + k * step);
+            hi = max(nlo, k == 32 ? hi : min(hi, lo + (k + 1) * step) - 1);
+            lo = nlo;
         }
         const int local = tile - s_tile_offs[lo];
-        e = p.active[lo];
+        e = s_active[lo];
         // pair block outermost: the row blocks of one pair block run back to back and reuse
         // the same activation rows from L2
         const int nb = local / mblocks;
         m0 = (local % mblocks) * mstep;
         // an expert's pairs are split evenly over its pair blocks (180 pairs: 96 + 84, not 160 + 20)
-        const int cnt = p.antok[lo], npb = (cnt + GEMM_BN - 1) / GEMM_BN;
+        const int cnt = s_antok[lo], npb = (cnt + GEMM_BN - 1) / GEMM_BN;
         const int bsz = ((cnt + npb - 1) / npb + 15) & ~15;
-        p0 = p.aoffs[lo] + nb * bsz;
+        p0 = s_aoffs[lo] + nb * bsz;
         np = max(0, min(bsz, cnt - nb * bsz));
     };
     // the second half of a tile exists unless the matrix ends after the first (rows a multiple of 128, not 256)
@@ -231,8 +245,9 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
     auto acc_col = [&](int nt, int np) -> uint32_t { return np <= GEMM_BN / 2 ? (uint32_t)((nt & 1) * GEMM_BN) : 0u; };
     auto acc_stride = [&](int np) -> uint32_t { return np <= GEMM_BN / 2 ? GEMM_BN / 2 : GEMM_BN; };
 
-    if (warp >= GEMM_CW0) {
+    if (warp >= GEMM_CW0 && warp < GEMM_DW0) {
         // ------------------------------- converters ------------------------------------
+        regs_inc<GEMM_REGS_CONV>();
         // thread -> (group, half tile, row); a warp may only touch the quarter warp % 4 of the tensor-memory lanes
         const int cw = warp - GEMM_CW0;
         const int q = cw & 3, which = (cw >> 2) & 1, grp = cw >> 3;
@@ -242,159 +257,177 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
         // row r = G * sr + j sits in sub-array j (the copy of position j of every group) at sr
         const int G = 1 << p.g_log2, rj = r & (G - 1), rsr = r >> p.g_log2;
         const uint32_t row_at = smem_u32(raw_base) + which * RAW_HALF + (rj * (GEMM_BM >> p.g_log2) + rsr) * PITCH;
-        int it = 0;   // k-steps of the tiles before the current one
-        int rc = 0;   // super-block columns of the tiles before the current one
+        uint32_t col = 0;                     // super-block columns so far: column col holds k-steps 4 col to 4 col + 3
+        uint32_t rs = 0, rph = 0;             // its raw slot, and that one's phase
+        uint32_t slot = grp;                  // operand slot of this group's next k-step
         GSTAT_DECL;
-        // ---- drain of a finished tile's accumulators (all converter warps) ----
-        // warp w reads its quarter of the lanes (rows) and every fourth 8-column chunk of the tile's pairs, from chunk
-        // w / 4 on; lane j of the metadata holds column j % 8 of the warp's chunk j / 8 (d_*[0]) or 4 + j / 8 (d_*[1]).
-        // The loop over the chunks stays rolled: the code runs once per tile and would otherwise be fetched anew each time.
-        const int cset = cw >> 2;
-        int nt = 0;                      // tiles converted so far
-        int d_m0 = 0, d_np = 0;          // the tile waiting for its drain
-        bool d_two = false;
-        int d_pair[2] = {-1, -1};
-        float d_sc[2] = {0.f, 0.f};
-        auto drain = [&]() -> bool {
-            const int t = nt - 1;
-            if (!mbar_wait_suspend(&acc_full[t & 1], (t >> 1) & 1)) return false;
+        HalfBlock<TYPE> hb;
+        // the half of column col, super-block b of its tile (rows of a half tile that does not exist: what lies there, never stored)
+        auto load = [&](int b) -> bool {
+            if (!mbar_wait(&raw_full[rs], rph)) {
+                atomicExch(p.err, 7);
+                return false;
+            }
+            hb.load(row_at + rs * RAW_SLOT + ((uint32_t)(rj * p.rb + b * BB) & 15u), grp, p.g_log2 == 0, tb);
+            return true;
+        };
+        // the k-step stored last: its stores may still be on their way; it is handed over halfway through the next one's conversion
+        int pending = -1;
+        auto finish = [&]() {
+            if (pending < 0) return;
+            tmem_st_wait();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&in_full[pending]);
+            pending = -1;
+        };
+        if ((int)blockIdx.x < n_tiles) alive = load(0);
+        for (int tile = blockIdx.x; alive && tile < n_tiles; tile += gridDim.x) {
+            int e, m0, p0, np;
+            tile_info(tile, e, m0, p0, np);
+            const bool worker = which == 0 || has_half1(m0);
+            // k-step 4 col + e into its operand slot, which was last read by the k-step three before: the next entry of the ring, of this
+            // column for the last step and of the one before for the others (before the first column: a phase that counts as complete).
+            uint32_t a[32];
+            auto put = [&](const uint32_t e) -> bool {
+                const uint32_t before = (e + 1) % GEMM_NB;
+                if (!mbar_wait(&done[before], (col + (before == 0 ? 0 : 1)) & 1)) {
+                    atomicExch(p.err, 3);
+                    return false;
+                }
+                GSTAT_END(3);
+                tc_fence_after_sync();
+                if (worker) tmem_st_32x32(a_slot + 64 * slot, a);
+                pending = (int)e;
+                slot = slot == 0 ? GEMM_NA - 1 : slot - 1;        // two steps on
+                GSTAT_END(4);
+                return true;
+            };
+            // the groups take alternate k-steps: 4 col + grp and 4 col + 2 + grp are the two of this group's half
+            for (int b = 0; b < nblk; ++b) {
+                GSTAT_BEGIN();
+                if (worker) hb.template step<0>(a, finish);
+                else finish();
+                GSTAT_END(1);
+                if (!put(grp)) {
+                    alive = false;
+                    break;
+                }
+                if (worker) hb.template step<1>(a, finish);
+                else finish();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&raw_empty[rs]);       // this warp is done with the raw slot
+                GSTAT_END(1);
+                if (!put(2 + grp)) {
+                    alive = false;
+                    break;
+                }
+                ++col;
+                if (++rs == GEMM_NRAW) { rs = 0; rph ^= 1; }
+                if ((b + 1 < nblk || tile + (int)gridDim.x < n_tiles) && !load(b + 1 < nblk ? b + 1 : 0)) {
+                    alive = false;
+                    break;
+                }
+                GSTAT_END(0);
+            }
+        }
+        finish();
+#ifdef ZMOE_GEMM_STATS
+        if (cw == 1 && lane == 0) {
+            GSTAT_COUNT(4 * col, 0);
+            GSTAT_STORE(0, 1); GSTAT_STORE(1, 2); GSTAT_STORE(3, 4); GSTAT_STORE(4, 5);
+        }
+#endif
+    } else if (warp >= GEMM_DW0) {
+        // ------------------------------- drain ------------------------------------
+        // Warp w reads its quarter of the lanes (rows) of a finished tile's accumulators, eight columns (pairs) at a time.  The
+        // loop over the columns stays rolled: the code runs once per tile and would otherwise be fetched anew each time.
+        const int q = warp & 3;
+        const uint32_t lanes = tmem_base + ((uint32_t)(32 * q) << 16);
+        int nt = 0;
+        GSTAT_DECL;
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++nt) {
+            int e, m0, p0, np;
+            tile_info(tile, e, m0, p0, np);
+            const bool two = has_half1(m0);
+            __syncwarp();
+            for (int c = lane; c < np; c += 32) s_col[q][c] = make_int2(__float_as_int(p.xscale[p0 + c]), p.slot[p0 + c]);
+            __syncwarp();
+            GSTAT_BEGIN();
+            if (!mbar_wait_suspend(&acc_full[nt & 1], (nt >> 1) & 1)) {
+                atomicExch(p.err, 6);
+                break;
+            }
+            GSTAT_END(0);
             tc_fence_after_sync();
-            const uint32_t acc0 = lanes + acc_col(t, d_np), acc1 = acc0 + acc_stride(d_np);
-            float *const yf = p.y + d_m0 + r;     // this thread's weight row (first half)
+            const uint32_t acc0 = lanes + acc_col(nt, np), acc1 = acc0 + acc_stride(np);
+            float *const yf = p.y + m0 + 32 * q + lane;          // this thread's weight row (first half)
 #pragma unroll 1
-            for (int i = 0; 8 * (cset + 4 * i) < d_np; ++i) {
-                const int c0 = 8 * (cset + 4 * i);
+            for (int c0 = 0; c0 < np; c0 += 8) {
                 uint32_t g[8], u[8];
                 tmem_ld_32x8(acc0 + c0, g);
-                if (d_two) tmem_ld_32x8(acc1 + c0, u);
-                const int my_pair = i < 4 ? d_pair[0] : d_pair[1], src = 8 * (i & 3);
-                const float my_sc = i < 4 ? d_sc[0] : d_sc[1];
+                if (two) tmem_ld_32x8(acc1 + c0, u);
                 tmem_ld_wait();
-                // the arithmetic of all columns first, without branches, so that the columns' dependency
-                // chains interleave; x - x is 0 for a finite x and NaN otherwise: the sum flags a non-finite
-                // gate / up value
+                // x * 0 is 0 for a finite x and NaN otherwise: the sum flags a non-finite gate / up value
                 float probe = 0.f;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const float sc = __shfl_sync(0xffffffffu, my_sc, src + j);
+                    const float sc = __int_as_float(s_col[q][c0 + j].x);   // columns past the tile's last: of an earlier one, not stored
                     const float gv = __uint_as_float(g[j]) * sc;
                     if (DUAL) {
                         const float uv = __uint_as_float(u[j]) * sc;
-                        probe += (gv - gv) + (uv - uv);
+                        if (c0 + j < np) probe = fmaf(gv, 0.f, fmaf(uv, 0.f, probe));
                         g[j] = __float_as_uint(swiglu_fast(gv, uv, p.clamp, p.clamp_fused));
                     } else {
                         g[j] = __float_as_uint(gv);
-                        if (d_two) u[j] = __float_as_uint(__uint_as_float(u[j]) * sc);
+                        if (two) u[j] = __float_as_uint(__uint_as_float(u[j]) * sc);
                     }
                 }
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const int pair = __shfl_sync(0xffffffffu, my_pair, src + j);
-                    if (pair >= 0) {
-                        float *row = yf + (size_t)pair * p.ldy;
+                    if (c0 + j < np) {
+                        float *row = yf + (size_t)(uint32_t)s_col[q][c0 + j].y * (uint32_t)p.ldy;
                         row[0] = __uint_as_float(g[j]);
-                        if (!DUAL && d_two) row[GEMM_BM] = __uint_as_float(u[j]);
+                        if (!DUAL && two) row[GEMM_BM] = __uint_as_float(u[j]);
                     }
                 }
-                // warp-uniform decision: the loads and shuffles below are warp-collective
+                // warp-uniform decision: the loads below are warp-collective
                 if (DUAL && p.bad && __any_sync(0xffffffffu, probe != probe)) {
                     // rare: recount this chunk's non-finite inputs exactly
 #pragma unroll 1
                     for (int j = 0; j < 8; ++j) {
-                        const float sc = __shfl_sync(0xffffffffu, my_sc, src + j);
                         uint32_t gj, uj;
                         tmem_ld_1(acc0 + c0 + j, gj);
                         tmem_ld_1(acc1 + c0 + j, uj);
                         tmem_ld_wait();
-                        if (c0 + j < d_np) count_bad(p.bad, __uint_as_float(gj) * sc, __uint_as_float(uj) * sc);
+                        const float sc = __int_as_float(s_col[q][c0 + j].x);
+                        if (c0 + j < np) count_bad(p.bad, __uint_as_float(gj) * sc, __uint_as_float(uj) * sc);
                     }
                 }
             }
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[t & 1]);
-            return true;
-        };
-        for (int tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x, ++nt, it += ksteps, rc += nblk) {
-            int e, m0, p0, np;
-            tile_info(tile, e, m0, p0, np);
-            const bool worker = which == 0 || has_half1(m0);
-            // pair ids and scales of this warp's column chunks: fetched now, used by the drain much later
-            int n_pair[2];
-            float n_sc[2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int col = 8 * (cset + 4 * (4 * i + (lane >> 3))) + (lane & 7);
-                n_pair[i] = col < np ? p.slot[p0 + col] : -1;
-                n_sc[i] = col < np ? p.xscale[p0 + col] : 0.f;
-            }
-            uint32_t blk = 0;
-            for (int ks = grp; ks < ksteps; ks += 2) {
-                const int col = rc + (ks >> 2), rs = col % GEMM_NRAW;
-                GSTAT_BEGIN();
-                if ((ks & 2) == 0) {
-                    // a new super-block column: its raw copy must have landed
-                    if (!mbar_wait_suspend(&raw_full[rs], (col / GEMM_NRAW) & 1)) {
-                        atomicExch(p.err, 7);
-                        alive = false;
-                        break;
-                    }
-                    blk = row_at + rs * RAW_SLOT + ((uint32_t)(rj * p.rb + (ks >> 2) * BB) & 15u);
-                }
-                GSTAT_END(0);
-                uint32_t a[32];
-                if (worker) convert64<TYPE>(blk, ks & 3, p.g_log2 == 0, tb, a);
-                if (ks & 2) {
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&raw_empty[rs]);   // this warp is done with the raw slot
-                }
-                GSTAT_END(1);
-                // the previous tile's accumulators, with this tile's first k-steps in the operand slots
-                if (ks == grp + 2 && nt > 0 && !drain()) {
-                    atomicExch(p.err, 6);
-                    alive = false;
-                    break;
-                }
-                GSTAT_END(2);
-                const int s = (it + ks) % GEMM_NA, n = (it + ks) / GEMM_NA;   // slot, and its uses so far
-                if (n >= 1 && !mbar_wait(&a_empty[s], (n - 1) & 1)) {
-                    atomicExch(p.err, 3);
-                    alive = false;
-                    break;
-                }
-                GSTAT_END(3);
-                tc_fence_after_sync();
-                if (worker) {
-                    tmem_st_32x32(a_slot + 64 * s, a);
-                    tmem_st_wait();
-                }
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&a_full[s]);
-                GSTAT_END(4);
-            }
-            d_m0 = m0; d_np = np; d_two = has_half1(m0);
-#pragma unroll
-            for (int i = 0; i < 2; ++i) { d_pair[i] = n_pair[i]; d_sc[i] = n_sc[i]; }
+            if (lane == 0) mbar_arrive(&acc_empty[nt & 1]);
+            GSTAT_END(2);
         }
-        if (alive && nt > 0 && !drain()) atomicExch(p.err, 6);
 #ifdef ZMOE_GEMM_STATS
-        if (cw == 1 && lane == 0) {
-            GSTAT_COUNT(it, 0);
-            GSTAT_STORE(0, 1); GSTAT_STORE(1, 2); GSTAT_STORE(2, 3); GSTAT_STORE(3, 4); GSTAT_STORE(4, 5);
-        }
+        if (q == 1 && lane == 0) { GSTAT_STORE(0, 7); GSTAT_STORE(2, 3); }
 #endif
-    } else if (warp == 0) {
-        // ------------------------------- MMA issuer ------------------------------------
+    } else {
+        regs_dec<GEMM_REGS_MISC>();
+        if (warp == 0 || warp == 3) {
+        // ------------------------------- MMA issuers ------------------------------------
+        // One warp per half tile: at the few instructions a lone warp gets through between sixteen converter warps, the eight MMAs of a
+        // k-step, their addresses and two commits took one warp 474 cycles where the tensor core takes 195 (48 pairs).
         // The whole warp runs this loop on values that are the same in all lanes and known to the compiler as such
         // (shuffles from lane 0), and one elected lane issues: the operands then live in uniform registers.  With a
-        // branch on the lane number every operand of every MMA was moved there one by one, and at the few instructions
-        // a lone warp gets through between sixteen converter warps the issue itself took about 1000 cycles per k-step.
+        // branch on the lane number every operand of every MMA was moved there one by one.
         int nt = 0;
-        uint32_t it = 0;
+        uint32_t it = 0, s = 0;                                     // k-steps so far; operand slot of the next
         const uint32_t tbase = __shfl_sync(0xffffffffu, tmem_base, 0);
         const uint64_t desc_b0 = umma_desc_sw128(__shfl_sync(0xffffffffu, smem_u32(smem), 0));   // a k-step of 16 advances the start address by 32 bytes
-        bool a_ready = false, b_ready = false;                      // the next k-step's slots, seen full
+        const uint32_t half = __shfl_sync(0xffffffffu, warp == 0 ? 0u : 1u, 0);
+        bool ready = false;                                         // the next k-step's operands, seen complete
         bool small_before = true;                                   // the tile before used one of the two small buffers
         GSTAT_DECL;
         for (int tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x, ++nt) {
@@ -404,8 +437,8 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
             m0 = __shfl_sync(0xffffffffu, m0, 0);
             const int ncols = (np + 15) & ~15;
             const uint32_t idesc = umma_idesc_f16(GEMM_BM, ncols);
-            const bool two = has_half1(m0), small = np <= GEMM_BN / 2;
-            const uint32_t d0 = tbase + acc_col(nt, np), d1 = d0 + acc_stride(np);
+            const bool mine = half == 0 || has_half1(m0), small = np <= GEMM_BN / 2;
+            const uint32_t d = tbase + acc_col(nt, np) + half * acc_stride(np);
             GSTAT_BEGIN();
             // what this tile's accumulators overwrite must have been drained: always the tile two before, and the
             // one before unless both fit the two small buffers
@@ -419,46 +452,38 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
             GSTAT_END(2);
             uint32_t acc = 0;
             for (int left = ksteps; left > 0; --left, ++it) {
-                const uint32_t s = it % GEMM_NA, sb = it % GEMM_NB;
+                const uint32_t sb = it % GEMM_NB;
                 GSTAT_BEGIN();
-                if (!b_ready && !mbar_wait(&b_full[sb], (it / GEMM_NB) & 1)) {
-                    if (lane == 0) atomicExch(p.err, 9);
-                    alive = false;
-                    break;
-                }
-                GSTAT_END(1);
-                if (!a_ready && !mbar_wait(&a_full[s], (it / GEMM_NA) & 1)) {
+                if (!ready && !mbar_wait(&in_full[sb], (it / GEMM_NB) & 1)) {
                     if (lane == 0) atomicExch(p.err, 5);
                     alive = false;
                     break;
                 }
                 GSTAT_END(0);
                 // Issuing blocks until the tensor core has taken the MMAs, and a wait that succeeds at once still costs
-                // about 100 cycles: the next step's slots are looked at before this step's MMAs go out, so that the
-                // answers are there when they have.
+                // about 100 cycles: the next step's operands are looked at before this step's MMAs go out, so that the
+                // answer is there when they have.
                 const uint32_t nx = it + 1;
-                b_ready = mbar_test_wait(&b_full[nx % GEMM_NB], (nx / GEMM_NB) & 1);
-                a_ready = mbar_test_wait(&a_full[nx % GEMM_NA], (nx / GEMM_NA) & 1);
+                ready = mbar_test_wait(&in_full[nx % GEMM_NB], (nx / GEMM_NB) & 1);
                 tc_fence_after_sync();
                 if (elect_one()) {
-                    const uint32_t a0 = tbase + GEMM_A_COL + 64 * s;
-                    const uint64_t b0 = desc_b0 + (uint64_t)(sb * (B_BYTES >> 4));
+                    if (mine) {
+                        const uint32_t a0 = tbase + GEMM_A_COL + 64 * s + 32 * half;
+                        const uint64_t b0 = desc_b0 + (uint64_t)(sb * (B_BYTES >> 4));
 #pragma unroll
-                    for (int k4 = 0; k4 < GEMM_BK / 16; ++k4) {
-                        umma_f16_ta(d0, a0 + 8 * k4, b0 + 2 * k4, idesc, k4 ? 1u : acc);
-                        if (two) umma_f16_ta(d1, a0 + 32 + 8 * k4, b0 + 2 * k4, idesc, k4 ? 1u : acc);
+                        for (int k4 = 0; k4 < GEMM_BK / 16; ++k4) umma_f16_ta(d, a0 + 8 * k4, b0 + 2 * k4, idesc, k4 ? 1u : acc);
                     }
-                    umma_commit(&a_empty[s]);                   // both operands are free once these MMAs have read them
-                    umma_commit(&b_empty[sb]);
+                    umma_commit(&done[sb]);                         // both operands are free once these MMAs have read them
                     if (left == 1) umma_commit(&acc_full[nt & 1]);  // accumulators complete
                 }
+                s = s == GEMM_NA - 1 ? 0 : s + 1;
                 __syncwarp();
                 acc = 1;
                 GSTAT_END(3);
             }
         }
 #ifdef ZMOE_GEMM_STATS
-        if (lane == 0) { GSTAT_STORE(0, 6); GSTAT_STORE(1, 7); GSTAT_STORE(2, 8); GSTAT_COUNT(nt, 9); GSTAT_STORE(3, 10); }
+        if (warp == 0 && lane == 0) { GSTAT_STORE(0, 6); GSTAT_STORE(2, 8); GSTAT_COUNT(nt, 9); GSTAT_STORE(3, 10); }
 #endif
     } else if (warp == 1) {
         // ------------------------------- weight loader ------------------------------------
@@ -469,7 +494,7 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
             const bool two = has_half1(m0);
             for (int b = 0; b < nblk; ++b, ++rc) {
                 const int rs = rc % GEMM_NRAW;
-                if (rc >= GEMM_NRAW && !mbar_wait_suspend(&raw_empty[rs], ((rc / GEMM_NRAW) - 1) & 1)) {
+                if (rc >= GEMM_NRAW && !mbar_wait_sleep(&raw_empty[rs], ((rc / GEMM_NRAW) - 1) & 1, 100)) {
                     if (lane == 0) atomicExch(p.err, 8);
                     alive = false;
                     break;
@@ -500,18 +525,21 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
             const int bi = (np + 31) / 32 - 1;       // the smallest box that covers the tile's pairs
             for (int ks = 0; ks < ksteps; ++ks, ++it) {
                 const int sb = it % GEMM_NB;
-                if (it >= GEMM_NB && !mbar_wait_suspend(&b_empty[sb], ((it / GEMM_NB) - 1) & 1)) {
+                if (!mbar_wait_sleep(&done[sb], ((it / GEMM_NB) - 1) & 1, 100)) {
                     if (lane == 0) atomicExch(p.err, 10);
                     alive = false;
                     break;
                 }
                 if (lane == 0) {
-                    // rows p0 .. of the sorted activations, columns 64 ks ..; rows past the end of the buffer arrive as zeros
-                    mbar_arrive_expect_tx(&b_full[sb], (uint32_t)(32 * (bi + 1) * GEMM_BK * 2));
-                    tma_load_2d(smem + sb * B_BYTES, &maps.box[bi], ks * GEMM_BK, p0, &b_full[sb]);
+                    // rows p0 .. of the sorted activations, 64 columns; rows past the end of the buffer arrive as zeros
+                    mbar_arrive_expect_tx(&in_full[sb], (uint32_t)(32 * (bi + 1) * GEMM_BK * 2));
+                    // the k of the four steps of a super-block: 0, 128, 64, 192 (the converters' groups take a half each, in turn)
+                    const int k64 = (ks & ~3) | ((ks & 1) << 1) | ((ks >> 1) & 1);
+                    tma_load_2d(smem + sb * B_BYTES, &maps.box[bi], k64 * GEMM_BK, p0, &in_full[sb]);
                 }
                 __syncwarp();
             }
+        }
         }
     }
     tc_fence_before_sync();

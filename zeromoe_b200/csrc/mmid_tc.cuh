@@ -120,8 +120,6 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src) {
 __device__ __forceinline__ void cp_async_8(uint32_t dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
-template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 __device__ __forceinline__ void tmem_ld_32xn(uint32_t taddr, uint32_t (&r)[8]) { tmem_ld_32x8(taddr, r); }
 __device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 __device__ __forceinline__ void tc_load_3d(uint32_t dst_smem, const void *tmap, int x, int row, int expert, uint64_t *bar) {
@@ -129,20 +127,6 @@ __device__ __forceinline__ void tc_load_3d(uint32_t dst_smem, const void *tmap, 
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
         ::"r"(dst_smem), "l"(tmap), "r"(x), "r"(row), "r"(expert), "r"(smem_u32(bar))
         : "memory");
-}
-
-// N words that start W words into 16-byte chunks, W known: 128-bit loads and no selects
-template <int N, int W>
-__device__ __forceinline__ void lds_words(uint32_t chunk, uint32_t (&out)[N]) {
-    constexpr int NC = (N + W + 3) / 4;
-    uint32_t c[4 * NC];
-#pragma unroll
-    for (int i = 0; i < NC; ++i) {
-        const uint4 v = lds128(chunk + 16 * i);
-        c[4 * i] = v.x; c[4 * i + 1] = v.y; c[4 * i + 2] = v.z; c[4 * i + 3] = v.w;
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) out[i] = c[W + i];
 }
 
 // fp16 pair of two small integers in the two halves of x (at most 1023 each)
