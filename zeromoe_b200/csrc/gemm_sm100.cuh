@@ -35,9 +35,12 @@
 // weight is converted once per pair block): 64 % of the issue slots at 44 pairs, the integer pipe half busy.
 // Measured on one B200, layers of 128 experts, us per layer with all its launches, this form against one where sixteen
 // warps converted 64 weights at a time and drained as well and one warp issued all MMAs: 4096 / 1536, Q2_K gate and up, Q3_K down, 512 tokens
-// 759 -> 565, 700 785 -> 594, 1024 831 -> 658; IQ2_XXS 700 tokens 836 -> 650; Q3_K 700 919 -> 683; Q4_K 2048 / 768 512 tokens 247 -> 204;
-// 4096 tokens of IQ2_XXS, skewed load, 2357 -> 2255; 8192 tokens of 7168 / 2048, 256 experts, Q4_K, with a shared expert 10 270 -> 9 710.
-// Of that the converters' instructions gave a third, the drain's own warps (before, 16 to 30 % of a converter's time) more than half.
+// 759 -> 560, 700 785 -> 587, 1024 831 -> 644; IQ2_XXS 700 tokens 836 -> 650; Q3_K 700 919 -> 690; Q4_K 2048 / 768 512 tokens 247 -> 203;
+// 4096 tokens of IQ2_XXS, skewed load, 2368 -> 2084; 8192 tokens of 7168 / 2048, 256 experts, Q4_K, with a shared expert 10 270 -> 9 160.
+// Tiles of more than 80 pairs wait for the drain of the one before: its instructions per column count (35 -> about 20 by a loop without clamps,
+// 128-bit loads of the columns' scales and pairs and no predicates on full chunks: 4096 tokens 1908 -> 1734 and, Q4_K 2048 / 768, 775 -> 645).
+// Eight drain warps instead of four took 1718 and 643 there, but 617 instead of 587 at 700 tokens; a drain that loads the next columns
+// ahead was slower (more moves), waits that sleep instead of polling made no difference.
 // Activations arrive already rounded through Q8_K (value = d * q) as fp16, each row divided by a
 // power of two that brings its largest value near 2^13 (undone exactly in the epilogue), so the
 // result follows the reference CPU path's activation quantisation and cannot overflow fp16;
@@ -146,7 +149,7 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
     __shared__ __align__(8) uint64_t in_full[GEMM_NB], done[GEMM_NB], raw_full[GEMM_NRAW], raw_empty[GEMM_NRAW], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_tile_offs[GEMM_MAX_ACTIVE + 1], s_active[GEMM_MAX_ACTIVE], s_aoffs[GEMM_MAX_ACTIVE], s_antok[GEMM_MAX_ACTIVE];
-    __shared__ int2 s_col[4][GEMM_BN];                       // per drain warp: scale (as bits) and pair of a tile's columns
+    __shared__ __align__(16) int2 s_col[4][GEMM_BN];                       // per drain warp: scale (as bits) and pair of a tile's columns
     __shared__ __align__(16) uint4 grid_s[TYPE == IQ2_XXS ? 256 * IQ2_TABLE_COPIES : 1];
 
     // 1024-byte alignment of the activation tiles (required by the 128-byte swizzle)
@@ -344,6 +347,7 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
         // loop over the columns stays rolled: the code runs once per tile and would otherwise be fetched anew each time.
         const int q = warp & 3;
         const uint32_t lanes = tmem_base + ((uint32_t)(32 * q) << 16);
+        const bool plain = p.clamp <= 0.f;                       // then both forms of the activation are the same
         int nt = 0;
         GSTAT_DECL;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++nt) {
@@ -351,7 +355,8 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
             tile_info(tile, e, m0, p0, np);
             const bool two = has_half1(m0);
             __syncwarp();
-            for (int c = lane; c < np; c += 32) s_col[q][c] = make_int2(__float_as_int(p.xscale[p0 + c]), p.slot[p0 + c]);
+            for (int c = lane; c < ((np + 7) & ~7); c += 32)
+                s_col[q][c] = c < np ? make_int2(__float_as_int(p.xscale[p0 + c]), p.slot[p0 + c]) : make_int2(0, 0);
             __syncwarp();
             GSTAT_BEGIN();
             if (!mbar_wait_suspend(&acc_full[nt & 1], (nt >> 1) & 1)) {
@@ -367,29 +372,45 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
                 uint32_t g[8], u[8];
                 tmem_ld_32x8(acc0 + c0, g);
                 if (two) tmem_ld_32x8(acc1 + c0, u);
+                int4 m[4];                                       // scale and pair of columns 2 i and 2 i + 1
+#pragma unroll
+                for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const int4 *>(&s_col[q][c0 + 2 * i]);
                 tmem_ld_wait();
-                // x * 0 is 0 for a finite x and NaN otherwise: the sum flags a non-finite gate / up value
+                // x * 0 is 0 for a finite x and NaN otherwise: the sum flags a value that is not finite, as every result of a gate or up
+                // value that is not finite is
                 float probe = 0.f;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const float sc = __int_as_float(s_col[q][c0 + j].x);   // columns past the tile's last: of an earlier one, not stored
+                    const float sc = __int_as_float(j & 1 ? m[j >> 1].z : m[j >> 1].x);
                     const float gv = __uint_as_float(g[j]) * sc;
                     if (DUAL) {
                         const float uv = __uint_as_float(u[j]) * sc;
-                        if (c0 + j < np) probe = fmaf(gv, 0.f, fmaf(uv, 0.f, probe));
-                        g[j] = __float_as_uint(swiglu_fast(gv, uv, p.clamp, p.clamp_fused));
+                        float v;
+                        if (plain) {
+                            v = swiglu_fast(gv, uv, 0.f, 0);
+                            probe = fmaf(v, 0.f, probe);
+                        } else {
+                            probe = fmaf(gv, 0.f, fmaf(uv, 0.f, probe));
+                            v = swiglu_fast(gv, uv, p.clamp, p.clamp_fused);
+                        }
+                        g[j] = __float_as_uint(v);
                     } else {
                         g[j] = __float_as_uint(gv);
                         if (two) u[j] = __float_as_uint(__uint_as_float(u[j]) * sc);
                     }
                 }
+                auto store = [&](int j) {
+                    float *row = yf + (size_t)(uint32_t)(j & 1 ? m[j >> 1].w : m[j >> 1].y) * (uint32_t)p.ldy;
+                    row[0] = __uint_as_float(g[j]);
+                    if (!DUAL && two) row[GEMM_BM] = __uint_as_float(u[j]);
+                };
+                if (c0 + 8 <= np) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if (c0 + j < np) {
-                        float *row = yf + (size_t)(uint32_t)s_col[q][c0 + j].y * (uint32_t)p.ldy;
-                        row[0] = __uint_as_float(g[j]);
-                        if (!DUAL && two) row[GEMM_BM] = __uint_as_float(u[j]);
-                    }
+                    for (int j = 0; j < 8; ++j) store(j);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 7; ++j)
+                        if (c0 + j < np) store(j);
                 }
                 // warp-uniform decision: the loads below are warp-collective
                 if (DUAL && p.bad && __any_sync(0xffffffffu, probe != probe)) {
