@@ -21,8 +21,7 @@
 //   warps 4-19 converters, two groups of eight: a thread reads 128 consecutive weights of one row from shared memory,
 //              converts 64 at a time to fp16 in 32 registers and stores them as its lane of the A operand in tensor memory.
 //              The groups take alternate k-steps (each has a half of the super-block), so that one group's loads and conversion
-//              overlap the other's waits.  A group converts before it waits for its operand slot, hands a stored step over halfway
-//              through the conversion of the next one, and loads its next half before it needs it.
+//              overlap the other's waits.  A group converts before it waits for its operand slot and loads its next half before it needs it.
 //   warps 20-23 drain the accumulators of a finished tile (tcgen05.ld, SwiGLU in DUAL mode, f32 stores).
 //
 // What bounds it.  A from tensor memory: with both operands in shared memory the fp16 weights cost a store and a read there
@@ -35,8 +34,8 @@
 // weight is converted once per pair block): 64 % of the issue slots at 44 pairs, the integer pipe half busy.
 // Measured on one B200, layers of 128 experts, us per layer with all its launches, this form against one where sixteen
 // warps converted 64 weights at a time and drained as well and one warp issued all MMAs: 4096 / 1536, Q2_K gate and up, Q3_K down, 512 tokens
-// 759 -> 560, 700 785 -> 587, 1024 831 -> 644; IQ2_XXS 700 tokens 836 -> 650; Q3_K 700 919 -> 690; Q4_K 2048 / 768 512 tokens 247 -> 203;
-// 4096 tokens of IQ2_XXS, skewed load, 2368 -> 2084; 8192 tokens of 7168 / 2048, 256 experts, Q4_K, with a shared expert 10 270 -> 9 160.
+// 759 -> 542, 700 785 -> 570, 1024 831 -> 625; IQ2_XXS 700 tokens 836 -> 650; Q3_K 700 919 -> 685; Q4_K 2048 / 768 512 tokens 247 -> 196;
+// 4096 tokens of IQ2_XXS, skewed load, 2368 -> 2080; 8192 tokens of 7168 / 2048, 256 experts, Q4_K, with a shared expert 10 270 -> 8 900.
 // Tiles of more than 80 pairs wait for the drain of the one before: its instructions per column count (35 -> about 20 by a loop without clamps,
 // 128-bit loads of the columns' scales and pairs and no predicates on full chunks: 4096 tokens 1908 -> 1734 and, Q4_K 2048 / 768, 775 -> 645).
 // Eight drain warps instead of four took 1718 and 643 there, but 617 instead of 587 at 700 tokens; a drain that loads the next columns
@@ -274,7 +273,11 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
             hb.load(row_at + rs * RAW_SLOT + ((uint32_t)(rj * p.rb + b * BB) & 15u), grp, p.g_log2 == 0, tb);
             return true;
         };
-        // the k-step stored last: its stores may still be on their way; it is handed over halfway through the next one's conversion
+        // The k-step stored last, whose stores may still be on their way.  It is handed over at once, since the MMAs of all k-steps come
+        // one after the other and a late one holds up the three operand slots, or halfway through the next one's conversion (us per
+        // layer, at once / halfway: Q2_K and Q3_K 700 tokens 569 / 582, Q4_K 2048 / 768 512 tokens 196 / 201, 7168 / 2048 8192 tokens 8183 / 8465;
+        // IQ2_XXS, whose conversion is the longest, 512 tokens 632 / 622).
+        constexpr bool LATE = TYPE == IQ2_XXS;
         int pending = -1;
         auto finish = [&]() {
             if (pending < 0) return;
@@ -284,6 +287,7 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
             if (lane == 0) mbar_arrive(&in_full[pending]);
             pending = -1;
         };
+        const auto midway = [&] { if (LATE) finish(); };
         if ((int)blockIdx.x < n_tiles) alive = load(0);
         for (int tile = blockIdx.x; alive && tile < n_tiles; tile += gridDim.x) {
             int e, m0, p0, np;
@@ -303,21 +307,22 @@ gemm_sm100_kernel(const GemmParams p, const __grid_constant__ GemmMaps maps) {
                 if (worker) tmem_st_32x32(a_slot + 64 * slot, a);
                 pending = (int)e;
                 slot = slot == 0 ? GEMM_NA - 1 : slot - 1;        // two steps on
+                if (!LATE) finish();
                 GSTAT_END(4);
                 return true;
             };
             // the groups take alternate k-steps: 4 col + grp and 4 col + 2 + grp are the two of this group's half
             for (int b = 0; b < nblk; ++b) {
                 GSTAT_BEGIN();
-                if (worker) hb.template step<0>(a, finish);
-                else finish();
+                if (worker) hb.template step<0>(a, midway);
+                else midway();
                 GSTAT_END(1);
                 if (!put(grp)) {
                     alive = false;
                     break;
                 }
-                if (worker) hb.template step<1>(a, finish);
-                else finish();
+                if (worker) hb.template step<1>(a, midway);
+                else midway();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&raw_empty[rs]);       // this warp is done with the raw slot
                 GSTAT_END(1);
