@@ -75,8 +75,9 @@ DecoderStep *decoder_step_create(const DecoderStepDesc &d) {
     // shared memory: what every CTA keeps, and as many rows on their way per warp as the rest has room for
     auto room = [](int bytes) { return (bytes + 47) & ~15; };
     const int rbd = d.D / 32 * 34, rbo = QO / 32 * 34;
-    const size_t rest = (size_t)d.D * 4 + widest + (size_t)((widest / 32 + 3) & ~3) * 4 + (size_t)G * d.HD * 4 + q8row_stride(d.D) +
-                        (size_t)K * q8row_stride(F) + ((size_t)2 * E + 8) * 4;
+    // from x on: a chunk of keys and values while attention runs
+    const size_t from_x = (size_t)d.D * 4 + q8row_stride(d.D) + (size_t)K * q8row_stride(F) + ((size_t)2 * E + 8) * 4, kv = step_kv_bytes(d.HD);
+    const size_t rest = widest + (size_t)((widest / 32 + 3) & ~3) * 4 + (size_t)G * d.HD * 4 + (from_x > kv ? from_x : kv);
     if (rest >= (size_t)STEP_SMEM) return nullptr;
     const int per_warp = (int)(((size_t)STEP_SMEM - rest) / SMALL_WARPS) & ~15;
     auto depth = [&](int bytes, int most) { const int n = per_warp / bytes; return n < most ? n : most; };

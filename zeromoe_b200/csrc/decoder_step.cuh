@@ -132,51 +132,112 @@ __device__ __forceinline__ void step_quantise(const float *x, int8_t *q, float *
     __syncthreads();
 }
 
-// One share of a KV head's keys: attention_kernel with the rotation of q and of the new key folded in.  qs: [G][HD] shared
+// ---- attention ----
+// Keys and values come a chunk of 32 keys at a time, into shared memory, where the heads of a KV head share them.  The chunk that a CTA meets
+// first is on its way while the CTA still multiplies rows of the QKV matrix (all of it but the new key lies in the cache since the step
+// before), and the dot products and the weighted sum then wait for no trip to memory: with the keys read by every warp for itself, and
+// the values eight at a time, attention over 34 to 81 keys took 18 200 cycles per layer, most of it such trips.
+constexpr int STEP_KEYS = 32;
+__host__ __device__ constexpr int step_kv_pitch(int hd) { return 2 * hd + 16; }      // 128-bit loads of one column meet every bank group
+__host__ __device__ constexpr int step_kv_bytes(int hd) { return 2 * STEP_KEYS * step_kv_pitch(hd); }
+
+// the shares of the keys at position p: their number, and the keys of each (a multiple of 32)
+__device__ __forceinline__ void step_shares(const StepArgs &a, int p, int &n_keys, int &per, int &ns) {
+    n_keys = min(p + 1, a.max_ctx);
+    const int chunks = (n_keys + 31) / 32;
+    per = (chunks + a.splits - 1) / a.splits;
+    ns = (chunks + per - 1) / per;
+}
+// rows [k0, k0 + 32) of one KV head up to key `end`, without the new one (it is written by the share that holds it), by one warp
+__device__ __forceinline__ void step_fetch_kv(uint32_t kv, const __half *kc, const __half *vc, int KV, int HD, int kvh, int k0, int end, int fresh, uint64_t *bar,
+                                              int lane) {
+    const int key = k0 + lane, n = max(0, min(STEP_KEYS, end - k0)) - (fresh >= k0 && fresh < min(end, k0 + STEP_KEYS) ? 1 : 0);
+    // what was read and written in this memory before, by ordinary loads and stores, comes before the copies
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)(4 * HD * n));
+    __syncwarp();
+    if (key < end && key != fresh) {
+        const size_t at = ((size_t)key * KV + kvh) * HD;
+        const uint32_t dst = kv + (uint32_t)(lane * step_kv_pitch(HD));
+        bulk_g2s_addr(dst, kc + at, (uint32_t)(2 * HD), bar);
+        bulk_g2s_addr(dst + (uint32_t)(STEP_KEYS * step_kv_pitch(HD)), vc + at, (uint32_t)(2 * HD), bar);
+    }
+}
+
+// Share z of a KV head's keys: attention_kernel with the rotation of q and of the new key folded in.  qs: [G][HD] shared; kv: the chunk;
+// ready: its first chunk is on its way already.  phase: of kv_bar, moved on with every chunk.  False: a wait ran out.
 template <int HD>
-__device__ __forceinline__ void step_attention(const StepArgs &a, __half *kc, __half *vc, int kvh, int z, int p, float *qs, const float2 *rot) {
-    constexpr int DPL = HD / 32;
+__device__ __forceinline__ bool step_attention(const StepArgs &a, __half *kc, __half *vc, int kvh, int z, int p, float *qs, const float2 *rot, uint8_t *kv,
+                                               uint64_t *kv_bar, uint32_t &phase, bool ready) {
+    constexpr int DPL = HD / 32, PITCH = step_kv_pitch(HD);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x, G = a.H / a.KV, KV = a.KV;
-    const int n_keys = min(p + 1, a.max_ctx);
-    const int chunks = (n_keys + 31) / 32, per = (chunks + a.splits - 1) / a.splits;
+    int n_keys, per, ns;
+    step_shares(a, p, n_keys, per, ns);
     const int key_lo = min(n_keys, z * per * 32), key_hi = min(n_keys, (z + 1) * per * 32);
+    const bool turn = p < a.max_ctx;                     // past the context nothing is rotated or appended
+    const bool fresh_here = turn && p >= key_lo && p < key_hi;
     for (int i = tid; i < G * (HD / 2); i += SMALL_THREADS) {
         const int g = i / (HD / 2), j = i % (HD / 2);
         const float2 v = __ldcg(reinterpret_cast<const float2 *>(a.qkv + (size_t)(kvh * G + g) * HD) + j), r = rot[j];
-        const bool turn = p < a.max_ctx;                 // past the context nothing is rotated
         qs[g * HD + 2 * j] = turn ? __fsub_rn(__fmul_rn(v.x, r.x), __fmul_rn(v.y, r.y)) : v.x;
         qs[g * HD + 2 * j + 1] = turn ? __fadd_rn(__fmul_rn(v.x, r.y), __fmul_rn(v.y, r.x)) : v.y;
     }
-    if (p < a.max_ctx && p >= key_lo && p < key_hi && tid < HD / 2) {     // this share holds the new key: append it
-        const size_t at = ((size_t)p * KV + kvh) * HD + 2 * tid;
-        const float2 k = __ldcg(reinterpret_cast<const float2 *>(a.qkv + (size_t)(a.H + kvh) * HD) + tid), r = rot[tid];
-        const float2 v = __ldcg(reinterpret_cast<const float2 *>(a.qkv + (size_t)(a.H + KV + kvh) * HD) + tid);
-        kc[at] = __float2half_rn(__fsub_rn(__fmul_rn(k.x, r.x), __fmul_rn(k.y, r.y)));
-        kc[at + 1] = __float2half_rn(__fadd_rn(__fmul_rn(k.x, r.y), __fmul_rn(k.y, r.x)));
-        vc[at] = __float2half_rn(v.x);
-        vc[at + 1] = __float2half_rn(v.y);
+    // the new key's halves, by threads whose warps have no head's rotation to wait for
+    __half2 fk = __half2half2(__ushort_as_half(0)), fv = fk;
+    const int ft = SMALL_THREADS - 1 - tid;
+    if (fresh_here && ft < HD / 2) {
+        const size_t at = ((size_t)p * KV + kvh) * HD + 2 * ft;
+        const float2 k = __ldcg(reinterpret_cast<const float2 *>(a.qkv + (size_t)(a.H + kvh) * HD) + ft), r = rot[ft];
+        const float2 v = __ldcg(reinterpret_cast<const float2 *>(a.qkv + (size_t)(a.H + KV + kvh) * HD) + ft);
+        fk = __halves2half2(__float2half_rn(__fsub_rn(__fmul_rn(k.x, r.x), __fmul_rn(k.y, r.y))),
+                            __float2half_rn(__fadd_rn(__fmul_rn(k.x, r.y), __fmul_rn(k.y, r.x))));
+        fv = __halves2half2(__float2half_rn(v.x), __float2half_rn(v.y));
+        *reinterpret_cast<__half2 *>(kc + at) = fk;
+        *reinterpret_cast<__half2 *>(vc + at) = fv;
     }
-    __syncthreads();
-    for (int g = warp; g < G; g += SMALL_WARPS) {
-        const float *q = qs + g * HD;
-        float m = -CUDART_INF_F, l = 0.f, acc[DPL];
+    float m[2], l[2], acc[2][DPL];                       // a warp's heads: warp and, with more than 16 heads to a KV head, warp + 16
 #pragma unroll
-        for (int i = 0; i < DPL; ++i) acc[i] = 0.f;
-        for (int k0 = key_lo; k0 < key_hi; k0 += 32) {
+    for (int h = 0; h < 2; ++h) {
+        m[h] = -CUDART_INF_F;
+        l[h] = 0.f;
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) acc[h][i] = 0.f;
+    }
+    bool ok = true;
+    for (int k0 = key_lo; k0 < key_hi; k0 += STEP_KEYS) {
+        if (!ready) {
+            __syncthreads();                             // the chunk before has been read
+            if (warp == 0) step_fetch_kv(smem_u32(kv), kc, vc, KV, HD, kvh, k0, key_hi, turn ? p : -1, kv_bar, lane);
+        }
+        ready = false;
+        if (fresh_here && p >= k0 && p < k0 + STEP_KEYS && ft < HD / 2) {
+            *reinterpret_cast<__half2 *>(kv + (p - k0) * PITCH + 4 * ft) = fk;
+            *reinterpret_cast<__half2 *>(kv + (STEP_KEYS + p - k0) * PITCH + 4 * ft) = fv;
+        }
+        ok = mbar_wait(kv_bar, phase) && ok;
+        phase ^= 1u;
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int g = warp + SMALL_WARPS * h;
+            if (g >= G) break;
+            const float *q = qs + g * HD;
             const int key = k0 + lane;
             float s = -CUDART_INF_F;
             if (key < key_hi) {
-                const uint4 *kr = reinterpret_cast<const uint4 *>(kc + ((size_t)key * KV + kvh) * HD);
+                const uint4 *kr = reinterpret_cast<const uint4 *>(kv + lane * PITCH);
                 float dot = 0.f;
 #pragma unroll
                 for (int c = 0; c < HD / 8; ++c) {
                     const uint4 u = kr[c];
                     const __half2 *hp = reinterpret_cast<const __half2 *>(&u);
+                    const float4 q0 = *reinterpret_cast<const float4 *>(q + 8 * c), q1 = *reinterpret_cast<const float4 *>(q + 8 * c + 4);
+                    const float qv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const float2 kf = __half22float2(hp[e]);
-                        dot = fmaf(q[8 * c + 2 * e], kf.x, dot);
-                        dot = fmaf(q[8 * c + 2 * e + 1], kf.y, dot);
+                        dot = fmaf(qv[2 * e], kf.x, dot);
+                        dot = fmaf(qv[2 * e + 1], kf.y, dot);
                     }
                 }
                 s = dot * a.scale;
@@ -184,38 +245,44 @@ __device__ __forceinline__ void step_attention(const StepArgs &a, __half *kc, __
             float cm = s;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
-            const float m_new = fmaxf(m, cm);
-            const float corr = expf(m - m_new);          // 0 on the first chunk (m = -inf)
+            const float m_new = fmaxf(m[h], cm);
+            const float corr = expf(m[h] - m_new);       // 0 on the first chunk (m = -inf)
             const float pr = key < key_hi ? expf(s - m_new) : 0.f;
             float ps = pr;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
-            l = l * corr + ps;
+            l[h] = l[h] * corr + ps;
 #pragma unroll
-            for (int i = 0; i < DPL; ++i) acc[i] *= corr;
+            for (int i = 0; i < DPL; ++i) acc[h][i] *= corr;
             const int nk = min(32, key_hi - k0);
+            const uint8_t *const vr = kv + STEP_KEYS * PITCH + 2 * DPL * lane;
 #pragma unroll 8
             for (int j = 0; j < nk; ++j) {
                 const float pj = __shfl_sync(0xffffffffu, pr, j);
-                const __half *vr = vc + ((size_t)(k0 + j) * KV + kvh) * HD + DPL * lane;
                 if (DPL == 4) {
-                    const uint2 u = *reinterpret_cast<const uint2 *>(vr);
+                    const uint2 u = *reinterpret_cast<const uint2 *>(vr + j * PITCH);
                     const float2 x = __half22float2(*reinterpret_cast<const __half2 *>(&u.x));
                     const float2 y = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
-                    acc[0] = fmaf(pj, x.x, acc[0]); acc[1] = fmaf(pj, x.y, acc[1]);
-                    acc[DPL - 2] = fmaf(pj, y.x, acc[DPL - 2]); acc[DPL - 1] = fmaf(pj, y.y, acc[DPL - 1]);
+                    acc[h][0] = fmaf(pj, x.x, acc[h][0]); acc[h][1] = fmaf(pj, x.y, acc[h][1]);
+                    acc[h][DPL - 2] = fmaf(pj, y.x, acc[h][DPL - 2]); acc[h][DPL - 1] = fmaf(pj, y.y, acc[h][DPL - 1]);
                 } else {
-#pragma unroll
-                    for (int i = 0; i < DPL; ++i) acc[i] = fmaf(pj, __half2float(vr[i]), acc[i]);
+                    const float2 x = __half22float2(*reinterpret_cast<const __half2 *>(vr + j * PITCH));
+                    acc[h][0] = fmaf(pj, x.x, acc[h][0]); acc[h][1] = fmaf(pj, x.y, acc[h][1]);
                 }
             }
-            m = m_new;
+            m[h] = m_new;
         }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int g = warp + SMALL_WARPS * h;
+        if (g >= G) break;
         float *pp = a.part + ((size_t)(kvh * G + g) * a.splits + z) * (HD + 2);
 #pragma unroll
-        for (int i = 0; i < DPL; ++i) pp[DPL * lane + i] = acc[i];
-        if (lane == 0) { pp[HD] = m; pp[HD + 1] = l; }
+        for (int i = 0; i < DPL; ++i) pp[DPL * lane + i] = acc[h][i];
+        if (lane == 0) { pp[HD] = m[h]; pp[HD + 1] = l[h]; }
     }
+    return ok;
 }
 // the first ns shares of a KV head, combined and quantised to Q8_0 (attention_merge_q8_0_kernel)
 template <int HD>
@@ -225,6 +292,20 @@ __device__ __forceinline__ void step_merge(const StepArgs &a, int kvh, int ns) {
     for (int g = warp; g < G; g += SMALL_WARPS) {
         const int hh = kvh * G + g;
         const float *pp = a.part + (size_t)hh * a.splits * (HD + 2);
+        // the first shares' sums are on their way before the largest score of all is known
+        constexpr int AHEAD = 4;
+        float lz[AHEAD], mz[AHEAD], v[AHEAD][DPL];
+        auto fetch = [&](int z0) {
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i) {
+                const float *pz = pp + min(z0 + i, ns - 1) * (HD + 2);
+                lz[i] = __ldcg(pz + HD + 1);
+                mz[i] = __ldcg(pz + HD);
+#pragma unroll
+                for (int d = 0; d < DPL; ++d) v[i][d] = __ldcg(pz + DPL * lane + d);
+            }
+        };
+        fetch(0);
         float mx = -CUDART_INF_F;
         for (int z = lane; z < ns; z += 32) mx = fmaxf(mx, __ldcg(pp + z * (HD + 2) + HD));
 #pragma unroll
@@ -232,17 +313,16 @@ __device__ __forceinline__ void step_merge(const StepArgs &a, int kvh, int ns) {
         float l = 0.f, acc[DPL];
 #pragma unroll
         for (int i = 0; i < DPL; ++i) acc[i] = 0.f;
-#pragma unroll 4
-        for (int z = 0; z < ns; ++z) {
-            const float lz = __ldcg(pp + z * (HD + 2) + HD + 1), mz = __ldcg(pp + z * (HD + 2) + HD);
-            float v[DPL];
+        for (int z0 = 0; z0 < ns; z0 += AHEAD) {
+            if (z0 > 0) fetch(z0);
 #pragma unroll
-            for (int i = 0; i < DPL; ++i) v[i] = __ldcg(pp + z * (HD + 2) + DPL * lane + i);
-            if (lz == 0.f) continue;
-            const float wz = expf(mz - mx);
-            l = fmaf(wz, lz, l);
+            for (int i = 0; i < AHEAD; ++i) {
+                if (z0 + i >= ns || lz[i] == 0.f) continue;
+                const float wz = expf(mz[i] - mx);
+                l = fmaf(wz, lz[i], l);
 #pragma unroll
-            for (int i = 0; i < DPL; ++i) acc[i] = fmaf(wz, v[i], acc[i]);
+                for (int d = 0; d < DPL; ++d) acc[d] = fmaf(wz, v[i][d], acc[d]);
+            }
         }
         const float inv = 1.0f / l;
         float amax = 0.f;
@@ -262,14 +342,15 @@ __device__ __forceinline__ void step_merge(const StepArgs &a, int kvh, int ns) {
 
 template <int GU, int DN, SmallSums SUMS>
 __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const StepArgs a) {
-    // a staging area per warp | x [D] | quantised row [max(D, H HD)] and its scales | rotated heads [G][HD] | packed input row | packed
-    // SwiGLU rows | probabilities and scores
+    // a staging area per warp | quantised row [max(D, H HD)] and its scales | rotated heads [G][HD] | x [D] | packed input row | packed
+    // SwiGLU rows | probabilities and scores.  From x on the memory holds a chunk of keys and values while attention runs.
     extern __shared__ __align__(128) uint8_t dyn[];
     __shared__ float s_part[SMALL_WARPS], s_w[SMALL_PAIRS];
     __shared__ int s_ids[SMALL_PAIRS];
     __shared__ unsigned s_last;
     __shared__ unsigned long long s_best[SMALL_WARPS];
     __shared__ float2 s_rot[64];
+    __shared__ __align__(8) uint64_t s_kv_bar;
     __shared__ __align__(16) uint8_t s_layer_raw[sizeof(StepLayer)];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.D, QO = a.H * a.HD, G = a.H / a.KV;
     const int widest = D > QO ? D : QO, cols = (a.H + 2 * a.KV) * a.HD, rbd = D / 32 * 34, rbo = QO / 32 * 34;
@@ -277,11 +358,12 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
     const SmallArgs &moe = s_layer.moe;
     SmallShared s;
     s.stage = smem_u32(dyn) + (uint32_t)(warp * a.stage);
-    float *const x = reinterpret_cast<float *>(dyn + SMALL_WARPS * a.stage);
-    int8_t *const xq = reinterpret_cast<int8_t *>(x + D);
+    int8_t *const xq = reinterpret_cast<int8_t *>(dyn + SMALL_WARPS * a.stage);
     float *const xd = reinterpret_cast<float *>(xq + widest);
     float *const qs = xd + ((widest / 32 + 3) & ~3);
-    s.q8x = reinterpret_cast<uint8_t *>(qs + G * a.HD);
+    float *const x = qs + G * a.HD;
+    uint8_t *const kv = reinterpret_cast<uint8_t *>(x);
+    s.q8x = reinterpret_cast<uint8_t *>(x + D);
     s.q8f = s.q8x + q8row_stride(D);
     s.prob = nullptr;                                    // set per layer: it follows the SwiGLU rows
     s.ids = s_ids; s.w = s_w; s.part = s_part;
@@ -291,6 +373,10 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
             reinterpret_cast<uint32_t *>(s_layer_raw)[i] = reinterpret_cast<const uint32_t *>(a.layers + l)[i];
         __syncthreads();
     };
+    if (tid == 0) {
+        mbar_init(&s_kv_bar, 1);
+        mbar_init_fence();
+    }
     load_layer(0);
     step_prefetch(s.stage, s_layer.wqkv, cols, rbd, a.depth_q);
     pdl_wait_prior_grid();
@@ -322,30 +408,39 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
         for (int i = tid; i < D / 4; i += SMALL_THREADS) reinterpret_cast<float4 *>(x)[i] = __ldcg(reinterpret_cast<const float4 *>(a.h) + i);
         __syncthreads();
     };
+    uint32_t kv_phase = 0;
+    int n_keys, per, ns;
+    step_shares(a, p, n_keys, per, ns);
     for (int l = 0; l < a.n_layers; ++l) {
+        const size_t layer_kv = (size_t)l * a.max_ctx * a.KV * a.HD;
         if (l > 0) load_h();
         s.prob = reinterpret_cast<float *>(s.q8f + moe.K * q8row_stride(moe.F));
         step_norm(x, s_layer.attn_norm, D, a.eps, s_part);
         step_quantise(x, xq, xd, D);
+        if (warp == 0 && blockIdx.x < a.KV * ns) {       // x is free: the first keys and values that this CTA will meet
+            const int z = blockIdx.x % ns;
+            step_fetch_kv(smem_u32(kv), a.kc + layer_kv, a.vc + layer_kv, a.KV, a.HD, blockIdx.x / ns, min(n_keys, z * per * 32),
+                          min(n_keys, (z + 1) * per * 32), p < a.max_ctx ? p : -1, &s_kv_bar, lane);
+        }
         step_rows(s.stage, s_layer.wqkv, cols, rbd, a.depth_q, xq, xd, [&](int o, float v) { a.qkv[o] = v; });
         step_prefetch(s.stage, s_layer.wo, D, rbo, a.depth_o);
         small_prefetch_router(moe);
         barrier();
         // ---- attention: a CTA per share of a KV head that has keys ----
         {
-            const int chunks = (min(p + 1, a.max_ctx) + 31) / 32, per = (chunks + a.splits - 1) / a.splits, ns = (chunks + per - 1) / per;
-            const size_t layer_kv = (size_t)l * a.max_ctx * a.KV * a.HD;
             for (int u = blockIdx.x; u < a.KV * ns; u += gridDim.x) {
                 const int kvh = u / ns, z = u % ns;
+                const bool first = u == (int)blockIdx.x;
+                if (!first) __syncthreads();             // qs is still read
+                const bool ok = a.HD == 128 ? step_attention<128>(a, a.kc + layer_kv, a.vc + layer_kv, kvh, z, p, qs, s_rot, kv, &s_kv_bar, kv_phase, first)
+                                            : step_attention<64>(a, a.kc + layer_kv, a.vc + layer_kv, kvh, z, p, qs, s_rot, kv, &s_kv_bar, kv_phase, first);
+                if (!ok && tid == 0)
+                    for (int i = 0; i < a.n_layers; ++i) atomicExch(a.layers[i].moe.err, 21);
                 __syncthreads();
-                if (a.HD == 128) step_attention<128>(a, a.kc + layer_kv, a.vc + layer_kv, kvh, z, p, qs, s_rot);
-                else step_attention<64>(a, a.kc + layer_kv, a.vc + layer_kv, kvh, z, p, qs, s_rot);
-                __threadfence();
-                __syncthreads();
-                if (tid == 0) s_last = atomicAdd(a.head_ticket + kvh, 1u);
+                // one thread's release and acquire order what the CTA wrote and what it reads next
+                if (tid == 0) asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(s_last) : "l"(a.head_ticket + kvh) : "memory");
                 __syncthreads();
                 if (s_last == (unsigned)ns - 1) {
-                    __threadfence();
                     if (a.HD == 128) step_merge<128>(a, kvh, ns); else step_merge<64>(a, kvh, ns);
                     if (tid == 0) a.head_ticket[kvh] = 0u;
                 }
