@@ -69,27 +69,31 @@ __device__ __forceinline__ float step_row_dot(uint32_t row, const int8_t *aq, co
 }
 
 // rows gw, gw + W, ... of a Q8_0 matrix, the first `depth` of them on their way (step_prefetch) before the activations are there
-__device__ __forceinline__ void step_fetch(uint32_t stage, const uint8_t *w, int n_rows, int rb, int o, int slot, int lane) {
-    if (o < n_rows) small_stage(stage + (uint32_t)(slot * ((rb + 47) & ~15)), w, (size_t)n_rows * rb, (size_t)o * rb, rb, lane);
-    small_commit();
+__device__ __forceinline__ void step_fetch(const SmallShared &s, const uint8_t *w, int n_rows, int rb, int o, int slot, int lane) {
+    if (o >= n_rows) return;
+    if (lane == 0) {
+        small_stage(s.stage + (uint32_t)(slot * ((rb + 47) & ~15)), w, (size_t)n_rows * rb, (size_t)o * rb, rb, &s.bars[slot]);
+        mbar_arrive(&s.bars[slot]);
+    }
+    __syncwarp();
 }
-__device__ __forceinline__ void step_prefetch(uint32_t stage, const uint8_t *w, int n_rows, int rb, int depth) {
+__device__ __forceinline__ void step_prefetch(const SmallShared &s, const uint8_t *w, int n_rows, int rb, int depth) {
     const int gw = blockIdx.x * SMALL_WARPS + (threadIdx.x >> 5), W = gridDim.x * SMALL_WARPS;
-    for (int i = 0; i < depth; ++i) step_fetch(stage, w, n_rows, rb, gw + i * W, i, threadIdx.x & 31);
+#pragma unroll 1
+    for (int i = 0; i < depth; ++i) step_fetch(s, w, n_rows, rb, gw + i * W, i, threadIdx.x & 31);
 }
 template <typename Put>
-__device__ __forceinline__ void step_rows(uint32_t stage, const uint8_t *w, int n_rows, int rb, int depth, const int8_t *aq, const float *ad, Put put) {
+__device__ __forceinline__ void step_rows(SmallShared &s, const uint8_t *w, int n_rows, int rb, int depth, const int8_t *aq, const float *ad, Put put) {
     const int lane = threadIdx.x & 31, gw = blockIdx.x * SMALL_WARPS + (threadIdx.x >> 5), W = gridDim.x * SMALL_WARPS;
     int slot = 0;
     for (int o = gw; o < n_rows; o += W) {
-        small_wait(depth - 1);
-        const float v = step_row_dot(stage + (uint32_t)(slot * ((rb + 47) & ~15)) + (uint32_t)(((size_t)o * rb) & 15), aq, ad, rb / 34, lane);
+        small_wait(s, slot);
+        const float v = step_row_dot(s.stage + (uint32_t)(slot * ((rb + 47) & ~15)) + (uint32_t)(((size_t)o * rb) & 15), aq, ad, rb / 34, lane);
         if (lane == 0) put(o, v);
         __syncwarp();
-        step_fetch(stage, w, n_rows, rb, o + depth * W, slot, lane);
+        step_fetch(s, w, n_rows, rb, o + depth * W, slot, lane);
         slot = slot + 1 == depth ? 0 : slot + 1;
     }
-    small_wait(0);
 }
 
 // x <- RMSNorm(x) * w, in shared memory, by the whole CTA.  The sum of squares is that of rmsnorm_kernel, by 256 threads in its order.
@@ -148,21 +152,24 @@ __device__ __forceinline__ void step_shares(const StepArgs &a, int p, int &n_key
     per = (chunks + a.splits - 1) / a.splits;
     ns = (chunks + per - 1) / per;
 }
-// rows [k0, k0 + 32) of one KV head up to key `end`, without the new one (it is written by the share that holds it), by one warp
-__device__ __forceinline__ void step_fetch_kv(uint32_t kv, const __half *kc, const __half *vc, int KV, int HD, int kvh, int k0, int end, int fresh, uint64_t *bar,
-                                              int lane) {
-    const int key = k0 + lane, n = max(0, min(STEP_KEYS, end - k0)) - (fresh >= k0 && fresh < min(end, k0 + STEP_KEYS) ? 1 : 0);
+// rows [k0, k0 + 32) of one KV head up to key `end`, without the new one (it is written by the share that holds it); called by all
+// warps, which take two keys each (64 copies of one warp kept its rows waiting for 2 800 cycles)
+__device__ __forceinline__ void step_fetch_kv(uint32_t kv, const __half *kc, const __half *vc, int KV, int HD, int kvh, int k0, int end, int fresh, uint64_t *bar) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // what was read and written in this memory before, by ordinary loads and stores, comes before the copies
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)(4 * HD * n));
-    __syncwarp();
-    if (key < end && key != fresh) {
-        const size_t at = ((size_t)key * KV + kvh) * HD;
-        const uint32_t dst = kv + (uint32_t)(lane * step_kv_pitch(HD));
-        bulk_g2s_addr(dst, kc + at, (uint32_t)(2 * HD), bar);
-        bulk_g2s_addr(dst + (uint32_t)(STEP_KEYS * step_kv_pitch(HD)), vc + at, (uint32_t)(2 * HD), bar);
+    if (threadIdx.x == 0) {
+        const int n = max(0, min(STEP_KEYS, end - k0)) - (fresh >= k0 && fresh < min(end, k0 + STEP_KEYS) ? 1 : 0);
+        mbar_arrive_expect_tx(bar, (uint32_t)(4 * HD * n));
     }
+    const int row = 2 * warp + (lane >> 1), key = k0 + row;
+    if (lane < 4 && key < end && key != fresh) {
+        const uint32_t dst = kv + (uint32_t)((row + (lane & 1) * STEP_KEYS) * step_kv_pitch(HD));
+        bulk_g2s_addr(dst, (lane & 1 ? vc : kc) + ((size_t)key * KV + kvh) * HD, (uint32_t)(2 * HD), bar);
+    }
+    __syncwarp();
 }
+static_assert(2 * SMALL_WARPS == STEP_KEYS, "keys of a warp");
 
 // Share z of a KV head's keys: attention_kernel with the rotation of q and of the new key folded in.  qs: [G][HD] shared; kv: the chunk;
 // ready: its first chunk is on its way already.  phase: of kv_bar, moved on with every chunk.  False: a wait ran out.
@@ -207,7 +214,7 @@ __device__ __forceinline__ bool step_attention(const StepArgs &a, __half *kc, __
     for (int k0 = key_lo; k0 < key_hi; k0 += STEP_KEYS) {
         if (!ready) {
             __syncthreads();                             // the chunk before has been read
-            if (warp == 0) step_fetch_kv(smem_u32(kv), kc, vc, KV, HD, kvh, k0, key_hi, turn ? p : -1, kv_bar, lane);
+            step_fetch_kv(smem_u32(kv), kc, vc, KV, HD, kvh, k0, key_hi, turn ? p : -1, kv_bar);
         }
         ready = false;
         if (fresh_here && p >= k0 && p < k0 + STEP_KEYS && ft < HD / 2) {
@@ -346,7 +353,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
     // SwiGLU rows | probabilities and scores.  From x on the memory holds a chunk of keys and values while attention runs.
     extern __shared__ __align__(128) uint8_t dyn[];
     __shared__ float s_part[SMALL_WARPS], s_w[SMALL_PAIRS];
-    __shared__ int s_ids[SMALL_PAIRS];
+    __shared__ int s_ids[SMALL_PAIRS], s_late;
+    __shared__ __align__(8) uint64_t s_bars[SMALL_WARPS][SMALL_SLOTS];
     __shared__ unsigned s_last;
     __shared__ unsigned long long s_best[SMALL_WARPS];
     __shared__ float2 s_rot[64];
@@ -373,12 +381,11 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
             reinterpret_cast<uint32_t *>(s_layer_raw)[i] = reinterpret_cast<const uint32_t *>(a.layers + l)[i];
         __syncthreads();
     };
-    if (tid == 0) {
-        mbar_init(&s_kv_bar, 1);
-        mbar_init_fence();
-    }
+    s.bars = s_bars[warp]; s.phase = 0; s.late = &s_late;
+    if (tid == 0) mbar_init(&s_kv_bar, 1);
+    small_init(s_bars, &s_late);
     load_layer(0);
-    step_prefetch(s.stage, s_layer.wqkv, cols, rbd, a.depth_q);
+    step_prefetch(s, s_layer.wqkv, cols, rbd, a.depth_q);
     pdl_wait_prior_grid();
     pdl_launch_dependents();
     const int p = *a.pos;
@@ -399,11 +406,10 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
     __syncthreads();
     unsigned n_bar = 0;
     // a wait that runs out is seen through every layer's context, as it would be after the separate launches of that layer
-    auto barrier = [&]() {
-        small_grid_barrier(a.bar, ++n_bar, [&]() {
-            for (int l = 0; l < a.n_layers; ++l) atomicExch(a.layers[l].moe.err, 21);
-        });
+    auto expired = [&]() {
+        for (int l = 0; l < a.n_layers; ++l) atomicExch(a.layers[l].moe.err, 21);
     };
+    auto barrier = [&]() { small_grid_barrier(a.bar, ++n_bar, expired); };
     auto load_h = [&]() {
         for (int i = tid; i < D / 4; i += SMALL_THREADS) reinterpret_cast<float4 *>(x)[i] = __ldcg(reinterpret_cast<const float4 *>(a.h) + i);
         __syncthreads();
@@ -417,13 +423,13 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
         s.prob = reinterpret_cast<float *>(s.q8f + moe.K * q8row_stride(moe.F));
         step_norm(x, s_layer.attn_norm, D, a.eps, s_part);
         step_quantise(x, xq, xd, D);
-        if (warp == 0 && blockIdx.x < a.KV * ns) {       // x is free: the first keys and values that this CTA will meet
+        if (blockIdx.x < a.KV * ns) {       // x is free: the first keys and values that this CTA will meet
             const int z = blockIdx.x % ns;
             step_fetch_kv(smem_u32(kv), a.kc + layer_kv, a.vc + layer_kv, a.KV, a.HD, blockIdx.x / ns, min(n_keys, z * per * 32),
-                          min(n_keys, (z + 1) * per * 32), p < a.max_ctx ? p : -1, &s_kv_bar, lane);
+                          min(n_keys, (z + 1) * per * 32), p < a.max_ctx ? p : -1, &s_kv_bar);
         }
-        step_rows(s.stage, s_layer.wqkv, cols, rbd, a.depth_q, xq, xd, [&](int o, float v) { a.qkv[o] = v; });
-        step_prefetch(s.stage, s_layer.wo, D, rbo, a.depth_o);
+        step_rows(s, s_layer.wqkv, cols, rbd, a.depth_q, xq, xd, [&](int o, float v) { a.qkv[o] = v; });
+        step_prefetch(s, s_layer.wo, D, rbo, a.depth_o);
         small_prefetch_router(moe);
         barrier();
         // ---- attention: a CTA per share of a KV head that has keys ----
@@ -434,8 +440,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
                 if (!first) __syncthreads();             // qs is still read
                 const bool ok = a.HD == 128 ? step_attention<128>(a, a.kc + layer_kv, a.vc + layer_kv, kvh, z, p, qs, s_rot, kv, &s_kv_bar, kv_phase, first)
                                             : step_attention<64>(a, a.kc + layer_kv, a.vc + layer_kv, kvh, z, p, qs, s_rot, kv, &s_kv_bar, kv_phase, first);
-                if (!ok && tid == 0)
-                    for (int i = 0; i < a.n_layers; ++i) atomicExch(a.layers[i].moe.err, 21);
+                if (!ok) s_late = 1;
                 __syncthreads();
                 // one thread's release and acquire order what the CTA wrote and what it reads next
                 if (tid == 0) asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(s_last) : "l"(a.head_ticket + kvh) : "memory");
@@ -451,7 +456,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
         for (int i = tid; i < QO / 16; i += SMALL_THREADS) reinterpret_cast<uint4 *>(xq)[i] = __ldcg(reinterpret_cast<const uint4 *>(a.aq) + i);
         for (int i = tid; i < QO / 32; i += SMALL_THREADS) xd[i] = __ldcg(a.ad + i);
         __syncthreads();
-        step_rows(s.stage, s_layer.wo, D, rbo, a.depth_o, xq, xd, [&](int o, float v) { a.h[o] = __ldcg(a.h + o) + v; });
+        step_rows(s, s_layer.wo, D, rbo, a.depth_o, xq, xd, [&](int o, float v) { a.h[o] = __ldcg(a.h + o) + v; });
         barrier();
         // ---- MoE block ----
         load_h();
@@ -459,7 +464,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
         small_logits<GU>(moe, s, x);
         barrier();
         small_gate_up<GU, SUMS>(moe, s);
-        small_prefetch_down(moe, s);
+        small_prefetch_down<SUMS != SUMS_BLOCKS>(moe, s);
         barrier();
         small_down<DN, SUMS>(moe, s);
         if (s_layer.leave_state && blockIdx.x == gridDim.x - 1) {
@@ -469,9 +474,9 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
         }
         if (l + 1 < a.n_layers) {
             load_layer(l + 1);
-            step_prefetch(s.stage, s_layer.wqkv, cols, rbd, a.depth_q);
+            step_prefetch(s, s_layer.wqkv, cols, rbd, a.depth_q);
         } else {
-            step_prefetch(s.stage, a.head, a.vocab, rbd, a.depth_q);
+            step_prefetch(s, a.head, a.vocab, rbd, a.depth_q);
         }
         barrier();
     }
@@ -480,7 +485,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
     step_norm(x, a.out_norm, D, a.eps, s_part);
     step_quantise(x, xq, xd, D);
     unsigned long long best = 0ull;
-    step_rows(s.stage, a.head, a.vocab, rbd, a.depth_q, xq, xd, [&](int o, float v) {
+    step_rows(s, a.head, a.vocab, rbd, a.depth_q, xq, xd, [&](int o, float v) {
         a.logits[o] = v;
         if (!isnan(v)) {
             const unsigned u = __float_as_uint(__fadd_rn(v, 0.f));
@@ -491,6 +496,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) decoder_step_kernel(const St
     if (lane == 0) s_best[warp] = best;
     __syncthreads();
     if (tid == 0) {
+        if (s_late) expired();
         for (int i = 1; i < SMALL_WARPS; ++i) best = s_best[i] > best ? s_best[i] : best;
         if (best) atomicMax(a.best, best);
         __threadfence();

@@ -11,7 +11,7 @@
 //   1  the CTA's experts' logits for all tokens; the tokens' rows quantised to Q8_K, by every CTA for itself
 //   -- barrier --
 //   2  top-k, by every CTA for itself, one warp per token; then gate / up: a warp takes row r of a pair, its bytes copied to shared
-//      memory by 16-byte asynchronous copies, several rows ahead
+//      memory by bulk copies, several rows ahead
 //   -- barrier, with the first down rows already on their way --
 //   3  the pairs' SwiGLU rows quantised, by every CTA for itself; then down: a warp takes output element d of a token, groups of its lanes
 //      multiply the rows d of its K experts side by side, and the weighted sum in k order needs no other warp
@@ -32,6 +32,7 @@ namespace zmoe {
 
 constexpr int SMALL_WARPS = 16, SMALL_THREADS = 32 * SMALL_WARPS;
 constexpr int SMALL_PAIRS = 32;      // most pairs of a call
+constexpr int SMALL_SLOTS = 4;       // most slots of a warp's staging area: rows (pairs of rows, K rows) on their way
 
 // A selection score as an integer that orders like it, 0 for none (a NaN); -0 counts as 0 and -inf is a candidate
 __device__ __forceinline__ unsigned score_key(float s) {
@@ -146,6 +147,9 @@ SmallArgs small_args(const RouterArgs &r, const SmallLaunch &L);   // all but th
 // a CTA's shared memory
 struct SmallShared {
     uint32_t stage;                  // this warp's staging area
+    uint64_t *bars;                  // [SMALL_SLOTS] this warp's: the rows of a slot of the area have landed
+    uint32_t phase;                  // the slots' next phases, a bit each
+    int *late;                       // set where a wait ran out
     uint8_t *q8x, *q8f;              // packed rows of the input [T] and of the SwiGLU output [T * K]
     float *prob;                     // probabilities and selection scores, 2 E floats per token
     int *ids;                        // [SMALL_PAIRS]
@@ -181,26 +185,42 @@ __device__ __forceinline__ void small_leave(unsigned *bar) {
     }
 }
 
-// `bytes` bytes at byte `at` of a tensor of `total` bytes go to dst, keeping their offset from a 16-byte boundary.  dst has room for
-// bytes + 32; only whole 16-byte pieces of the tensor are read, but for its last, which may be short.
-__device__ __forceinline__ void small_stage(uint32_t dst, const uint8_t *w, size_t total, size_t at, int bytes, int lane) {
+// `bytes` bytes at byte `at` of a tensor of `total` bytes go to dst, keeping their offset from a 16-byte boundary; called by one lane.
+// dst has room for bytes + 32; only whole 16-byte pieces of the tensor are read, but for its last, which may be short.
+// One bulk copy per row and not 16 bytes per lane: those wait at the load / store unit for the rows before them, so that a warp multiplied
+// its first row only when its last was nearly there, and came to the grid's barrier late by what it had sent for beforehand (a
+// layer of 2048 / 768, one token: fetching 4 200 cycles before gate / up, 4 400 before the barrier after it).
+__device__ __forceinline__ void small_stage(uint32_t dst, const uint8_t *w, size_t total, size_t at, int bytes, uint64_t *bar) {
     const int off = (int)(at & 15);
     const size_t g0 = at - off;
-    const int n = (off + bytes + 15) >> 4;
-    for (int c = lane; c < n; c += 32) {
-        const size_t g = g0 + 16 * (size_t)c;
-        const int have = g + 16 <= total ? 16 : (int)(total - g);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 16 * c), "l"(w + g), "r"(have) : "memory");
+    int n = (off + bytes + 15) & ~15;
+    if (g0 + (size_t)n > total) {                        // the tensor's last row
+        n -= 16;
+        for (size_t i = g0 + n; i < total; ++i) {
+            const uint32_t v = w[i];
+            asm volatile("st.shared.u8 [%0], %1;" ::"r"(dst + (uint32_t)(i - g0)), "r"(v) : "memory");
+        }
+        if (n == 0) return;
     }
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
+    bulk_g2s_addr(dst, w + g0, (uint32_t)n, bar);
 }
-__device__ __forceinline__ void small_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// at most n groups of copies still on their way (n up to 3)
-__device__ __forceinline__ void small_wait(int n) {
-    if (n <= 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
-    else if (n == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
-    else if (n == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
-    else asm volatile("cp.async.wait_group 3;" ::: "memory");
+// after a slot's copies have been issued; called by the warp
+__device__ __forceinline__ void small_issued(uint64_t *bar, int lane) {
     __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
+// a slot's rows have landed
+__device__ __forceinline__ void small_wait(SmallShared &s, int slot) {
+    if (!mbar_wait(&s.bars[slot], (s.phase >> slot) & 1u)) *s.late = 1;
+    s.phase ^= 1u << slot;
+    __syncwarp();
+}
+// The kernel's barriers; called by all threads, before a CTA barrier that orders them before their use
+__device__ __forceinline__ void small_init(uint64_t (*bars)[SMALL_SLOTS], int *late) {
+    if (threadIdx.x < SMALL_WARPS * SMALL_SLOTS) mbar_init(&bars[0][0] + threadIdx.x, 1);
+    if (threadIdx.x == 0) *late = 0;
+    mbar_init_fence();
 }
 
 __device__ __forceinline__ void small_prefetch_router(const SmallArgs &a) {
@@ -280,7 +300,7 @@ __device__ __forceinline__ void small_add(float &v, int is, int ms, float d, flo
 
 // phase 2: routes, then SwiGLU(gate, up) of the warp's rows into a.act
 template <int GU, SmallSums SUMS>
-__device__ __forceinline__ void small_gate_up(const SmallArgs &a, const SmallShared &s) {
+__device__ __forceinline__ void small_gate_up(const SmallArgs &a, SmallShared &s) {
     constexpr bool ONE = SUMS != SUMS_BLOCKS, SHORT = SUMS == SUMS_SHORT;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.D, F = a.F, E = a.E, K = a.K;
     if (warp < a.T) {
@@ -292,16 +312,26 @@ __device__ __forceinline__ void small_gate_up(const SmallArgs &a, const SmallSha
     __syncthreads();
     const int gw = blockIdx.x * SMALL_WARPS + warp, W = gridDim.x * SMALL_WARPS;
     const int n_units = a.T * K * F, room = (a.rb_gu + 47) & ~15, str = q8row_stride(D), U = D / 64;
-    auto fetch = [&](int u, int slot) {
-        if (u < n_units) {
-            const int p = u / F, e = s.ids[p];
-            const size_t at = (size_t)(u - p * F) * a.rb_gu;
-            small_stage(s.stage + (uint32_t)(2 * slot * room), a.wg, a.tg, (size_t)e * a.sg + at, a.rb_gu, lane);
-            small_stage(s.stage + (uint32_t)((2 * slot + 1) * room), a.wu, a.tu, (size_t)e * a.su + at, a.rb_gu, lane);
-        }
-        small_commit();
+    // unit u is row u % F of pair u / F; the next of the warp's units to fetch and the one at hand move on by W, without divisions
+    const int step_p = W / F, step_r = W - step_p * F;
+    int fu = gw, fp = gw / F, fr = gw - fp * F, p = fp, r = fr;
+    auto move_on = [&](int &pair, int &row) {
+        pair += step_p;
+        row += step_r;
+        if (row >= F) { row -= F; ++pair; }
     };
-    for (int i = 0; i < a.depth_gu; ++i) fetch(gw + i * W, i);
+    auto fetch = [&](int slot) {
+        if (fu < n_units) {
+            if (lane < 2)                                // one lane a matrix
+                small_stage(s.stage + (uint32_t)((2 * slot + lane) * room), lane ? a.wu : a.wg, lane ? a.tu : a.tg,
+                            (size_t)(uint32_t)s.ids[fp] * (lane ? a.su : a.sg) + (size_t)(uint32_t)fr * (uint32_t)a.rb_gu, a.rb_gu, &s.bars[slot]);
+            small_issued(&s.bars[slot], lane);
+        }
+        fu += W;
+        move_on(fp, fr);
+    };
+#pragma unroll 1
+    for (int i = 0; i < a.depth_gu; ++i) fetch(i);
     UnitAct mine;                                          // one token: the lane's unit of its row, for all weight rows
     mine.d = 0.f;
     if (ONE && (SHORT || U <= 32) && lane < U) load_unit_act<GU>(smem_u32(s.q8x), D, lane, mine);
@@ -309,11 +339,10 @@ __device__ __forceinline__ void small_gate_up(const SmallArgs &a, const SmallSha
     const int keeper = ONE && (SHORT || U <= 32) ? (U - 1) & ~7 : 0;   // first of the eight lanes
     int n_done = 0, slot = 0;
     for (int u = gw; u < n_units; u += W, ++n_done) {
-        small_wait(a.depth_gu - 1);
-        const int p = u / F, r = u - p * F, e = s.ids[p];
-        const uint32_t bg = s.stage + (uint32_t)(2 * slot * room) + (uint32_t)(((size_t)e * a.sg + (size_t)r * a.rb_gu) & 15);
-        const uint32_t bu = s.stage + (uint32_t)((2 * slot + 1) * room) + (uint32_t)(((size_t)e * a.su + (size_t)r * a.rb_gu) & 15);
-        const uint32_t row = smem_u32(s.q8x) + (uint32_t)((p / K) * str);
+        small_wait(s, slot);
+        const uint32_t off = ((uint32_t)r * (uint32_t)a.rb_gu) & 15u;    // experts lie a multiple of 16 bytes apart
+        const uint32_t bg = s.stage + (uint32_t)(2 * slot * room) + off, bu = s.stage + (uint32_t)((2 * slot + 1) * room) + off;
+        const uint32_t row = smem_u32(s.q8x) + (uint32_t)(ONE ? 0 : (p / K) * str);
         float g = 0.f, v = 0.f;
         if (SHORT || (ONE && U <= 32)) {
             // A unit per lane, added up as by the eight lanes that mmid_kernel gives a row: lane l of eight takes units l, l + 8, .. in turn.
@@ -369,8 +398,9 @@ __device__ __forceinline__ void small_gate_up(const SmallArgs &a, const SmallSha
         // lane i of the eight that hold the sums keeps the i-th row's: SwiGLU runs once for all rows (once per 8)
         if (lane == keeper + (n_done & 7)) { keep_g = g; keep_u = v; }
         __syncwarp();
-        fetch(u + a.depth_gu * W, slot);
+        fetch(slot);
         slot = slot + 1 == a.depth_gu ? 0 : slot + 1;
+        move_on(p, r);
         if (u + W >= n_units || (n_done & 7) == 7) {
             const int nth = lane - keeper, at = u + (nth - (n_done & 7)) * W;
             if (nth >= 0 && nth <= (n_done & 7)) {
@@ -379,27 +409,30 @@ __device__ __forceinline__ void small_gate_up(const SmallArgs &a, const SmallSha
             }
         }
     }
-    small_wait(0);
 }
 
-// the first down rows of the warp on their way (before the barrier that completes a.act)
+// the first down rows of the warp on their way (before the barrier that completes a.act).  ONE: one token
+template <bool ONE>
 __device__ __forceinline__ void small_fetch_down(const SmallArgs &a, const SmallShared &s, int u, int slot) {
     const int D = a.D, K = a.K, room = (a.rb_dn + 47) & ~15, lane = threadIdx.x & 31;
     if (u < a.T * D) {
-        const int t = u / D, d = u - t * D;
-        for (int k = 0; k < K; ++k)
-            small_stage(s.stage + (uint32_t)((slot * K + k) * room), a.wd, a.td, (size_t)s.ids[t * K + k] * a.sd + (size_t)d * a.rb_dn, a.rb_dn, lane);
+        const int t = ONE ? 0 : u / D, d = u - t * D;
+        if (lane < K)                                    // one lane a row (K is at most 32)
+            small_stage(s.stage + (uint32_t)((slot * K + lane) * room), a.wd, a.td,
+                        (size_t)(uint32_t)s.ids[t * K + lane] * a.sd + (size_t)(uint32_t)d * (uint32_t)a.rb_dn, a.rb_dn, &s.bars[slot]);
+        small_issued(&s.bars[slot], lane);
     }
-    small_commit();
 }
+template <bool ONE>
 __device__ __forceinline__ void small_prefetch_down(const SmallArgs &a, const SmallShared &s) {
     const int gw = blockIdx.x * SMALL_WARPS + (threadIdx.x >> 5), W = gridDim.x * SMALL_WARPS;
-    for (int i = 0; i < a.depth_dn; ++i) small_fetch_down(a, s, gw + i * W, i);
+#pragma unroll 1
+    for (int i = 0; i < a.depth_dn; ++i) small_fetch_down<ONE>(a, s, gw + i * W, i);
 }
 
 // phase 3 (after small_prefetch_down and the barrier)
 template <int DN, SmallSums SUMS>
-__device__ __forceinline__ void small_down(const SmallArgs &a, const SmallShared &s) {
+__device__ __forceinline__ void small_down(const SmallArgs &a, SmallShared &s) {
     constexpr bool ONE = SUMS != SUMS_BLOCKS, SHORT = SUMS == SUMS_SHORT;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.D, F = a.F, K = a.K, P = a.T * K;
     const int nb = F / QK_K, str = q8row_stride(F), U = F / 64, room = (a.rb_dn + 47) & ~15;
@@ -409,8 +442,9 @@ __device__ __forceinline__ void small_down(const SmallArgs &a, const SmallShared
     const int gw = blockIdx.x * SMALL_WARPS + warp, W = gridDim.x * SMALL_WARPS;
     int slot = 0;
     for (int u = gw; u < a.T * D; u += W) {
-        small_wait(a.depth_dn - 1);
-        const int t = u / D, d = u - t * D;
+        small_wait(s, slot);
+        const int t = ONE ? 0 : u / D, d = u - t * D;
+        const uint32_t off = ((uint32_t)d * (uint32_t)a.rb_dn) & 15u;    // experts lie a multiple of 16 bytes apart
         float acc = 0.f;
         // separately rounded products and sums in k order, from the sums of rows k0, k0 + 1, .. in every LPR-th lane
         auto add = [&](int k0, float v, auto lanes) {
@@ -426,7 +460,7 @@ __device__ __forceinline__ void small_down(const SmallArgs &a, const SmallShared
         };
         auto row_of = [&](int k, uint32_t &blk, uint32_t &row) {
             const int p = t * K + k;
-            blk = s.stage + (uint32_t)((slot * K + k) * room) + (uint32_t)(((size_t)s.ids[p] * a.sd + (size_t)d * a.rb_dn) & 15);
+            blk = s.stage + (uint32_t)((slot * K + k) * room) + off;
             row = smem_u32(s.q8f) + (uint32_t)(p * str);
         };
         // lanes per row: eight, four rows at once, or the whole warp for rows of more than 32 units
@@ -488,10 +522,9 @@ __device__ __forceinline__ void small_down(const SmallArgs &a, const SmallShared
         }
         if (lane == 0) a.out[u] = a.accumulate ? __fadd_rn(__ldcg(a.out + u), acc) : acc;
         __syncwarp();
-        small_fetch_down(a, s, u + a.depth_dn * W, slot);
+        small_fetch_down<ONE>(a, s, u + a.depth_dn * W, slot);
         slot = slot + 1 == a.depth_dn ? 0 : slot + 1;
     }
-    small_wait(0);
 }
 
 // what the separate launches leave in the context; called by all threads of one CTA, after the second barrier
@@ -513,8 +546,11 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) moe_small_kernel(const Small
     // a staging area per warp | packed input rows | packed SwiGLU rows | probabilities and scores
     extern __shared__ __align__(128) uint8_t dyn[];
     __shared__ float s_part[SMALL_WARPS], s_w[SMALL_PAIRS];
-    __shared__ int s_ids[SMALL_PAIRS];
+    __shared__ int s_ids[SMALL_PAIRS], s_late;
+    __shared__ __align__(8) uint64_t s_bars[SMALL_WARPS][SMALL_SLOTS];
     SmallShared s;
+    s.bars = s_bars[threadIdx.x >> 5]; s.phase = 0; s.late = &s_late;
+    small_init(s_bars, &s_late);                         // used after the first barrier
     s.stage = smem_u32(dyn) + (uint32_t)((threadIdx.x >> 5) * a.stage);
     s.q8x = dyn + SMALL_WARPS * a.stage;
     s.q8f = s.q8x + a.T * q8row_stride(a.D);
@@ -527,13 +563,15 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) moe_small_kernel(const Small
     auto expired = [&]() { atomicExch(a.err, 21); };
     small_grid_barrier(a.bar, 1, expired);
     small_gate_up<GU, SUMS>(a, s);
-    small_prefetch_down(a, s);
+    small_prefetch_down<SUMS != SUMS_BLOCKS>(a, s);
     small_grid_barrier(a.bar, 2, expired);
     small_down<DN, SUMS>(a, s);
     if (blockIdx.x == gridDim.x - 1) {
         __syncthreads();
         small_leave_state(a, s);
     }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_late) expired();
     small_leave(a.bar);
 }
 
