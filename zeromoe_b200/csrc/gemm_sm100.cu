@@ -17,6 +17,76 @@ namespace zmoe {
 // reference core/batched_dispatch_pipeline.cpp:1661-1671 done on the device: afterwards every
 // expert's activation rows are contiguous.  One CTA per row, one warp per block.
 constexpr int RT_MAXB = 4;   // blocks per warp: rows up to 8192 elements
+
+// The Q8_K round trip of eight values of a lane's share of a 256-block (the block is the warp's); returns the block's largest magnitude
+__device__ __forceinline__ float roundtrip_block(const float4 v0, const float4 v1, int lane, float (&o)[8]) {
+    const float xv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+    float amax = 0.f, mx = 0.f;
+    int id = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float ax = fabsf(xv[j]);
+        if (ax > amax) { amax = ax; mx = xv[j]; id = 8 * lane + j; }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const float oa = __shfl_xor_sync(0xffffffffu, amax, off), om = __shfl_xor_sync(0xffffffffu, mx, off);
+        const int oi = __shfl_xor_sync(0xffffffffu, id, off);
+        if (oa > amax || (oa == amax && oi < id)) { amax = oa; mx = om; id = oi; }
+    }
+    if (amax == 0.f) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = 0.f;
+    } else {
+        const float iscale = __fdiv_rn(-127.f, mx), d = __fdiv_rn(1.f, iscale);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = __fmul_rn(d, (float)min(127, __float2int_rn(__fmul_rn(iscale, xv[j]))));
+    }
+    return amax;
+}
+// power of two sc with rmax / sc in [2^13, 2^14); 1 for an all-zero or non-finite row
+__device__ __forceinline__ float roundtrip_scale(float rmax) {
+    float sc = 1.f;
+    if (rmax > 0.f && rmax < 3.0e38f) {
+        int ex;
+        frexpf(rmax, &ex);              // rmax = m * 2^ex, m in [0.5, 1)
+        sc = ldexpf(1.f, ex - 14);
+    }
+    return sc;
+}
+
+// The same for rows of up to NB blocks, a warp per row: all of the row's loads are on their way at once and no warp waits for another.  What
+// bounds it: HBM.  (A CTA per row has a quarter of its warps idle at 1536 columns and two barriers per row.)
+template <int NB>
+__global__ void __launch_bounds__(256) q8_roundtrip_rows_kernel(const float *__restrict__ x, int ldx, __half *__restrict__ out, float *__restrict__ scale,
+                                                                const int *__restrict__ hdr, const int *__restrict__ slot, int xdiv, int I) {
+    pdl_wait_prior_grid();
+    pdl_launch_dependents();
+    const int nb = I / QK_K, lane = threadIdx.x & 31, rows = hdr[3];   // pairs with a valid expert
+    for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += 8 * gridDim.x) {
+        const float *const src = x + (size_t)(slot[r] / xdiv) * ldx + 8 * lane;
+        float4 v[NB][2];
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+            if (b < nb) {
+                v[b][0] = *reinterpret_cast<const float4 *>(src + QK_K * b);
+                v[b][1] = *reinterpret_cast<const float4 *>(src + QK_K * b + 4);
+            }
+        float o[NB][8], rmax = 0.f;
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+            if (b < nb) rmax = fmaxf(rmax, roundtrip_block(v[b][0], v[b][1], lane, o[b]));   // |d*q| <= amax up to rounding
+        const float sc = roundtrip_scale(rmax), inv = 1.f / sc;
+        if (lane == 0) scale[r] = sc;
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+            if (b < nb) {
+                const uint2 lo = kpair_pack(o[b][0] * inv, o[b][1] * inv, o[b][2] * inv, o[b][3] * inv);
+                const uint2 hi = kpair_pack(o[b][4] * inv, o[b][5] * inv, o[b][6] * inv, o[b][7] * inv);
+                *reinterpret_cast<uint4 *>(out + (size_t)r * I + QK_K * b + 8 * lane) = make_uint4(lo.x, lo.y, hi.x, hi.y);
+            }
+    }
+}
 __global__ void __launch_bounds__(256) q8_roundtrip_f16_kernel(const float *__restrict__ x, int ldx,
                                                                __half *__restrict__ out, float *__restrict__ scale,
                                                                const int *__restrict__ hdr,
@@ -37,30 +107,7 @@ __global__ void __launch_bounds__(256) q8_roundtrip_f16_kernel(const float *__re
             if (b >= nb) break;
             const float *src = x + (size_t)srow * ldx + QK_K * b + 8 * lane;
             const float4 v0 = *reinterpret_cast<const float4 *>(src), v1 = *reinterpret_cast<const float4 *>(src + 4);
-            const float xv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-            float amax = 0.f, mx = 0.f;
-            int id = 0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float ax = fabsf(xv[j]);
-                if (ax > amax) { amax = ax; mx = xv[j]; id = 8 * lane + j; }
-            }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const float oa = __shfl_xor_sync(0xffffffffu, amax, off), om = __shfl_xor_sync(0xffffffffu, mx, off);
-                const int oi = __shfl_xor_sync(0xffffffffu, id, off);
-                if (oa > amax || (oa == amax && oi < id)) { amax = oa; mx = om; id = oi; }
-            }
-            if (amax == 0.f) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) o[i][j] = 0.f;
-            } else {
-                const float iscale = __fdiv_rn(-127.f, mx), d = __fdiv_rn(1.f, iscale);
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    o[i][j] = __fmul_rn(d, (float)min(127, __float2int_rn(__fmul_rn(iscale, xv[j]))));
-            }
-            wmax = fmaxf(wmax, amax);   // |d*q| <= amax up to rounding
+            wmax = fmaxf(wmax, roundtrip_block(v0, v1, lane, o[i]));   // |d*q| <= amax up to rounding
         }
         __syncthreads();
         if (lane == 0) s_max[warp] = wmax;
@@ -68,14 +115,7 @@ __global__ void __launch_bounds__(256) q8_roundtrip_f16_kernel(const float *__re
         float rmax = 0.f;
 #pragma unroll
         for (int w = 0; w < 8; ++w) rmax = fmaxf(rmax, s_max[w]);
-        // power of two sc with rmax / sc in [2^13, 2^14); 1 for an all-zero or non-finite row
-        float sc = 1.f;
-        if (rmax > 0.f && rmax < 3.0e38f) {
-            int ex;
-            frexpf(rmax, &ex);              // rmax = m * 2^ex, m in [0.5, 1)
-            sc = ldexpf(1.f, ex - 14);
-        }
-        const float inv = 1.f / sc;
+        const float sc = roundtrip_scale(rmax), inv = 1.f / sc;
         if (threadIdx.x == 0) scale[r] = sc;
 #pragma unroll
         for (int i = 0; i < RT_MAXB; ++i) {
@@ -108,30 +148,7 @@ __global__ void __launch_bounds__(256) q8_roundtrip_tokens_kernel(const float *_
             if (b >= nb) break;
             const float *src = x + (size_t)t * ldx + QK_K * b + 8 * lane;
             const float4 v0 = *reinterpret_cast<const float4 *>(src), v1 = *reinterpret_cast<const float4 *>(src + 4);
-            const float xv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-            float amax = 0.f, mx = 0.f;
-            int id = 0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float ax = fabsf(xv[j]);
-                if (ax > amax) { amax = ax; mx = xv[j]; id = 8 * lane + j; }
-            }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const float oa = __shfl_xor_sync(0xffffffffu, amax, off), om = __shfl_xor_sync(0xffffffffu, mx, off);
-                const int oi = __shfl_xor_sync(0xffffffffu, id, off);
-                if (oa > amax || (oa == amax && oi < id)) { amax = oa; mx = om; id = oi; }
-            }
-            if (amax == 0.f) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) o[i][j] = 0.f;
-            } else {
-                const float iscale = __fdiv_rn(-127.f, mx), d = __fdiv_rn(1.f, iscale);
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    o[i][j] = __fmul_rn(d, (float)min(127, __float2int_rn(__fmul_rn(iscale, xv[j]))));
-            }
-            wmax = fmaxf(wmax, amax);
+            wmax = fmaxf(wmax, roundtrip_block(v0, v1, lane, o[i]));   // |d*q| <= amax up to rounding
         }
         __syncthreads();
         if (lane == 0) s_max[warp] = wmax;
@@ -139,13 +156,7 @@ __global__ void __launch_bounds__(256) q8_roundtrip_tokens_kernel(const float *_
         float rmax = 0.f;
 #pragma unroll
         for (int w = 0; w < 8; ++w) rmax = fmaxf(rmax, s_max[w]);
-        float sc = 1.f;
-        if (rmax > 0.f && rmax < 3.0e38f) {
-            int ex;
-            frexpf(rmax, &ex);
-            sc = ldexpf(1.f, ex - 14);
-        }
-        const float inv = 1.f / sc;
+        const float sc = roundtrip_scale(rmax), inv = 1.f / sc;
         uint4 pk[RT_MAXB];
 #pragma unroll
         for (int i = 0; i < RT_MAXB; ++i) {
@@ -184,6 +195,14 @@ int launch_q8_roundtrip_f16(const float *x, int ldx, void *out_f16, float *scale
     if (max_rows <= 0) return ZMOE_OK;
     if (I / QK_K > 8 * RT_MAXB) return ZMOE_ERR_SHAPE;
     const int cap = 8 * device_sm_count();
+    if (I <= 6 * QK_K) {
+        // A warp per row while its registers hold it.  A CTA per row / a warp per row, us: 5 600 rows of 1536 20.5 / 18.7, 32 768 107 / 72; eight
+        // blocks, a CTA's eight warps: 65 536 rows of 2048 238 / 279.
+        const int g8 = (max_rows + 7) / 8, grid8 = g8 < cap ? g8 : cap;
+        return launch_pdl(I <= 4 * QK_K ? q8_roundtrip_rows_kernel<4> : q8_roundtrip_rows_kernel<6>,
+                          dim3((unsigned)grid8), dim3(256), 0, st, x, ldx, static_cast<__half *>(out_f16), scale, (const int *)plan.hdr,
+                          (const int *)plan.slot, xdiv, I) == cudaSuccess ? ZMOE_OK : ZMOE_ERR_CUDA;
+    }
     const int grid = max_rows < cap ? max_rows : cap;
     return launch_pdl(q8_roundtrip_f16_kernel, dim3((unsigned)grid), dim3(256), 0, st, x, ldx,
                       static_cast<__half *>(out_f16), scale, (const int *)plan.hdr, (const int *)plan.slot, xdiv,

@@ -305,9 +305,14 @@ __global__ void __launch_bounds__(128) router_select_kernel(float *logits, const
                     for (int z = 0; z < ROUTER_MAX_SPLIT; z += 2 * w) v[z] = __fadd_rn(v[z], v[z + w]);
                 row[e] = v[0];
             } else {
-                float v = part[(size_t)t * sp.E + e];
-                for (int z = 1; z < ksplit; ++z) v = __fadd_rn(v, part[((size_t)z * T + t) * sp.E + e]);
-                row[e] = v;
+                // all parts on their way before the first is added (one after the other: 17.5 us instead of 11.6 for 700 tokens, sixteen parts)
+                float v[ROUTER_MAX_SPLIT];
+#pragma unroll
+                for (int z = 0; z < ROUTER_MAX_SPLIT; ++z) v[z] = z < ksplit ? part[((size_t)z * T + t) * sp.E + e] : 0.f;
+#pragma unroll
+                for (int z = 1; z < ROUTER_MAX_SPLIT; ++z)
+                    if (z < ksplit) v[0] = __fadd_rn(v[0], v[z]);
+                row[e] = v[0];
             }
         }
         __syncwarp();
