@@ -169,9 +169,10 @@ struct zmoe_layer {
 };
 // Layers whose calls of T tokens the one-kernel forms take: the pairs' experts hold at most this many bytes, and no IQ2_XXS, whose
 // one-pair dot is bound by its table lookups.  One kernel saves about 10 us of launches and plans, and its rows come a little slower
-// than those of the kernels it stands for.  us per layer, one kernel / five launches: Q4_K 2048 / 768: one token (21 MB) 21.5 / 30.5, two (42 MB)
-// 32.9 / 38.0, three (64 MB) 43.4 / 46.9, four (85 MB) 55.6 / 50.4; 4096 / 1536, one token: Q2_K and Q3_K (55 MB) 42.8 / 41.4, Q3_K (65 MB) 48.3 / 47.7.
-static const size_t kFusedCallBytes = (size_t)48 << 20;
+// than those of the kernels it stands for.  us per layer, one kernel / five launches, by MiB: Q4_K 2048 / 768: two tokens (40) 29.0 / 38.0, three
+// (61) 37.5 / 47.6, four (81) 49.0 / 49.8; 4096 / 1536, one token: Q2_K and Q3_K (53) 37.0 / 42.2, Q3_K (62) 41.3 / 48.1; two: Q2_K and
+// Q3_K (105) 60.3 / 52.8.
+static const size_t kFusedCallBytes = (size_t)64 << 20;
 static bool takes_fused(const zmoe_layer_desc &d, int T) {
     const size_t gu = (size_t)d.d_ff * (d.d_model / QK_K) * (block_bytes(d.gate.type) + block_bytes(d.up.type));
     const size_t dn = (size_t)d.d_model * (d.d_ff / QK_K) * block_bytes(d.down.type);
@@ -180,13 +181,16 @@ static bool takes_fused(const zmoe_layer_desc &d, int T) {
 }
 
 // A layer call runs as one kernel only where what every CTA quantises for itself, the tokens' and the pairs' rows, is little too, counted in blocks
-// of 256.  Q4_K, one kernel / five launches, by blocks: 32 (512 / 256, 8 tokens of 2 experts) 18.8 / 28.7, 40 (512 / 1024, 4 of 2) 20.1 / 22.0, 48 (1024 / 512,
-// 4 of 4) 25.2 / 28.6, 51 (256 / 2048, 3 of 2) 24.1 / 22.3, 60 (1024 / 512, 3 of 8) 31.3 / 30.1, 66 (512 / 8192, one of 2) 27.6 / 22.8; with more output
-// rows to share the cost 56 (2048 / 768, 4 of 2) 26.2 / 29.8, 64 (2048 / 768, 2 of 8) 32.9 / 38.0, 72 (2048 / 512, 3 of 8, Q2_K) 37.3 / 34.8.
-// (The decoder step saves far more launches and does not ask.)
+// of 256.  us per layer, one kernel / five launches, by blocks, 2048 output rows and more: 72 (2048 / 512, 3 tokens of 8 experts, Q2_K) 29.9 / 37.1, (2048 /
+// 2048, 3 of 2, Q4_K) 30.9 / 37.3, 80 (2048 / 768, 4 of 4) 31.2 / 34.7, 84 (2048 / 768, 6 of 2) 34.1 / 35.2, 96 (2048 / 768, 3 of 8) 37.5 / 47.6, (2048 /
+// 2048, 4 of 2) 36.2 / 41.7, 98 (2048 / 768, 7 of 2) 38.7 / 36.7, 120 (6 of 4) 41.4 / 40.6.  Fewer rows share that cost among fewer: Q4_K, 32 (512 / 256, 8 of 2)
+// 18.8 / 28.7, 40 (512 / 1024, 4 of 2) 20.1 / 22.0, 48 (1024 / 512, 4 of 4) 25.2 / 28.6, 51 (256 / 2048, 3 of 2) 24.1 / 22.3, 60 (1024 / 512, 3 of
+// 8) 31.3 / 30.1 (these before the rows came by bulk copies).  (The decoder step saves far more launches and does not ask.)
+// Above 64 blocks only with twice as many experts as pairs or more, as in all of these: where pairs share experts, the launches
+// read a shared expert's rows once and the one kernel once per pair.
 static bool repeats_little(const zmoe_layer_desc &d, int T) {
-    const long blocks = (long)T * (d.d_model / QK_K) + (long)T * d.topk * (d.d_ff / QK_K);
-    return blocks <= (d.d_model >= 2048 ? 64 : 48);
+    const long pairs = (long)T * d.topk, blocks = (long)T * (d.d_model / QK_K) + pairs * (d.d_ff / QK_K);
+    return blocks <= (d.d_model < 2048 ? 48 : 2 * pairs <= d.n_experts ? 96 : 64);
 }
 
 namespace zmoe {
