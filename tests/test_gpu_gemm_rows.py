@@ -51,6 +51,8 @@ def test_rows_of_every_alignment(zlib, dev, qtype, D, F):
         torch.cuda.synchronize()
         ctx.check()
         outs[path] = (ctx.act(T, F).copy(), out.cpu().numpy())
+    # the grouped GEMM ran, and not the decode kernels a second time: its weights and activations are fp16
+    assert not np.array_equal(outs[2][0], outs[1][0])
     for got, ref in zip(outs[2], outs[1]):
         got, ref = got.reshape(T, -1), ref.reshape(T, -1)
         assert np.isfinite(got).all()

@@ -165,6 +165,7 @@ struct zmoe_layer {
     } big, small, tc;
     const Proj &set(KernelSet s) const { return s == SET_SMALL ? small : s == SET_BIG ? big : tc; }
     bool dual;
+    bool gemm_shape = false, gemm = false;   // the shapes allow the tensor-core grouped GEMM; and its kernels are as they have to be
     size_t bytes_gate, bytes_up, bytes_down;
 };
 // Layers whose calls of T tokens the one-kernel forms take: the pairs' experts hold at most this many bytes, and no IQ2_XXS, whose
@@ -442,6 +443,9 @@ int zmoe_layer_create(zmoe_ctx *ctx, const zmoe_layer_desc *desc, zmoe_layer **o
         return rc;
     }
     build_tc(d, L->dual, &L->tc);
+    L->gemm_shape = L->dual && gemm_sm100_supported(d.gate.type, d.d_model, d.d_ff) && gemm_sm100_supported(d.down.type, d.d_ff, d.d_model) &&
+                    d.n_experts <= 512;
+    L->gemm = L->gemm_shape && gemm_sm100_built(d.gate.type, true) && gemm_sm100_built(d.down.type, false);
     *out = L;
     return ZMOE_OK;
 }
@@ -451,12 +455,8 @@ void zmoe_layer_destroy(zmoe_layer *layer) { delete layer; }
 // whether zmoe_expert_ffn will take the tensor-core grouped GEMM for T tokens (the rule of the header:
 // shapes allow it, and the path is forced to 2 or left at 0 with enough pairs per expert)
 static bool takes_gemm(const zmoe_layer *L, int T) {
-    const zmoe_layer_desc &d = L->d;
-    const zmoe_ctx *c = L->ctx;
-    const bool gemm_ok = L->dual && gemm_sm100_supported(d.gate.type, d.d_model, d.d_ff) &&
-                         gemm_sm100_supported(d.down.type, d.d_ff, d.d_model) && d.n_experts <= 512;
-    const long P = (long)T * d.topk;
-    return gemm_ok && (c->path == 2 || (c->path == 0 && P >= (long)kGemmMinPairsPerExpert * d.n_experts));
+    const int path = L->ctx->path;
+    return L->gemm && (path == 2 || (path == 0 && (long)T * L->d.topk >= (long)kGemmMinPairsPerExpert * L->d.n_experts));
 }
 
 // how the quantiser writes rows that meet weights of `type`
@@ -574,6 +574,7 @@ int zmoe_expert_ffn_events(zmoe_layer *L, float *out_dev, int T, int accumulate,
     if (!L || !out_dev || T <= 0) return ZMOE_ERR_ARG;
     zmoe_ctx *c = L->ctx;
     if (c->routed_t != T) return ZMOE_ERR_STATE;
+    if (c->path == 2 && L->gemm_shape && !L->gemm) return ZMOE_ERR_CUDA;   // asked for, and lost in the build: not another kernel without a word
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const zmoe_layer_desc &d = L->d;
     const int P = T * d.topk;

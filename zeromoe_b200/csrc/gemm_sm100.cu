@@ -2,7 +2,6 @@
 // the tcgen05 grouped GEMM.
 #include <map>
 #include <mutex>
-#include <set>
 #include <utility>
 
 #include "gemm_sm100.cuh"
@@ -223,25 +222,20 @@ static GemmFn pick_gemm(int type, bool dual) {
     return nullptr;
 }
 
-// The roles' register shares are drawn from the launch's: a build that has fewer would wait for them without end.
-static bool gemm_regs_ok(GemmFn fn) {
-    static std::mutex mu;
-    static std::set<GemmFn> seen;
-    std::lock_guard<std::mutex> lock(mu);
-    if (seen.count(fn)) return true;
+bool gemm_sm100_supported(int type, int I, int O) {
+    return block_bytes(type) != 0 && I > 0 && O > 0 && I % QK_K == 0 && O % GEMM_BM == 0 && pick_gemm(type, true);
+}
+
+// The roles' register shares are drawn from the launch's: a build that has fewer would wait for them without end.  Asked when a layer is
+// created, not per call: the answer loads the kernel.
+bool gemm_sm100_built(int type, bool dual) {
     cudaFuncAttributes at;
-    if (cudaFuncGetAttributes(&at, fn) != cudaSuccess) {
+    const GemmFn fn = pick_gemm(type, dual);
+    if (!fn || cudaFuncGetAttributes(&at, fn) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    if (at.numRegs != GEMM_REGS) return false;
-    seen.insert(fn);
-    return true;
-}
-
-bool gemm_sm100_supported(int type, int I, int O) {
-    return block_bytes(type) != 0 && I > 0 && O > 0 && I % QK_K == 0 && O % GEMM_BM == 0 && pick_gemm(type, true) &&
-           gemm_regs_ok(pick_gemm(type, true)) && gemm_regs_ok(pick_gemm(type, false));
+    return at.numRegs == GEMM_REGS;
 }
 
 // Cycle counters of the instrumented build (see GSTAT_* in gemm_sm100.cuh): two sets of 16 counters on the
