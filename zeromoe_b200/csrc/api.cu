@@ -167,6 +167,7 @@ struct zmoe_layer {
     bool dual;
     bool gemm_shape = false, gemm = false;   // the shapes allow the tensor-core grouped GEMM; and its kernels are as they have to be
     size_t bytes_gate, bytes_up, bytes_down;
+    bool whole = true;          // these hold every row of every expert: the one-kernel forms read whole rows, the others stop at the end
 };
 // Layers whose calls of T tokens the one-kernel forms take: the pairs' experts hold at most this many bytes, and no IQ2_XXS, whose
 // one-pair dot is bound by its table lookups.  One kernel saves about 10 us of launches and plans, and its rows come a little slower
@@ -434,7 +435,9 @@ int zmoe_layer_create(zmoe_ctx *ctx, const zmoe_layer_desc *desc, zmoe_layer **o
         const size_t need = (size_t)O * (I / QK_K) * block_bytes(ws[i]->type);
         if (ws[i]->expert_stride < need) rc = ZMOE_ERR_ARG;
         if ((reinterpret_cast<size_t>(ws[i]->data_dev) & 15) || (ws[i]->expert_stride & 15)) rc = ZMOE_ERR_ALIGN;
-        *tot[i] = ws[i]->bytes ? ws[i]->bytes : (size_t)(d.n_experts - 1) * ws[i]->expert_stride + need;
+        const size_t end = (size_t)(d.n_experts - 1) * ws[i]->expert_stride + need;
+        *tot[i] = ws[i]->bytes ? ws[i]->bytes : end;
+        if (*tot[i] < end) L->whole = false;
     }
     if (!rc && !L->dual && !ctx->act2)
         rc = dev_alloc(&ctx->act2, (size_t)2 * ctx->max_t * ctx->max_k * ctx->max_f);
@@ -816,7 +819,7 @@ uint64_t zmoe_kernel_launches(void) { return g_launches.load(); }
 
 bool zmoe::layer_small_args(zmoe_layer *L, const float *x_dev, float *out_dev, int T, int accumulate, RouterArgs *r, SmallLaunch *s) {
     const zmoe_layer_desc &d = L->d;
-    if (T > L->ctx->max_t || !d.router_w_dev || !L->dual || !takes_fused(d, T) ||
+    if (T > L->ctx->max_t || !d.router_w_dev || !L->dual || !L->whole || !takes_fused(d, T) ||
         !moe_small_supported(d.gate.type, d.down.type, T, d.d_model, d.d_ff, d.n_experts, d.topk))
         return false;
     zmoe_ctx *c = L->ctx;
@@ -824,7 +827,6 @@ bool zmoe::layer_small_args(zmoe_layer *L, const float *x_dev, float *out_dev, i
     s->type_gu = d.gate.type; s->type_dn = d.down.type; s->F = d.d_ff;
     s->w_gate = d.gate.data_dev; s->w_up = d.up.data_dev; s->w_down = d.down.data_dev;
     s->stride_gate = d.gate.expert_stride; s->stride_up = d.up.expert_stride; s->stride_down = d.down.expert_stride;
-    s->total_gate = L->bytes_gate; s->total_up = L->bytes_up; s->total_down = L->bytes_down;
     s->clamp = d.swiglu_clamp; s->clamp_fused = d.swiglu_clamp_fused;
     s->act = c->act; s->out = out_dev; s->accumulate = accumulate;
     s->err = c->err; s->bad = c->bad; s->bar = c->small_bar;

@@ -72,7 +72,7 @@ __device__ __forceinline__ float step_row_dot(uint32_t row, const int8_t *aq, co
 __device__ __forceinline__ void step_fetch(const SmallShared &s, const uint8_t *w, int n_rows, int rb, int o, int slot, int lane) {
     if (o >= n_rows) return;
     if (lane == 0) {
-        small_stage(s.stage + (uint32_t)(slot * ((rb + 47) & ~15)), w, (size_t)n_rows * rb, (size_t)o * rb, rb, &s.bars[slot]);
+        small_stage(s.stage + (uint32_t)(slot * ((rb + 47) & ~15)), w, (size_t)o * rb, rb, &s.bars[slot]);
         mbar_arrive(&s.bars[slot]);
     }
     __syncwarp();

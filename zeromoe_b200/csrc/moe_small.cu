@@ -59,7 +59,6 @@ SmallArgs small_args(const RouterArgs &r, const SmallLaunch &L) {
     a.sp = RouterSpec{r.E, r.K, r.gating, r.normalize, r.weight_scale, r.n_groups, r.n_groups_used};
     a.wg = static_cast<const uint8_t *>(L.w_gate); a.wu = static_cast<const uint8_t *>(L.w_up); a.wd = static_cast<const uint8_t *>(L.w_down);
     a.sg = L.stride_gate; a.su = L.stride_up; a.sd = L.stride_down;
-    a.tg = L.total_gate; a.tu = L.total_up; a.td = L.total_down;
     a.rb_gu = (r.D / QK_K) * block_bytes(L.type_gu);
     a.rb_dn = (L.F / QK_K) * block_bytes(L.type_dn);
     a.clamp = L.clamp; a.clamp_fused = L.clamp_fused;

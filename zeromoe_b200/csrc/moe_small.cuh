@@ -123,7 +123,7 @@ struct SmallArgs {
     int T, D, F, E, K;
     RouterSpec sp;
     const uint8_t *wg, *wu, *wd;
-    size_t sg, su, sd, tg, tu, td;   // bytes between experts, bytes of the tensors
+    size_t sg, su, sd;               // bytes between experts
     int rb_gu, rb_dn;
     float clamp;
     int clamp_fused;
@@ -185,25 +185,17 @@ __device__ __forceinline__ void small_leave(unsigned *bar) {
     }
 }
 
-// `bytes` bytes at byte `at` of a tensor of `total` bytes go to dst, keeping their offset from a 16-byte boundary; called by one lane.
-// dst has room for bytes + 32; only whole 16-byte pieces of the tensor are read, but for its last, which may be short.
+// `bytes` bytes at byte `at` of a tensor go to dst, keeping their offset from a 16-byte boundary; called by one lane.
+// dst has room for bytes + 32.  Only whole 16-byte pieces are read, all of them the tensor's: it begins and ends on a 16-byte boundary, since
+// a matrix has a multiple of 256 rows, or (the QKV matrix and the output head) rows of a multiple of 272 bytes.
 // One bulk copy per row and not 16 bytes per lane: those wait at the load / store unit for the rows before them, so that a warp multiplied
 // its first row only when its last was nearly there, and came to the grid's barrier late by what it had sent for beforehand (a
 // layer of 2048 / 768, one token: fetching 4 200 cycles before gate / up, 4 400 before the barrier after it).
-__device__ __forceinline__ void small_stage(uint32_t dst, const uint8_t *w, size_t total, size_t at, int bytes, uint64_t *bar) {
+__device__ __forceinline__ void small_stage(uint32_t dst, const uint8_t *w, size_t at, int bytes, uint64_t *bar) {
     const int off = (int)(at & 15);
-    const size_t g0 = at - off;
-    int n = (off + bytes + 15) & ~15;
-    if (g0 + (size_t)n > total) {                        // the tensor's last row
-        n -= 16;
-        for (size_t i = g0 + n; i < total; ++i) {
-            const uint32_t v = w[i];
-            asm volatile("st.shared.u8 [%0], %1;" ::"r"(dst + (uint32_t)(i - g0)), "r"(v) : "memory");
-        }
-        if (n == 0) return;
-    }
+    const uint32_t n = (uint32_t)((off + bytes + 15) & ~15);
     asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
-    bulk_g2s_addr(dst, w + g0, (uint32_t)n, bar);
+    bulk_g2s_addr(dst, w + (at - off), n, bar);
 }
 // after a slot's copies have been issued; called by the warp
 __device__ __forceinline__ void small_issued(uint64_t *bar, int lane) {
@@ -323,7 +315,7 @@ __device__ __forceinline__ void small_gate_up(const SmallArgs &a, SmallShared &s
     auto fetch = [&](int slot) {
         if (fu < n_units) {
             if (lane < 2)                                // one lane a matrix
-                small_stage(s.stage + (uint32_t)((2 * slot + lane) * room), lane ? a.wu : a.wg, lane ? a.tu : a.tg,
+                small_stage(s.stage + (uint32_t)((2 * slot + lane) * room), lane ? a.wu : a.wg,
                             (size_t)(uint32_t)s.ids[fp] * (lane ? a.su : a.sg) + (size_t)(uint32_t)fr * (uint32_t)a.rb_gu, a.rb_gu, &s.bars[slot]);
             small_issued(&s.bars[slot], lane);
         }
@@ -418,7 +410,7 @@ __device__ __forceinline__ void small_fetch_down(const SmallArgs &a, const Small
     if (u < a.T * D) {
         const int t = ONE ? 0 : u / D, d = u - t * D;
         if (lane < K)                                    // one lane a row (K is at most 32)
-            small_stage(s.stage + (uint32_t)((slot * K + lane) * room), a.wd, a.td,
+            small_stage(s.stage + (uint32_t)((slot * K + lane) * room), a.wd,
                         (size_t)(uint32_t)s.ids[t * K + lane] * a.sd + (size_t)(uint32_t)d * (uint32_t)a.rb_dn, a.rb_dn, &s.bars[slot]);
         small_issued(&s.bars[slot], lane);
     }

@@ -208,7 +208,7 @@ int launch_block_isums(int type, const void *w, const uint8_t *q8, int32_t *isum
 struct SmallLaunch {
     int type_gu, type_dn, F;
     const void *w_gate, *w_up, *w_down;
-    size_t stride_gate, stride_up, stride_down, total_gate, total_up, total_down;
+    size_t stride_gate, stride_up, stride_down;
     float clamp;
     int clamp_fused;
     float *act, *out;
