@@ -171,9 +171,10 @@ struct zmoe_layer {
 };
 // Layers whose calls of T tokens the one-kernel forms take: the pairs' experts hold at most this many bytes, and no IQ2_XXS, whose
 // one-pair dot is bound by its table lookups.  One kernel saves about 10 us of launches and plans, and its rows come a little slower
-// than those of the kernels it stands for.  us per layer, one kernel / five launches, by MiB: Q4_K 2048 / 768: two tokens (40) 29.0 / 38.0, three
-// (61) 37.5 / 47.6, four (81) 49.0 / 49.8; 4096 / 1536, one token: Q2_K and Q3_K (53) 37.0 / 42.2, Q3_K (62) 41.3 / 48.1; two: Q2_K and
-// Q3_K (105) 60.3 / 52.8.
+// than those of the kernels it stands for.  us per layer, one kernel / five launches, by MiB: Q4_K 2048 / 768: two tokens (40) 28.8 / 37.8, three
+// (61) 37.9 / 47.2, four (81) 50.0 / 51.1; 4096 / 1536, one token: Q2_K and Q3_K (52) 36.9 / 42.2, Q3_K (62) 41.3 / 48.8; two: Q2_K and
+// Q3_K (105) 60.3 / 52.8.  The decoder step, us for four layers, one kernel / separate launches: 4096 / 1536, Q2_K and Q3_K (52) 327 / 366, Q3_K
+// (62) 363 / 391, at position 1024 400 / 514; Q4_K 2048 / 768 (20) 207 / 284.
 static const size_t kFusedCallBytes = (size_t)64 << 20;
 static bool takes_fused(const zmoe_layer_desc &d, int T) {
     const size_t gu = (size_t)d.d_ff * (d.d_model / QK_K) * (block_bytes(d.gate.type) + block_bytes(d.up.type));
@@ -183,16 +184,24 @@ static bool takes_fused(const zmoe_layer_desc &d, int T) {
 }
 
 // A layer call runs as one kernel only where what every CTA quantises for itself, the tokens' and the pairs' rows, is little too, counted in blocks
-// of 256.  us per layer, one kernel / five launches, by blocks, 2048 output rows and more: 72 (2048 / 512, 3 tokens of 8 experts, Q2_K) 29.9 / 37.1, (2048 /
-// 2048, 3 of 2, Q4_K) 30.9 / 37.3, 80 (2048 / 768, 4 of 4) 31.2 / 34.7, 84 (2048 / 768, 6 of 2) 34.1 / 35.2, 96 (2048 / 768, 3 of 8) 37.5 / 47.6, (2048 /
-// 2048, 4 of 2) 36.2 / 41.7, 98 (2048 / 768, 7 of 2) 38.7 / 36.7, 120 (6 of 4) 41.4 / 40.6.  Fewer rows share that cost among fewer: Q4_K, 32 (512 / 256, 8 of 2)
-// 18.8 / 28.7, 40 (512 / 1024, 4 of 2) 20.1 / 22.0, 48 (1024 / 512, 4 of 4) 25.2 / 28.6, 51 (256 / 2048, 3 of 2) 24.1 / 22.3, 60 (1024 / 512, 3 of
-// 8) 31.3 / 30.1 (these before the rows came by bulk copies).  (The decoder step saves far more launches and does not ask.)
-// Above 64 blocks only with twice as many experts as pairs or more, as in all of these: where pairs share experts, the launches
-// read a shared expert's rows once and the one kernel once per pair.
+// of 256 (about 0.15 us for one).  us per layer, one kernel / five launches, experts chosen evenly | by a router with favourites (Zipf 1.1), whose
+// shared rows the launches read once and the one kernel once per pair; "3 of 8": tokens of experts.
+//   Up to 64 blocks, from 2048 output rows on: Q4_K 2048 / 768, 2 of 8 28.8 / 37.8 | 30.1 / 37.7, 4096 / 1024, 2 of 4 31.8 / 41.1 | 32.5 / 43.4, 7168 / 256, 2 of
+//   2 27.7 / 27.5 | 27.9 / 28.3.  Fewer rows share that cost among less work: up to 48, Q4_K 1024 / 512, 4 of 4 22.3 / 29.5 | 22.5 / 27.1, 512 / 256, 8 of 4
+//   23.3 / 30.4 | 23.4 / 32.2; above, 256 / 2048, 3 of 2 (51) 22.9 / 21.9, 512 / 8192, 1 of 2 (66) 25.4 / 23.4.
+//   65 to 96, up to three tokens, to 80 with more: the launches' time grows with the pairs' rows on their way, so a token needs a few experts.  Q4_K 2048 /
+//   768, 3 of 8 (96) 37.9 / 47.2 | 39.1 / 39.4, 4 of 4 (80) 31.1 / 35.6 | 31.5 / 33.5, 7168 / 256, 3 of 4 (96) 40.5 / 52.3 | 40.1 / 53.2, 8192 / 1024, 2 of 2 (80)
+//   37.5 / 42.1 | 36.7 / 41.4; Q2_K 4096 / 512, 3 of 4 (72) 34.5 / 35.4 | 34.2 / 35.3; Q3_K 2048 / 1024, 3 of 4 (72) 20 and 13 % less.  Not taken: Q4_K 3072 / 768, 4
+//   of 4 (96) 43.2 / 42.2 | 42.7 / 37.7, 2048 / 2048, 4 of 2 (96) 35.9 / 40.9 | 36.1 / 27.4, 7168 / 256, 3 of 2 (90) 34.9 / 32.3 | 34.5 / 32.0, 8192 / 2048,
+//   2 of 1 (80) 41.9 / 40.1 | 41.1 / 38.4, 4096 / 1536, 4 of 1 (88) 38.5 / 35.9 | 38.2 / 29.3.
+//   Of 178 shapes in that range (Q4_K, Q3_K, Q2_K with Q3_K; 2048 to 8192 / 256 to 3072; 1 to 8 tokens of 1 to 10 experts) the 97 taken are 11.7 %
+//   faster on average as one kernel with evenly chosen experts, 7.6 % with favourites (worst: 11 and 14 % slower), the 81 not taken 0.3 and 12.0 % slower.
+// Above 64 also only with twice as many experts as pairs or more, as in all of these: among fewer, evenly chosen experts are shared too (2048 / 768, 3 of 8
+// of 32 experts 37.5 / 42.7 | 37.8 / 36.9).  (The decoder step saves far more launches and does not ask.)
 static bool repeats_little(const zmoe_layer_desc &d, int T) {
     const long pairs = (long)T * d.topk, blocks = (long)T * (d.d_model / QK_K) + pairs * (d.d_ff / QK_K);
-    return blocks <= (d.d_model < 2048 ? 48 : 2 * pairs <= d.n_experts ? 96 : 64);
+    if (blocks <= (d.d_model < 2048 ? 48 : 64)) return true;
+    return blocks <= (T <= 3 ? 96 : 80) && d.topk >= (T <= 2 ? 2 : 3) && d.d_model >= 2048 && 2 * pairs <= d.n_experts;
 }
 
 namespace zmoe {
