@@ -406,13 +406,14 @@ __global__ void __launch_bounds__(256) embed_q8_0_kernel(const int32_t *__restri
 // rows of q | k | v.  Token t sits at position *pos + t.  grid (T, ceil((H + KV) / HEADS)), hd / 2 threads: a thread turns its pair of HEADS heads,
 // whose values are on their way while it builds the angle.  What bounds it: the angle, up to 63 products in a row and a sine and a cosine; a head at a
 // time, every head built it anew (512 tokens of 32 + 4 heads: 21.0 us, 5.8 now).
+// late: the attention behind it may not be placed before this kernel's work is done (rope_holds_attention).
 // ---------------------------------------------------------------------------
 constexpr int ROPE_TOKENS = 16;      // from so many tokens on the grid is large enough with six heads per CTA
 template <int HEADS>
 __global__ void rope_kv_kernel(float *__restrict__ qkv, __half *__restrict__ kc, __half *__restrict__ vc,
-                               const int *__restrict__ pos, int H, int KV, int hd, float theta_scale, int max_ctx) {
+                               const int *__restrict__ pos, int H, int KV, int hd, float theta_scale, int max_ctx, int late) {
     pdl_wait_prior_grid();
-    pdl_launch_dependents();
+    if (!late) pdl_launch_dependents();
     const int t = blockIdx.x, h0 = blockIdx.y * HEADS, j = threadIdx.x;
     const int p = *pos + t;
     if (p >= max_ctx) return;
@@ -442,6 +443,7 @@ __global__ void rope_kv_kernel(float *__restrict__ qkv, __half *__restrict__ kc,
             *reinterpret_cast<__half2 *>(vc + at) = __halves2half2(__float2half_rn(vv[i].x), __float2half_rn(vv[i].y));
         }
     }
+    if (late) pdl_launch_dependents();
 }
 
 // ---------------------------------------------------------------------------
@@ -869,13 +871,30 @@ int launch_attention_prompt(const float *qkv, const __half *kc, const __half *vc
                          scale, max_ctx));
 }
 
+// CTAs of the query tiles of T tokens; 0 where the keys are split instead: too few for half of the chip
+int query_tiles(int T, int H, int KV) {
+    const int TQ = AP_ROWS / (H / KV), n = (T + TQ - 1) / TQ * KV;
+    return n >= device_sm_count() / 2 ? n : 0;
+}
+
+// Where the query tiles are about one per SM they must not be placed while the six-head form of RoPE still runs: all of that grid is resident at once, so its
+// dependants may come at once too, and find room for two beside each other on some SMs while others get none.  (A head per CTA is too many CTAs for
+// that; the tiles then came as the last of them left.)  A prompt step of two layers of 2048 / 768, us, tiles early / late, by tiles on 148 SMs: 32 heads
+// on 4 of 128 76 590 / 590, 100 751 / 720, 120 832 / 789, 148 964 / 914, 156 1009 / 961, 176 1109 / 1094, 188 1134 / 1135, 192 817 / 827, 228 908 /
+// 896, 300 1149 / 1173; 64 on 8 80 562 / 578, 96 595 / 607, 104 623 / 600, 144 724 / 701, 176 783 / 770, 184 769 / 800; 32 on 8 104 763 / 726, 136 932 / 886,
+// 176 1108 / 1100; 16 on 2 100 676 / 665, 126 825 / 742, 176 1038 / 957; of 64 16 on 16 112 635 / 615.  With split keys early: 64 on 8, 40 tokens 425 / 454.
+bool rope_holds_attention(int tiles) {
+    const int n = device_sm_count();
+    return 3 * tiles >= 2 * n && 5 * tiles <= 6 * n;
+}
+
 // Attention of T tokens, its rows quantised to Q8_0 (aq, ad): by query tiles where those are enough CTAs for half of the chip (a tile walks all keys on its
 // own, and the number of earlier positions is not known here); below that, keys split over CTAs token by token.
 template <int HD>
 int launch_attention(const float *qkv, const __half *kc, const __half *vc, float *part, float *out, const int *pos, int T, int H,
                      int KV, float scale, int max_ctx, int8_t *aq, float *ad, cudaStream_t st) {
-    const int G = H / KV, TQ = AP_ROWS / G, tiles = (T + TQ - 1) / TQ;
-    if (tiles * KV >= device_sm_count() / 2) {
+    const int G = H / KV;
+    if (query_tiles(T, H, KV)) {
         const int rc = launch_attention_prompt<HD>(qkv, kc, vc, out, pos, T, H, KV, scale, max_ctx, st);
         return rc ? rc : launch_quantize_q8_0(out, H * HD, aq, ad, T, H * HD, st);
     }
@@ -1049,9 +1068,10 @@ int zmoe_decoder_step(zmoe_decoder *dec, const int32_t *tokens_dev, int T, void 
                            (const float *)dec->attn_norm[l], D, d.rms_eps));
         count_launches(1);
         if (!rc) rc = launch_q8_0_mm(dec->qkv, dec->qkv_cols, dec->wqkv[l], dec->aq, dec->ad, T, D, dec->qkv_cols, 0, st);
-        if (!rc) rc = cu(launch_pdl(T >= ROPE_TOKENS ? rope_kv_kernel<6> : rope_kv_kernel<1>, dim3(T, T >= ROPE_TOKENS ? (H + KV + 5) / 6 : H + KV),
-                                    dim3(hd / 2), 0, st, dec->qkv, dec->kc + l * kv_layer,
-                                    dec->vc + l * kv_layer, (const int *)dec->pos, H, KV, hd, theta_scale, d.max_ctx));
+        const bool six = T >= ROPE_TOKENS;
+        if (!rc) rc = cu(launch_pdl(six ? rope_kv_kernel<6> : rope_kv_kernel<1>, dim3(T, six ? (H + KV + 5) / 6 : H + KV), dim3(hd / 2), 0, st, dec->qkv,
+                                    dec->kc + l * kv_layer, dec->vc + l * kv_layer, (const int *)dec->pos, H, KV, hd, theta_scale, d.max_ctx,
+                                    six && rope_holds_attention(query_tiles(T, H, KV)) ? 1 : 0));
         if (!rc) {
             const __half *kl = dec->kc + l * kv_layer, *vl = dec->vc + l * kv_layer;
             rc = hd == 128 ? launch_attention<128>(dec->qkv, kl, vl, dec->apart, dec->ao, dec->pos, T, H, KV, scale, d.max_ctx, dec->aq, dec->ad, st)
