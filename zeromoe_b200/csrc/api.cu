@@ -457,7 +457,7 @@ int zmoe_layer_create(zmoe_ctx *ctx, const zmoe_layer_desc *desc, zmoe_layer **o
     build_tc(d, L->dual, &L->tc);
     L->gemm_shape = L->dual && gemm_sm100_supported(d.gate.type, d.d_model, d.d_ff) && gemm_sm100_supported(d.down.type, d.d_ff, d.d_model) &&
                     d.n_experts <= 512;
-    L->gemm = L->gemm_shape && gemm_sm100_built(d.gate.type, true) && gemm_sm100_built(d.down.type, false);
+    L->gemm = L->gemm_shape && gemm_sm100_built(d.gate.type) && gemm_sm100_built(d.down.type);
     *out = L;
     return ZMOE_OK;
 }

@@ -227,15 +227,19 @@ bool gemm_sm100_supported(int type, int I, int O) {
 }
 
 // The roles' register shares are drawn from the launch's: a build that has fewer would wait for them without end.  Asked when a layer is
-// created, not per call: the answer loads the kernel.
-bool gemm_sm100_built(int type, bool dual) {
-    cudaFuncAttributes at;
-    const GemmFn fn = pick_gemm(type, dual);
-    if (!fn || cudaFuncGetAttributes(&at, fn) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
+// created, not per call: the answer loads the kernels.  Both forms of a type at once: with only the layer's own two loaded, the decode kernels that are
+// loaded next ran up to 0.7 % slower (eight layers of 4096 / 1536, 16 tokens 1377 and 1386 us, in every run), presumably by where they come to lie.
+bool gemm_sm100_built(int type) {
+    for (bool dual : {true, false}) {
+        cudaFuncAttributes at;
+        const GemmFn fn = pick_gemm(type, dual);
+        if (!fn || cudaFuncGetAttributes(&at, fn) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.numRegs != GEMM_REGS) return false;
     }
-    return at.numRegs == GEMM_REGS;
+    return true;
 }
 
 // Cycle counters of the instrumented build (see GSTAT_* in gemm_sm100.cuh): two sets of 16 counters on the

@@ -177,7 +177,7 @@ struct GemmLaunch {
     int n_sm;
 };
 bool gemm_sm100_supported(int type, int I, int O);
-bool gemm_sm100_built(int type, bool dual);   // the compiled kernel has the registers its roles share out
+bool gemm_sm100_built(int type);   // the type's compiled kernels have the registers their roles share out
 unsigned long long *gemm_stats_buffer(int which);
 int gemm_stats_read(unsigned long long *out32);
 int launch_gemm_sm100(const GemmLaunch &L, cudaStream_t st);
