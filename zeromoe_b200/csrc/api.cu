@@ -165,7 +165,7 @@ struct zmoe_layer {
     } big, small, tc;
     const Proj &set(KernelSet s) const { return s == SET_SMALL ? small : s == SET_BIG ? big : tc; }
     bool dual;
-    bool gemm_shape = false, gemm = false;   // the shapes allow the tensor-core grouped GEMM; and its kernels are as they have to be
+    bool gemm_shape = false;    // the shapes allow the tensor-core grouped GEMM
     size_t bytes_gate, bytes_up, bytes_down;
     bool whole = true;          // these hold every row of every expert: the one-kernel forms read whole rows, the others stop at the end
 };
@@ -457,7 +457,6 @@ int zmoe_layer_create(zmoe_ctx *ctx, const zmoe_layer_desc *desc, zmoe_layer **o
     build_tc(d, L->dual, &L->tc);
     L->gemm_shape = L->dual && gemm_sm100_supported(d.gate.type, d.d_model, d.d_ff) && gemm_sm100_supported(d.down.type, d.d_ff, d.d_model) &&
                     d.n_experts <= 512;
-    L->gemm = L->gemm_shape && gemm_sm100_built(d.gate.type) && gemm_sm100_built(d.down.type);
     *out = L;
     return ZMOE_OK;
 }
@@ -468,7 +467,8 @@ void zmoe_layer_destroy(zmoe_layer *layer) { delete layer; }
 // shapes allow it, and the path is forced to 2 or left at 0 with enough pairs per expert)
 static bool takes_gemm(const zmoe_layer *L, int T) {
     const int path = L->ctx->path;
-    return L->gemm && (path == 2 || (path == 0 && (long)T * L->d.topk >= (long)kGemmMinPairsPerExpert * L->d.n_experts));
+    return L->gemm_shape && (path == 2 || (path == 0 && (long)T * L->d.topk >= (long)kGemmMinPairsPerExpert * L->d.n_experts)) &&
+           gemm_sm100_built(L->d.gate.type) && gemm_sm100_built(L->d.down.type);
 }
 
 // how the quantiser writes rows that meet weights of `type`
@@ -586,7 +586,7 @@ int zmoe_expert_ffn_events(zmoe_layer *L, float *out_dev, int T, int accumulate,
     if (!L || !out_dev || T <= 0) return ZMOE_ERR_ARG;
     zmoe_ctx *c = L->ctx;
     if (c->routed_t != T) return ZMOE_ERR_STATE;
-    if (c->path == 2 && L->gemm_shape && !L->gemm) return ZMOE_ERR_CUDA;   // asked for, and lost in the build: not another kernel without a word
+    if (c->path == 2 && L->gemm_shape && !takes_gemm(L, T)) return ZMOE_ERR_CUDA;   // asked for, and lost in the build: not another kernel without a word
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const zmoe_layer_desc &d = L->d;
     const int P = T * d.topk;

@@ -1,5 +1,6 @@
 // gemm_sm100.cu -- launchers of the prefill path: Q8_K round trip of activations to fp16 and
 // the tcgen05 grouped GEMM.
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -226,20 +227,27 @@ bool gemm_sm100_supported(int type, int I, int O) {
     return block_bytes(type) != 0 && I > 0 && O > 0 && I % QK_K == 0 && O % GEMM_BM == 0 && pick_gemm(type, true);
 }
 
-// The roles' register shares are drawn from the launch's: a build that has fewer would wait for them without end.  Asked when a layer is
-// created, not per call: the answer loads the kernels.  Both forms of a type at once: with only the layer's own two loaded, the decode kernels that are
-// loaded next ran up to 0.7 % slower (eight layers of 4096 / 1536, 16 tokens 1377 and 1386 us, in every run), presumably by where they come to lie.
+// The roles' register shares are drawn from the launch's: a build that has fewer would wait for them without end.  Asked by calls that are about to
+// run the kernels, once per type: the first answer loads them (2 ms).
 bool gemm_sm100_built(int type) {
-    for (bool dual : {true, false}) {
-        cudaFuncAttributes at;
-        const GemmFn fn = pick_gemm(type, dual);
-        if (!fn || cudaFuncGetAttributes(&at, fn) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
+    static std::atomic<int> known[32];               // 0 not asked yet, 1 no, 2 yes
+    if (type < 0 || type >= 32) return false;
+    int k = known[type].load(std::memory_order_relaxed);
+    if (k == 0) {
+        k = 2;
+        for (bool dual : {true, false}) {
+            cudaFuncAttributes at;
+            const GemmFn fn = pick_gemm(type, dual);
+            if (!fn) return false;
+            if (cudaFuncGetAttributes(&at, fn) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            if (at.numRegs != GEMM_REGS) k = 1;
         }
-        if (at.numRegs != GEMM_REGS) return false;
+        known[type].store(k, std::memory_order_relaxed);
     }
-    return true;
+    return k == 2;
 }
 
 // Cycle counters of the instrumented build (see GSTAT_* in gemm_sm100.cuh): two sets of 16 counters on the
