@@ -17,7 +17,7 @@
  *   - the tensor-core grouped GEMM (the layer entry from that threshold up, or
  *     zmoe_ctx_set_path(ctx, 2)) multiplies fp16 operands with f32 accumulation:
  *     the activation operand is the exact Q8_K value d*q divided by a power of two,
- *     the weight operand is the dequantised weight rounded to fp16 once.  There is no
+ *     the weight operand is dequantised in fp16 (block scale and min rounded once each, then the weight).  There is no
  *     int32 block sum on that path; results agree with the CPU path to about 3e-4 of
  *     the output norm (1e-3 is the bound the tests hold it to), and a token's output
  *     therefore depends, within that bound, on whether its batch took this path.

@@ -44,7 +44,9 @@ struct DecoderStep {
 // [0, 1] grid barrier, [2, 3] arg-max key, then a ticket per KV head
 int decoder_step_sync_words(int KV) { return 4 + KV; }
 
-constexpr int STEP_STATIC = 2 * 1024, STEP_SMEM = 227 * 1024 - STEP_STATIC;   // the kernel's static arrays, rounded up
+// The kernel's static arrays (1920 bytes), rounded up.  With more of them the request for all of STEP_SMEM fails when a decoder is created, and its
+// steps are separate launches.
+constexpr int STEP_STATIC = 2 * 1024, STEP_SMEM = 227 * 1024 - STEP_STATIC;
 
 DecoderStep *decoder_step_create(const DecoderStepDesc &d) {
     int dev = 0, coop = 0;

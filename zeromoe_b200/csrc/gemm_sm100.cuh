@@ -32,10 +32,11 @@
 // 80 pairs use half of the accumulator columns and alternate between two buffers, so that the
 // drain of one overlaps the MMAs of the next.  Below about 100 pairs the converters' instruction issue is the limit (every
 // weight is converted once per pair block): 64 % of the issue slots at 44 pairs, the integer pipe half busy.
-// Measured on one B200, layers of 128 experts, us per layer with all its launches, this form against one where sixteen
-// warps converted 64 weights at a time and drained as well and one warp issued all MMAs: 4096 / 1536, Q2_K gate and up, Q3_K down, 512 tokens
-// 759 -> 542, 700 785 -> 570, 1024 831 -> 625; IQ2_XXS 700 tokens 836 -> 650; Q3_K 700 919 -> 685; Q4_K 2048 / 768 512 tokens 247 -> 196;
-// 4096 tokens of IQ2_XXS, skewed load, 2368 -> 2080; 8192 tokens of 7168 / 2048, 256 experts, Q4_K, with a shared expert 10 270 -> 8 900.
+// Measured on one B200, layers of 128 experts, us per layer with all its launches, the same layer and input called over and over, this form against
+// one where sixteen warps converted 64 weights at a time and drained as well and one warp issued all MMAs: 4096 / 1536, Q2_K gate and up, Q3_K down, 512
+// tokens 760 -> 548, 700 785 -> 576, 1024 831 -> 624; IQ2_XXS 700 tokens 836 -> 637; Q3_K 700 928 -> 671; Q4_K 2048 / 768 512 tokens 247 -> 189.
+// With layers and inputs that change from call to call: 700 tokens 785 -> 616; 4096 tokens of IQ2_XXS, skewed load, 2351 -> 2058; 8192 tokens of 7168 / 2048, 256
+// experts, Q4_K, with a shared expert 10 250 -> 8 820.
 // Tiles of more than 80 pairs wait for the drain of the one before: its instructions per column count (35 -> about 20 by a loop without clamps,
 // 128-bit loads of the columns' scales and pairs and no predicates on full chunks: 4096 tokens 1908 -> 1734 and, Q4_K 2048 / 768, 775 -> 645).
 // Eight drain warps instead of four took 1718 and 643 there, but 617 instead of 587 at 700 tokens; a drain that loads the next columns
@@ -43,7 +44,8 @@
 // Activations arrive already rounded through Q8_K (value = d * q) as fp16, each row divided by a
 // power of two that brings its largest value near 2^13 (undone exactly in the epilogue), so the
 // result follows the reference CPU path's activation quantisation and cannot overflow fp16;
-// weights are rounded to fp16 after the reference dequantiser's f32 arithmetic.
+// weights are fp16 too (dequant_f16.cuh): exact integer part, block scale and min each rounded once, then one fp16 multiplication or multiply-add.
+// A weight is off by at most 2^-11 of itself for that and 2^-11 of the scaled part and of the min (IQ2_XXS: one rounding of a scaled magnitude).
 // Every wait is bounded; on expiry the CTA raises the error flag and unwinds, and the
 // tensor memory is always released.
 #pragma once

@@ -28,7 +28,7 @@ static SmallFn pick_sums(SmallSums sums, int gu, int dn) {
     return sums == SUMS_SHORT ? pick_small<SUMS_SHORT>(gu, dn) : sums == SUMS_LONG ? pick_small<SUMS_LONG>(gu, dn) : pick_small<SUMS_BLOCKS>(gu, dn);
 }
 
-// shared memory of the kernel's static arrays, rounded up
+// shared memory of the kernel's static arrays (896 bytes), rounded up; a launch asks for all of SMALL_SMEM, so a build with more of them is refused
 constexpr int SMALL_STATIC = 1024, SMALL_SMEM = 227 * 1024 - SMALL_STATIC;
 
 // Rows on their way per warp and the bytes they take; 0 where a shape does not fit
